@@ -14,6 +14,7 @@
 
 #include "../../include/tenax_b200.h"
 #include "common.cuh"
+#include "contract_f64.hpp"
 #include "kernels.cuh"
 #include "planner.hpp"
 #include "planner_dev.hpp"
@@ -239,6 +240,13 @@ struct StepDev {
   DevMem packA, chunksA, packB, chunksB, groups, tiles, rowoff, scat, chunksS, out_tab;
   int nA = 0, nB = 0, nT = 0, nS = 0;
   bool res_f32 = false;
+  // FP64 in one launch (contract_f64.cu): tables of the step in one buffer
+  bool direct = false, swapped = false;
+  DevMem blob;
+  ContractLaunch dl{};
+  // a single operand's permutation: one strided copy
+  bool copy = false;
+  int n_copy = 0;
 };
 
 struct tnx_plan {
@@ -553,6 +561,256 @@ int tnx_plan_workspace(const tnx_plan* plan, int32_t precision, size_t* bytes) {
   })
 }
 
+namespace {
+// Offset tables of one step's axes: an axis of legs (extent, stride), outermost
+// first, is affine where the legs merge into one stride, and otherwise a table
+// shared by every axis of the same legs.
+struct AxisTabs {
+  std::vector<int32_t> tab;
+  std::map<std::vector<std::pair<int64_t, int64_t>>, int32_t> seen;
+  void add(const std::vector<std::pair<int64_t, int64_t>>& legs, int32_t* t, int32_t* str) {
+    std::vector<std::pair<int64_t, int64_t>> m;
+    for (const auto& l : legs) {
+      if (l.first == 1) continue;
+      if (!m.empty() && m.back().second == l.first * l.second)
+        m.back() = {m.back().first * l.first, l.second};
+      else
+        m.push_back(l);
+    }
+    *t = -1;
+    *str = m.empty() ? 0 : static_cast<int32_t>(m[0].second);
+    if (m.size() < 2) return;
+    *str = static_cast<int32_t>(m.back().second);
+    auto it = seen.find(m);
+    if (it == seen.end()) {
+      it = seen.emplace(m, static_cast<int32_t>(tab.size())).first;
+      int64_t n = 1;
+      for (const auto& l : m) n *= l.first;
+      if (static_cast<int64_t>(tab.size()) + n > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "axis tables too large"};
+      for (int64_t i = 0; i < n; ++i) {
+        int64_t rem = i, off = 0;
+        for (size_t l = m.size(); l-- > 0;) {
+          off += (rem % m[l].first) * m[l].second;
+          rem /= m[l].first;
+        }
+        tab.push_back(static_cast<int32_t>(off));
+      }
+    }
+    *t = it->second;
+  }
+};
+
+// The legs with a nonzero stride in `order` (the planner's row, K or column
+// flattening), outermost first, with their strides inside the row-major block.
+std::vector<std::pair<int64_t, int64_t>> axis_legs(int nlegs, const int32_t* dims, const int32_t* order) {
+  std::vector<std::pair<int32_t, int>> by;
+  for (int l = 0; l < nlegs; ++l)
+    if (order[l]) by.push_back({order[l], l});
+  // larger flattening stride = outer; equal strides only differ by extent-1 legs
+  std::stable_sort(by.begin(), by.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::vector<std::pair<int64_t, int64_t>> legs;
+  for (const auto& b : by) {
+    int64_t str = 1;
+    for (int l = b.second + 1; l < nlegs; ++l) str *= dims[l];
+    legs.push_back({dims[b.second], str});
+  }
+  return legs;
+}
+
+int64_t extent_of(const std::vector<std::pair<int64_t, int64_t>>& legs) {
+  int64_t n = 1;
+  for (const auto& l : legs) n *= l.first;
+  return n;
+}
+
+// whether the fastest leg of the axis `k` is nearer in memory than that of `r`
+bool k_is_fast(const std::vector<std::pair<int64_t, int64_t>>& r, const std::vector<std::pair<int64_t, int64_t>>& k) {
+  int64_t sr = INT64_MAX, sk = INT64_MAX;
+  for (const auto& l : r)
+    if (l.first > 1) sr = std::min(sr, l.second);
+  for (const auto& l : k)
+    if (l.first > 1) sk = std::min(sk, l.second);
+  return sk < sr;
+}
+
+// Tables of the one-launch FP64 kernel for one step.  It serves every step
+// whose blocks hold fewer than 2^31 elements (its in-block offsets are 32-bit)
+// and carry no fermionic sign; the others keep the packed path, which negates
+// on the way in and out.  Measured, packed against one launch: theta of
+// chi = 64 24 -> 6 us of device time, a CTM step's 196 products 33 -> 8 ms.
+bool build_direct(const PairPlan& P, StepDev& d) {
+  constexpr int64_t kMaxBlock = int64_t{1} << 31;
+  for (const auto* v : {&P.packA, &P.packB})
+    for (const auto& s : *v)
+      if (s.neg || s.count >= kMaxBlock) return false;
+  for (const auto& s : P.scatter)
+    if (s.neg || s.count >= kMaxBlock) return false;
+  AxisTabs T;
+  struct Side {
+    int64_t off = 0, rows = 0, k = 0;
+    int32_t rt, rs, kt, ks;
+  };
+  // per group: (row origin, K origin) -> block, and the K origins of each row origin
+  auto index = [&](const std::vector<PackSeg>& segs, bool* kfast) {
+    std::map<std::pair<int32_t, int32_t>, std::map<int32_t, Side>> by;  // (group, row0) -> k0 -> block
+    int64_t fast = 0, slow = 0;
+    for (const auto& s : segs) {
+      Side x;
+      const auto r = axis_legs(s.nlegs, s.dims, s.rstr), k = axis_legs(s.nlegs, s.dims, s.kstr);
+      x.off = s.src_off;
+      x.rows = extent_of(r);
+      x.k = extent_of(k);
+      T.add(r, &x.rt, &x.rs);
+      T.add(k, &x.kt, &x.ks);
+      (k_is_fast(r, k) ? fast : slow) += s.count;
+      by[{s.group, s.row0}][s.k0] = x;
+    }
+    *kfast = fast > slow;
+    return by;
+  };
+  bool a_kfast = false, b_kfast = false;
+  const auto A = index(P.packA, &a_kfast), B = index(P.packB, &b_kfast);
+  // rows are the longer side of a tile (128 x 16)
+  int64_t sm = 0, sn = 0;
+  for (const auto& sc : P.scatter) {
+    sm += extent_of(axis_legs(sc.nlegs, sc.dims, sc.rstr));
+    sn += extent_of(axis_legs(sc.nlegs, sc.dims, sc.cstr));
+  }
+  d.swapped = sn > sm;
+  std::vector<ContractSpan> spans;
+  std::vector<ContractTile> proto;
+  std::vector<ContractBlk> blks;
+  for (const auto& sc : P.scatter) {
+    if (sc.count == 0) continue;
+    ContractTile t{};
+    ContractBlk blk{};
+    const auto r = axis_legs(sc.nlegs, sc.dims, sc.rstr), c = axis_legs(sc.nlegs, sc.dims, sc.cstr);
+    t.out_off = sc.dst_off;
+    t.M = static_cast<int32_t>(extent_of(r));
+    t.N = static_cast<int32_t>(extent_of(c));
+    T.add(r, &t.r_tab, &t.r_str);
+    T.add(c, &t.c_tab, &t.c_str);
+    t.span0 = static_cast<int32_t>(spans.size());
+    auto ia = A.find({sc.group, sc.row0});
+    auto ib = B.find({sc.group, sc.col0});
+    if (ia != A.end() && ib != B.end())
+      for (const auto& kv : ia->second) {
+        auto jb = ib->second.find(kv.first);
+        if (jb == ib->second.end()) continue;
+        const Side &x = kv.second, &y = jb->second;
+        if (x.rows != t.M || y.rows != t.N || x.k != y.k) return false;
+        ContractSpan g{};
+        g.a_off = x.off;
+        g.b_off = y.off;
+        g.ar_tab = x.rt, g.ar_str = x.rs, g.ak_tab = x.kt, g.ak_str = x.ks;
+        g.br_tab = y.rt, g.br_str = y.rs, g.bk_tab = y.kt, g.bk_str = y.ks;
+        g.K = static_cast<int32_t>(x.k);
+        spans.push_back(g);
+        blk.ktiles += cdiv(x.k, 16);
+        blk.k4 += cdiv(x.k, 4);
+      }
+    t.nspan = static_cast<int32_t>(spans.size()) - t.span0;
+    if (blk.ktiles > INT32_MAX) return false;
+    t.ktiles = static_cast<int32_t>(blk.ktiles);
+    if (d.swapped) {
+      std::swap(t.M, t.N);
+      std::swap(t.r_tab, t.c_tab);
+      std::swap(t.r_str, t.c_str);
+    }
+    blk.M = t.M;
+    blk.N = t.N;
+    blks.push_back(blk);
+    proto.push_back(t);
+  }
+  if (d.swapped) {
+    std::swap(a_kfast, b_kfast);
+    for (auto& g : spans) {
+      std::swap(g.a_off, g.b_off);
+      std::swap(g.ar_tab, g.br_tab);
+      std::swap(g.ar_str, g.br_str);
+      std::swap(g.ak_tab, g.bk_tab);
+      std::swap(g.ak_str, g.bk_str);
+    }
+  }
+  ContractLaunch& L = d.dl;
+  contract_choose(blks, device_sm_count(), &L.shape, &L.split);
+  L.a_kfast = a_kfast;
+  L.b_kfast = b_kfast;
+  int bm, bn;
+  contract_tile_shape(L.shape, &bm, &bn);
+  // longest tiles first
+  std::vector<std::pair<int64_t, ContractTile>> tl;
+  for (size_t i = 0; i < proto.size(); ++i)
+    for (int64_t m0 = 0; m0 < proto[i].M; m0 += bm)
+      for (int64_t n0 = 0; n0 < proto[i].N; n0 += bn) {
+        ContractTile t = proto[i];
+        t.m0 = static_cast<int32_t>(m0);
+        t.n0 = static_cast<int32_t>(n0);
+        const int64_t cost = blks[i].k4 * cdiv(std::min<int64_t>(bm, t.M - m0), 8) *
+                             cdiv(std::min<int64_t>(bn, t.N - n0), 8);
+        tl.push_back({cost, t});
+      }
+  if (static_cast<int64_t>(tl.size()) * L.split > INT32_MAX) return false;
+  std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  std::vector<ContractTile> tiles;
+  tiles.reserve(tl.size());
+  for (const auto& x : tl) tiles.push_back(x.second);
+  L.n_tiles = static_cast<int>(tiles.size());
+  // one buffer, one copy: spans, tiles, axis tables
+  const size_t o_t = spans.size() * sizeof(ContractSpan), o_x = o_t + tiles.size() * sizeof(ContractTile);
+  std::vector<uint8_t> h(std::max<size_t>(64, o_x + T.tab.size() * sizeof(int32_t)));
+  if (!spans.empty()) std::memcpy(h.data(), spans.data(), spans.size() * sizeof(ContractSpan));
+  if (!tiles.empty()) std::memcpy(h.data() + o_t, tiles.data(), tiles.size() * sizeof(ContractTile));
+  if (!T.tab.empty()) std::memcpy(h.data() + o_x, T.tab.data(), T.tab.size() * sizeof(int32_t));
+  upload(d.blob, h);
+  uint8_t* base = d.blob.as<uint8_t>();
+  L.spans = reinterpret_cast<const ContractSpan*>(base);
+  L.tiles = reinterpret_cast<const ContractTile*>(base + o_t);
+  L.tab = reinterpret_cast<const int32_t*>(base + o_x);
+  d.direct = true;
+  return true;
+}
+
+// A single operand without fermionic signs: each block is copied to its
+// permuted place, in any precision (the packed path's product with a scalar 1
+// rounds in the mixed precisions, so those keep it).
+bool build_copy(const PairPlan& P, StepDev& d) {
+  for (const auto& s : P.packA)
+    if (s.neg) return false;
+  std::map<std::pair<int32_t, int32_t>, const PackSeg*> by_row;
+  for (const auto& s : P.packA) by_row[{s.group, s.row0}] = &s;
+  std::vector<DevCopySeg> segs;
+  std::vector<DevChunk> chunks;
+  for (const auto& sc : P.scatter) {
+    if (sc.neg) return false;
+    auto it = by_row.find({sc.group, sc.row0});
+    if (it == by_row.end() || it->second->count != sc.count) return false;
+    const PackSeg& s = *it->second;
+    DevCopySeg c{};
+    c.src_off = s.src_off;
+    c.dst_off = sc.dst_off;
+    c.nlegs = s.nlegs;
+    for (int l = 0; l < s.nlegs; ++l) {
+      // the output leg that comes from this operand leg
+      const size_t pos = P.out_subs.find(P.a_subs[l]);
+      if (pos == std::string::npos) return false;
+      int64_t str = 1;
+      for (int o = static_cast<int>(pos) + 1; o < sc.nlegs; ++o) str *= sc.dims[o];
+      c.dims[l] = s.dims[l];
+      c.dstr[l] = str;
+    }
+    const int id = static_cast<int>(segs.size());
+    segs.push_back(c);
+    for (int64_t e = 0; e < sc.count; e += 2048) chunks.push_back({id, 0, e, std::min<int64_t>(2048, sc.count - e)});
+  }
+  upload(d.scat, segs);
+  upload(d.chunksS, chunks);
+  d.n_copy = static_cast<int>(chunks.size());
+  d.copy = true;
+  return true;
+}
+}  // namespace
+
 static void plan_build_device(tnx_plan* p, int precision) {
   const int mode = img_mode_of(precision);
   const ImgGeom ig = img_geom(mode);
@@ -570,6 +828,10 @@ static void plan_build_device(tnx_plan* p, int precision) {
     const PairPlan& P = p->steps[s];
     auto d = std::make_unique<StepDev>();
     d->mode = mode;
+    if (mode == IMG_F64 && (p->has_scalar ? build_copy(P, *d) : build_direct(P, *d))) {
+      p->dev.push_back(std::move(d));
+      continue;
+    }
     d->G = pair_geom(P, mode);
     const int split = mode == IMG_BF16 ? 2 : 1;
     d->a_img.alloc(std::max<int64_t>(1, d->G.a_tiles) * ig.tile_bytes * split);
@@ -664,6 +926,19 @@ int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, i
       const double* a_ptr = plan->a_src[s] >= 0 ? inputs[plan->a_src[s]] : plan->inter[s - 1]->as<double>();
       const double* b_ptr = plan->has_scalar ? plan->scalar_one.as<double>() : inputs[plan->b_src[s]];
       double* o_ptr = (s + 1 == plan->steps.size()) ? out : plan->inter[s]->as<double>();
+      if (d.direct) {
+        ContractLaunch L = d.dl;
+        L.a = d.swapped ? b_ptr : a_ptr;
+        L.b = d.swapped ? a_ptr : b_ptr;
+        L.c = o_ptr;
+        CUDA_OK(launch_contract_f64(L, st));
+        continue;
+      }
+      if (d.copy) {
+        launch_strided_copy(a_ptr, o_ptr, d.scat.as<DevCopySeg>(), d.chunksS.as<DevChunk>(), d.n_copy, st);
+        CUDA_OK(cudaGetLastError());
+        continue;
+      }
       PtrTab src{};
       src.p[0] = reinterpret_cast<uint64_t>(a_ptr);
       src.p[1] = reinterpret_cast<uint64_t>(b_ptr);

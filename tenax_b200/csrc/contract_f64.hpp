@@ -1,0 +1,50 @@
+// One-launch FP64 contraction (contract_f64.cu): its tables and launch.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+namespace tnx {
+
+// One (A block, B block) pair of an output block.  An axis maps an index to an
+// element offset inside its block: index * str, or tab[index] where `*_tab` is
+// the first entry of a table (>= 0).
+struct ContractSpan {
+  int64_t a_off, b_off;  // element offsets of the two blocks
+  int32_t ar_tab, ar_str, ak_tab, ak_str;
+  int32_t br_tab, br_str, bk_tab, bk_str;
+  int32_t K, pad0, pad1, pad2;
+};
+static_assert(sizeof(ContractSpan) == 64, "read as four 16-byte units");
+
+struct ContractTile {
+  int64_t out_off;        // element offset of the output block
+  int32_t M, N, m0, n0;   // the block's extents, the tile's origin
+  int32_t span0, nspan, ktiles;  // pairs summed; 16-deep K tiles of all of them
+  int32_t r_tab, r_str, c_tab, c_str;
+  int32_t pad;
+};
+
+// an output block as the choice of tile shape sees it
+struct ContractBlk {
+  int64_t M, N, ktiles, k4;  // k4: 4-deep K steps of all pairs
+};
+
+struct ContractLaunch {
+  const double *a, *b;
+  double* c;
+  const ContractTile* tiles;
+  const ContractSpan* spans;
+  const int32_t* tab;
+  int n_tiles, shape, split;
+  bool a_kfast, b_kfast;  // whether K is the fast axis of the operand's blocks
+};
+
+constexpr int kContractShapes = 3;
+void contract_tile_shape(int shape, int* bm, int* bn);
+void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split);
+cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st);
+
+}  // namespace tnx
