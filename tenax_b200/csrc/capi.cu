@@ -637,7 +637,7 @@ bool k_is_fast(const std::vector<std::pair<int64_t, int64_t>>& r, const std::vec
 // whose blocks hold fewer than 2^31 elements (its in-block offsets are 32-bit)
 // and carry no fermionic sign; the others keep the packed path, which negates
 // on the way in and out.  Measured, packed against one launch: theta of
-// chi = 64 24 -> 6 us of device time, a CTM step's 196 products 33 -> 8 ms.
+// chi = 64 24 -> 3 us of device time, a CTM step's 196 products 33 -> 6 ms.
 bool build_direct(const PairPlan& P, StepDev& d) {
   constexpr int64_t kMaxBlock = int64_t{1} << 31;
   for (const auto* v : {&P.packA, &P.packB})
@@ -650,26 +650,50 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     int64_t off = 0, rows = 0, k = 0;
     int32_t rt, rs, kt, ks;
   };
-  // per group: (row origin, K origin) -> block, and the K origins of each row origin
-  auto index = [&](const std::vector<PackSeg>& segs, bool* kfast) {
+  // Whether K is the fast axis of an operand, and the order in which K is
+  // walked: any order of the contracted legs gives the same sum, so it is the
+  // memory order of an operand whose fast axis is K (of the larger one, if both
+  // are), whose lanes then read consecutive elements.
+  auto kfast_of = [&](const std::vector<PackSeg>& segs, int64_t* elems) {
+    int64_t fast = 0;
+    *elems = 0;
+    for (const auto& s : segs) {
+      *elems += s.count;
+      if (k_is_fast(axis_legs(s.nlegs, s.dims, s.rstr), axis_legs(s.nlegs, s.dims, s.kstr))) fast += s.count;
+    }
+    return 2 * fast > *elems;
+  };
+  int64_t na = 0, nb = 0;
+  bool a_kfast = kfast_of(P.packA, &na), b_kfast = kfast_of(P.packB, &nb);
+  const bool b_order = b_kfast && (!a_kfast || nb > na);
+  std::string korder;
+  for (char c : b_order ? P.b_subs : P.a_subs)
+    if ((b_order ? P.a_subs : P.b_subs).find(c) != std::string::npos) korder.push_back(c);
+  auto k_legs = [&](const PackSeg& s, const std::string& subs) {
+    std::vector<std::pair<int64_t, int64_t>> legs;
+    for (char c : korder) {
+      const int l = static_cast<int>(subs.find(c));
+      int64_t str = 1;
+      for (int m = l + 1; m < s.nlegs; ++m) str *= s.dims[m];
+      legs.push_back({s.dims[l], str});
+    }
+    return legs;
+  };
+  auto index = [&](const std::vector<PackSeg>& segs, const std::string& subs) {
     std::map<std::pair<int32_t, int32_t>, std::map<int32_t, Side>> by;  // (group, row0) -> k0 -> block
-    int64_t fast = 0, slow = 0;
     for (const auto& s : segs) {
       Side x;
-      const auto r = axis_legs(s.nlegs, s.dims, s.rstr), k = axis_legs(s.nlegs, s.dims, s.kstr);
+      const auto r = axis_legs(s.nlegs, s.dims, s.rstr), k = k_legs(s, subs);
       x.off = s.src_off;
       x.rows = extent_of(r);
       x.k = extent_of(k);
       T.add(r, &x.rt, &x.rs);
       T.add(k, &x.kt, &x.ks);
-      (k_is_fast(r, k) ? fast : slow) += s.count;
       by[{s.group, s.row0}][s.k0] = x;
     }
-    *kfast = fast > slow;
     return by;
   };
-  bool a_kfast = false, b_kfast = false;
-  const auto A = index(P.packA, &a_kfast), B = index(P.packB, &b_kfast);
+  const auto A = index(P.packA, P.a_subs), B = index(P.packB, P.b_subs);
   // rows are the longer side of a tile (128 x 16)
   int64_t sm = 0, sn = 0;
   for (const auto& sc : P.scatter) {
@@ -733,7 +757,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     }
   }
   ContractLaunch& L = d.dl;
-  contract_choose(blks, device_sm_count(), &L.shape, &L.split);
+  contract_choose(blks, device_sm_count(), &L.shape, &L.split, &L.parts);
   L.a_kfast = a_kfast;
   L.b_kfast = b_kfast;
   int bm, bn;
@@ -750,7 +774,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
                              cdiv(std::min<int64_t>(bn, t.N - n0), 8);
         tl.push_back({cost, t});
       }
-  if (static_cast<int64_t>(tl.size()) * L.split > INT32_MAX) return false;
+  if (static_cast<int64_t>(tl.size()) * L.split * L.parts > INT32_MAX) return false;
   std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
   std::vector<ContractTile> tiles;
   tiles.reserve(tl.size());

@@ -19,8 +19,14 @@
 // Shapes with few output tiles and a long K (CTM projections: 80 x 80 x 1280)
 // split K over the CTAs of one cluster, which add their partial tiles through
 // distributed shared memory in rank order: no workspace, no atomics, and the
-// same bits on every run.  contract_choose() picks tile and split from a cost
-// model of the step's tiles.
+// same bits on every run.  A K too long for eight CTAs (the last product of a
+// two-site density matrix: 4 x 4 x 102400, 1200 us with a cluster alone, 33 us)
+// takes several clusters a tile, whose parts a second launch adds in order.
+//
+// Measured, CUDA events: 80 x 80 x 1280 76 us unsplit, 10.5 us; 1280 x 1280 x
+// 80 18.8 us (14 TFLOP/s); 6400 x 1024 x 256 131 us (26 TFLOP/s); 4096^3 4.35
+// ms (31.6 TFLOP/s; the packed path's GEMM alone 4.15 ms).  Below about a
+// thousand tiles the last wave and one or two CTAs an SM are what is lost.
 #include <algorithm>
 
 #include "common.cuh"
@@ -39,10 +45,11 @@ __device__ __forceinline__ int axis_off(const int32_t* __restrict__ tab, int32_t
   return t < 0 ? i * str : __ldg(tab + t + i);
 }
 
-// 8-byte asynchronous copy; ok = false writes a zero without reading
+// 8-byte asynchronous copy; ok = false writes a zero without reading.  No
+// memory clobber: it fills a stage that no fragment load touches before the
+// next barrier, so the two may be interleaved.
 __device__ __forceinline__ void cp8(double* dst, const double* src, bool ok) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 8 : 0)
-               : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 8 : 0));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -91,32 +98,78 @@ struct Operand {
       off[i] = r < rows ? axis_off(tab, rt, rs, row0 + r) : -1;  // -1: past the block, not loaded
     }
   }
-  __device__ __forceinline__ void load(double* s, const int32_t* tab, int k0, int K) const {
+  // quarter Q of the tile's elements (Q = 4: all of them)
+  // TAB: the K axis is a table (several legs that do not merge), else a stride
+  template <bool TAB, int Q>
+  __device__ __forceinline__ void load_as(double* s, const int32_t* tab, int k0, int K) const {
     if constexpr (KF) {
       const int kk = threadIdx.x & 15;
       const bool ok = k0 + kk < K;
-      const int ko = ok ? axis_off(tab, kt, ks, k0 + kk) : 0;
+      const int ko = ok ? (TAB ? __ldg(tab + kt + k0 + kk) : (k0 + kk) * ks) : 0;
+      double* d = s + (threadIdx.x >> 4) * BK + (kk ^ (((threadIdx.x >> 4) & 3) << 2));
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        const int r = (static_cast<int>(threadIdx.x) >> 4) + 8 * i;
-        if (off[i] >= 0) cp8(s + r * BK + (kk ^ ((r & 3) << 2)), base + (off[i] + ko), ok);
-      }
+      for (int i = 0; i < kPer; ++i)
+        if ((Q == 4 || (i & 3) == Q) && off[i] >= 0) cp8(d + i * 8 * BK, base + (off[i] + ko), ok);
     } else {
-      const int r = static_cast<int>(threadIdx.x) % R;
+      const int r = static_cast<int>(threadIdx.x) % R, q = static_cast<int>(threadIdx.x) / R;
       if (off[0] < 0) return;
+      double* d = s + q * (R + 4) + r;
 #pragma unroll
       for (int i = 0; i < kPer; ++i) {
-        const int kk = static_cast<int>(threadIdx.x) / R + i * (THREADS / R);
-        const bool ok = k0 + kk < K;
-        const int ko = ok ? axis_off(tab, kt, ks, k0 + kk) : 0;
-        cp8(s + kk * (R + 4) + r, base + (off[0] + ko), ok);
+        if (Q != 4 && (i & 3) != Q) continue;
+        const int kk = k0 + q + i * (THREADS / R);
+        const bool ok = kk < K;
+        const int ko = ok ? (TAB ? __ldg(tab + kt + kk) : kk * ks) : 0;
+        cp8(d + i * (THREADS / R) * (R + 4), base + (off[0] + ko), ok);
       }
     }
+  }
+  template <int Q>
+  __device__ __forceinline__ void load(double* s, const int32_t* tab, int k0, int K) const {
+    if (kt < 0)
+      load_as<false, Q>(s, tab, k0, K);
+    else
+      load_as<true, Q>(s, tab, k0, K);
   }
   static __device__ __forceinline__ double frag(const double* s, int r, int kk) {
     return KF ? s[r * BK + (kk ^ ((r & 3) << 2))] : s[kk * (R + 4) + r];
   }
 };
+
+// One 4-deep K step of a warp with MV x NV valid fragments.  The counts are
+// compile-time: guarding each DMMA at run time cost 10 issued instructions per
+// DMMA against 4 and held the 6400 x 256 x 1024 product at 53 % of the pipe.
+template <int MV, int NV, int WM, int WN, class OpA, class OpB, int MI, int NI>
+__device__ __forceinline__ void products(double (&acc)[MI][NI][2], const double* as, const double* bs, int wm, int wn,
+                                         int lane, int k4) {
+  {
+    const int kk = k4 * 4 + (lane & 3);
+    double af[MV], bf[NV];
+#pragma unroll
+    for (int i = 0; i < MV; ++i) af[i] = OpA::frag(as, (i * WM + wm) * 8 + (lane >> 2), kk);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) bf[j] = OpB::frag(bs, (j * WN + wn) * 8 + (lane >> 2), kk);
+#pragma unroll
+    for (int i = 0; i < MV; ++i)
+#pragma unroll
+      for (int j = 0; j < NV; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+  }
+}
+template <int MV, int WM, int WN, class OpA, class OpB, int MI, int NI>
+__device__ __forceinline__ void products_n(double (&acc)[MI][NI][2], const double* as, const double* bs, int wm,
+                                           int wn, int lane, int nv, int n4) {
+  if constexpr (MV <= MI) {
+    for (int k4 = 0; k4 < n4; ++k4) {
+      if (nv == 1) products<MV, 1, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, k4);
+      if constexpr (NI >= 2)
+        if (nv == 2) products<MV, 2, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, k4);
+      if constexpr (NI >= 4) {
+        if (nv == 3) products<MV, 3, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, k4);
+        if (nv == 4) products<MV, 4, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, k4);
+      }
+    }
+  }
+}
 
 template <int BM, int BN, bool AK, bool BKF>
 constexpr int smem_doubles() {
@@ -129,7 +182,7 @@ template <int BM, int BN, int WM, int WN, bool AK, bool BKF>
 __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     contract_f64_kernel(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
                         const ContractTile* __restrict__ tiles, const ContractSpan* __restrict__ spans,
-                        const int32_t* __restrict__ tab, int split) {
+                        const int32_t* __restrict__ tab, int split, int parts, double* __restrict__ ws) {
   static_assert(WM * WN == 4, "four warps");
   constexpr int MI = BM / 8 / WM, NI = BN / 8 / WN;
   using OpA = Operand<BM, AK>;
@@ -140,15 +193,16 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
   double* Bs = ring + STAGES * OpA::kTile;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp / WN, wn = warp % WN;
-  const int rank = static_cast<int>(blockIdx.x) % split;
-  const ContractTile t = tiles[blockIdx.x / split];
+  const int rank = static_cast<int>(blockIdx.x) % split, part = static_cast<int>(blockIdx.x) / split % parts;
+  const ContractTile t = tiles[blockIdx.x / (split * parts)];
   for (int i = tid; i < t.nspan * 4 && i < kSmemSpans * 4; i += THREADS)
     reinterpret_cast<int4*>(sspan)[i] = __ldg(reinterpret_cast<const int4*>(spans + t.span0) + i);
   __syncthreads();
   const int rows = min(BM, t.M - t.m0), cols = min(BN, t.N - t.n0);
-  // this CTA's K tiles: an even share of the cluster's
-  const int kt0 = static_cast<int>(static_cast<int64_t>(t.ktiles) * rank / split);
-  const int nkt = static_cast<int>(static_cast<int64_t>(t.ktiles) * (rank + 1) / split) - kt0;
+  // this CTA's K tiles: an even share of the output tile's
+  const int share = part * split + rank, shares = split * parts;
+  const int kt0 = static_cast<int>(static_cast<int64_t>(t.ktiles) * share / shares);
+  const int nkt = static_cast<int>(static_cast<int64_t>(t.ktiles) * (share + 1) / shares) - kt0;
   // valid fragments of this warp, dealt cyclically
   const int mv = ((rows + 7) / 8 - wm + WM - 1) / WM, nv = ((cols + 7) / 8 - wn + WN - 1) / WN;
 
@@ -172,7 +226,8 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     k0 = skip * BK;
   }
   uint32_t steps = 0;  // 4-deep K steps of each stage, one byte a stage
-  auto issue = [&](int s) {
+  // the next K tile's span, before its loads; then past it, after them
+  auto begin = [&](int s) {
     if (fresh) {
       const ContractSpan g = sp < kSmemSpans ? sspan[sp] : spans[t.span0 + sp];
       K = g.K;
@@ -180,16 +235,22 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
       ob.set_span(B + g.b_off, tab, g.br_tab, g.br_str, g.bk_tab, g.bk_str, t.n0, cols);
       fresh = false;
     }
-    oa.load(As + s * OpA::kTile, tab, k0, K);
-    ob.load(Bs + s * OpB::kTile, tab, k0, K);
     const uint32_t n4 = static_cast<uint32_t>((min(BK, K - k0) + 3) / 4);
     steps = (steps & ~(0xffu << (8 * s))) | (n4 << (8 * s));
+  };
+  auto finish = [&]() {
     k0 += BK;
     if (k0 >= K) {
       k0 = 0;
       ++sp;
       fresh = true;
     }
+  };
+  auto issue = [&](int s) {
+    begin(s);
+    oa.template load<4>(As + s * OpA::kTile, tab, k0, K);
+    ob.template load<4>(Bs + s * OpB::kTile, tab, k0, K);
+    finish();
   };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -199,29 +260,23 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
   for (int kt = 0; kt < nkt; ++kt) {
     cp_wait<STAGES - 2>();
     __syncthreads();
-    const int s = kt % STAGES;
+    const int s = kt % STAGES, sn = (kt + STAGES - 1) % STAGES;
     const int n4 = static_cast<int>((steps >> (8 * s)) & 0xffu);
-    if (kt + STAGES - 1 < nkt) issue((kt + STAGES - 1) % STAGES);
-    cp_commit();
+    const bool more = kt + STAGES - 1 < nkt;
     const double* as = As + s * OpA::kTile;
     const double* bs = Bs + s * OpB::kTile;
+    if (more) issue(sn);
+    cp_commit();
+    if (mv == MI && nv == NI && n4 == BK / 4) {
 #pragma unroll
-    for (int k4 = 0; k4 < BK / 4; ++k4) {
-      if (k4 >= n4) break;
-      const int kk = k4 * 4 + (lane & 3);
-      double af[MI], bf[NI];
-#pragma unroll
-      for (int i = 0; i < MI; ++i) af[i] = OpA::frag(as, (i * WM + wm) * 8 + (lane >> 2), kk);
-#pragma unroll
-      for (int j = 0; j < NI; ++j) bf[j] = OpB::frag(bs, (j * WN + wn) * 8 + (lane >> 2), kk);
-#pragma unroll
-      for (int i = 0; i < MI; ++i) {
-        if (i >= mv) break;
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-          if (j >= nv) break;
-          dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
-        }
+      for (int k4 = 0; k4 < BK / 4; ++k4) products<MI, NI, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, k4);
+    } else {
+      switch (mv) {
+        case 1: products_n<1, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, nv, n4); break;
+        case 2: products_n<2, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, nv, n4); break;
+        case 3: products_n<3, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, nv, n4); break;
+        case 4: products_n<4, WM, WN, OpA, OpB>(acc, as, bs, wm, wn, lane, nv, n4); break;
+        default: break;  // no valid row fragment
       }
     }
   }
@@ -259,6 +314,7 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
   cluster_sync();
   const int mine = (rows - rank + split - 1) / split;  // rows rank, rank + split, ...
   const bool rfast = t.c_str != 1 && t.r_str == 1;     // lanes along whichever axis the output has contiguous
+  double* wpart = parts > 1 ? ws + static_cast<int64_t>(blockIdx.x / split) * (BM * BN) : nullptr;
   for (int e = tid; e < mine * cols; e += THREADS) {
     const int q = rfast ? e % mine : e / cols;
     const int c = rfast ? e / mine : e - q * cols;
@@ -266,9 +322,27 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     const uint32_t sa = smem_u32(ring + r * P + c);
     double v = ld_peer(sa, 0);
     for (int p = 1; p < split; ++p) v += ld_peer(sa, p);
-    out[axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v;
+    if (parts > 1)
+      wpart[r * BN + c] = v;
+    else
+      out[axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v;
   }
   cluster_sync();  // no CTA leaves while a peer reads its shared memory
+}
+
+// The parts of every output tile added in order (a K too long for one cluster).
+__global__ void __launch_bounds__(256)
+    contract_parts_kernel(const double* __restrict__ ws, double* __restrict__ C, const ContractTile* __restrict__ tiles,
+                          const int32_t* __restrict__ tab, int parts, int bm, int bn) {
+  const ContractTile t = tiles[blockIdx.x];
+  const int rows = min(bm, t.M - t.m0), cols = min(bn, t.N - t.n0);
+  const double* w = ws + static_cast<int64_t>(blockIdx.x) * parts * bm * bn;
+  for (int e = blockIdx.y * 256 + threadIdx.x; e < rows * cols; e += gridDim.y * 256) {
+    const int r = e / cols, c = e - r * cols;
+    double v = 0.0;
+    for (int p = 0; p < parts; ++p) v += w[static_cast<int64_t>(p) * bm * bn + r * bn + c];
+    C[t.out_off + axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v;
+  }
 }
 
 template <int BM, int BN, int WM, int WN, bool AK, bool BKF>
@@ -278,7 +352,7 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(L.n_tiles) * L.split);
+  cfg.gridDim = dim3(static_cast<unsigned>(L.n_tiles) * L.split * L.parts);
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -291,7 +365,24 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
   }
-  return cudaLaunchKernelEx(&cfg, kernel, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split);
+  double* ws = nullptr;
+  if (L.parts > 1) {
+    // partial tiles of this call, from the stream-ordered pool: safe with any
+    // number of streams and threads, returned as soon as the sum is queued
+    e = cudaMallocAsync(&ws, sizeof(double) * BM * BN * static_cast<size_t>(L.n_tiles) * L.parts, st);
+    if (e != cudaSuccess) return e;
+  }
+  e = cudaLaunchKernelEx(&cfg, kernel, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws);
+  if (L.parts > 1) {
+    if (e == cudaSuccess) {
+      contract_parts_kernel<<<dim3(L.n_tiles, (BM * BN + 255) / 256), 256, 0, st>>>(ws, L.c, L.tiles, L.tab, L.parts,
+                                                                                  BM, BN);
+      e = cudaGetLastError();
+    }
+    const cudaError_t f = cudaFreeAsync(ws, st);
+    if (e == cudaSuccess) e = f;
+  }
+  return e;
 }
 
 template <int BM, int BN, int WM, int WN>
@@ -303,9 +394,9 @@ cudaError_t go_layout(const ContractLaunch& L, cudaStream_t st) {
 struct Shape {
   int bm, bn, wm, wn, resident;
 };
-// 64 x 64: the DMMA-bound shape; 32 x 32: few tiles or small blocks; 128 x 16:
-// narrow column blocks (an MPO leg), whose rows are many
-constexpr Shape kShapes[kContractShapes] = {{64, 64, 2, 2, 3}, {32, 32, 2, 2, 4}, {128, 16, 4, 1, 3}};
+// 64 x 64: the DMMA-bound shape; 64 x 32 and 32 x 32: few tiles or small
+// blocks; 128 x 16: narrow column blocks (an MPO leg), whose rows are many
+constexpr Shape kShapes[kContractShapes] = {{64, 64, 2, 2, 3}, {32, 32, 2, 2, 4}, {128, 16, 4, 1, 3}, {64, 32, 2, 2, 4}};
 }  // namespace
 
 void contract_tile_shape(int shape, int* bm, int* bn) {
@@ -313,17 +404,17 @@ void contract_tile_shape(int shape, int* bm, int* bn) {
   *bn = kShapes[shape].bn;
 }
 
-// Estimated clocks of a step for every (tile shape, K split); the smallest
-// wins.  Per CTA: the longest warp's DMMA chain (16 clocks each) or its
-// operand loads (about 48 bytes a clock and SM), and a fixed 2500 clocks of
-// table reads, ring fill and stores, overlapped over the resident CTAs; a
-// split adds 2000 clocks for its exchange.  Fitted to: 80 x 80 x 1280 in
-// 64 x 64 tiles without a split 48 us, and the 6400 x 256 x 256 product 30 us.
-void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split) {
+// Estimated clocks of a step for every tile shape and number of K shares (up
+// to 8 in one cluster, beyond that parts of 8 summed by a second launch); the
+// smallest wins.  Per CTA: the longest warp's DMMA chain (16 clocks each), its
+// operand loads (about 48 bytes a clock and SM), and at least 270 clocks a K
+// tile (the latency of a load over the ring's depth).  One CTA on an SM keeps
+// about 0.6 of its tensor pipes busy, three 0.9.
+void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split, int* parts) {
   double best = -1.0;
   *shape = 0;
-  *split = 1;
-  for (int s = 0; s < kContractShapes; ++s) {
+  *split = *parts = 1;
+  for (int s : {1, 3, 2, 0}) {  // the smallest tile of equal estimates
     const Shape& h = kShapes[s];
     double sum = 0.0, longest = 0.0;
     int64_t n = 0, kmax = 0;
@@ -338,7 +429,7 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape,
         const double mem = static_cast<double>((r + c) * b.ktiles) * 16.0 * 8.0 / 48.0;
         const double x = std::max(mma, mem);
         sum += static_cast<double>(count) * x;
-        longest = std::max(longest, x);
+        longest = std::max(longest, std::max(x / 0.6, 270.0 * static_cast<double>(b.ktiles)));
         n += count;
       };
       add(fm * fn, h.bm, h.bn);
@@ -346,15 +437,19 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape,
       add(fm, h.bm, en);
       add(em > 0 && en > 0 ? 1 : 0, em, en);
     }
-    for (int sp = 1; sp <= 8; sp *= 2) {
+    for (int sp = 1; sp <= 256; sp *= 2) {
       if (sp > 1 && kmax < 2 * sp) break;
-      const double over = 2500.0 + (sp > 1 ? 2000.0 : 0.0);
-      const double waves = std::max(1.0, static_cast<double>(n * sp) / (static_cast<double>(n_sm) * h.resident));
-      const double est = std::max(sum / n_sm, longest / sp) + over * waves;
+      const double ctas = static_cast<double>(n * sp);
+      const double per_sm = std::min(static_cast<double>(h.resident), std::max(1.0, ctas / n_sm));
+      const double eff = std::min(0.9, 0.45 + 0.15 * per_sm);
+      const double over = 2500.0 + (sp > 1 ? 1500.0 : 0.0);
+      const double waves = std::max(1.0, ctas / (static_cast<double>(n_sm) * h.resident));
+      const double est = std::max(sum / n_sm / eff, longest / sp) + over * waves + (sp > 8 ? 6000.0 : 0.0);
       if (best < 0.0 || est < best) {
         best = est;
         *shape = s;
-        *split = sp;
+        *split = std::min(sp, 8);
+        *parts = sp / *split;
       }
     }
   }
@@ -365,7 +460,8 @@ cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st) {
   switch (L.shape) {
     case 0: return go_layout<64, 64, 2, 2>(L, st);
     case 1: return go_layout<32, 32, 2, 2>(L, st);
-    default: return go_layout<128, 16, 4, 1>(L, st);
+    case 2: return go_layout<128, 16, 4, 1>(L, st);
+    default: return go_layout<64, 32, 2, 2>(L, st);
   }
 }
 

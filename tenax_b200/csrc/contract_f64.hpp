@@ -38,13 +38,14 @@ struct ContractLaunch {
   const ContractTile* tiles;
   const ContractSpan* spans;
   const int32_t* tab;
-  int n_tiles, shape, split;
+  int n_tiles, shape;
+  int split, parts;  // K shares of one cluster, and clusters per output tile
   bool a_kfast, b_kfast;  // whether K is the fast axis of the operand's blocks
 };
 
-constexpr int kContractShapes = 3;
+constexpr int kContractShapes = 4;
 void contract_tile_shape(int shape, int* bm, int* bn);
-void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split);
+void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split, int* parts);
 cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st);
 
 }  // namespace tnx
