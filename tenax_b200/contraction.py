@@ -18,15 +18,12 @@ import numpy as np
 import torch
 
 from tenax_b200 import _capi
-from tenax_b200.tensor import SymmetricTensor, _device
+from tenax_b200.tensor import SymmetricTensor, make_layout
+from tenax_b200.vector import _stream_ptr
 
 _PLANS: "OrderedDict[tuple, Plan]" = OrderedDict()
 _PLAN_CACHE_SIZE = 512
 DEFAULT_PRECISION = "fp64"
-
-
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 class Plan:
@@ -56,13 +53,19 @@ class Plan:
         self.total = tot.value
         self.target = tgt.value if has_t.value else None
         self.flops = float(_capi.LIB.tnx_plan_flops(h))
+        # the result's layout depends on the plan's structure alone
+        self.layout = make_layout(out_indices, self.out_keys)
+
+    def wrap(self, out_indices, data: torch.Tensor) -> SymmetricTensor:
+        """The result over ``out_indices`` (the charges this plan was made for)."""
+        return SymmetricTensor.from_layout(out_indices, self.layout, data)
 
     def execute(self, tensors, precision: str) -> torch.Tensor:
-        out = torch.empty(max(1, self.total), dtype=torch.float64, device=_device())
+        out = torch.empty(max(1, self.total), dtype=torch.float64, device="cuda")
         ptrs = (C.c_void_p * max(1, len(tensors)))(*[t.data.data_ptr() for t in tensors])
         _capi.check(_capi.LIB.tnx_plan_execute(self.handle, ptrs, out.data_ptr(), _capi.PRECISIONS[precision], None,
                                                0, _stream_ptr()))
-        return out[: self.total]
+        return out if self.total else out[:0]
 
     def __del__(self):
         if getattr(self, "handle", None) and _capi is not None and _capi.LIB is not None:
@@ -86,7 +89,7 @@ def _structure_key(tensors, in_subs, out_subs, mode, out_indices, fermionic=Fals
     parts = [mode, out_subs, bool(fermionic)]
     for t, s in zip(tensors, in_subs):
         parts.append((s, tuple(int(i.flow) for i in t.indices), tuple(i.charges.tobytes() for i in t.indices),
-                      tuple(t.keys)))
+                      t._layout.keys))
     parts.append(tuple((int(i.flow), i.charges.tobytes()) for i in out_indices))
     return tuple(parts)
 
@@ -153,7 +156,7 @@ def _contract_symmetric(tensors, subscripts, output_indices=None, precision=None
     # fermionic operands: the exchange sign of the leg reordering (contractor.py:460-470)
     plan = get_plan(tensors, in_subs, out_subs, _capi.MATCH_FILTERED, out_indices, _fermionic(tensors))
     data = plan.execute(tensors, precision or DEFAULT_PRECISION)
-    out = SymmetricTensor.from_flat(out_indices, plan.out_keys, data)
+    out = plan.wrap(out_indices, data)
     if plan.target is None:
         out._validate()
     return out
@@ -165,7 +168,7 @@ def blockwise_contract(tensors, subscripts, output_indices, precision=None) -> S
     in_subs = lhs.split(",")
     plan = get_plan(tensors, in_subs, out_subs, _capi.MATCH_UNFILTERED, tuple(output_indices))
     data = plan.execute(tensors, precision or DEFAULT_PRECISION)
-    return SymmetricTensor.from_flat(tuple(output_indices), plan.out_keys, data)
+    return plan.wrap(tuple(output_indices), data)
 
 
 def transpose_symmetric(t: SymmetricTensor, axes) -> SymmetricTensor:
@@ -177,7 +180,7 @@ def transpose_symmetric(t: SymmetricTensor, axes) -> SymmetricTensor:
     lhs, out_subs = sub.split("->")
     plan = get_plan([t], [lhs], out_subs, _capi.MATCH_UNFILTERED, new_idx, _fermionic([t]))
     data = plan.execute([t], DEFAULT_PRECISION)
-    return SymmetricTensor.from_flat(new_idx, plan.out_keys, data)
+    return plan.wrap(new_idx, data)
 
 
 def contract_with_subscripts(tensors, subscripts, output_indices, optimize="auto", precision=None):
@@ -213,6 +216,8 @@ def _onto_keys(t: SymmetricTensor, keys) -> torch.Tensor:
     from tenax_b200.tensor import embed_in_keys, restrict_to_keys
 
     keys = sorted(keys)
+    if keys == t.keys:
+        return t.data
     common = sorted(set(t.keys) & set(keys))
     return embed_in_keys(restrict_to_keys(t, common), keys).data
 
@@ -226,32 +231,32 @@ class _SymContract(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, spec, a_data, b_data):
-        a_idx, a_keys, b_idx, b_keys, subs, out_idx, filtered, precision = spec
-        a = SymmetricTensor.from_flat(a_idx, a_keys, a_data)
-        b = SymmetricTensor.from_flat(b_idx, b_keys, b_data)
+        a_idx, a_lay, b_idx, b_lay, subs, out_idx, filtered, precision = spec
+        a = SymmetricTensor.from_layout(a_idx, a_lay, a_data)
+        b = SymmetricTensor.from_layout(b_idx, b_lay, b_data)
         if filtered:
             out = _contract_symmetric([a, b], subs, out_idx, precision)
         else:
             out = blockwise_contract([a, b], subs, out_idx, precision)
         ctx.spec = spec
-        ctx.out_keys = out.keys
+        ctx.out_layout = out._layout
         ctx.save_for_backward(a_data, b_data)
         return out.data
 
     @staticmethod
     def backward(ctx, g):
-        a_idx, a_keys, b_idx, b_keys, subs, out_idx, _, precision = ctx.spec
+        a_idx, a_lay, b_idx, b_lay, subs, out_idx, _, precision = ctx.spec
         a_data, b_data = ctx.saved_tensors
         lhs, so = subs.split("->")
         sa, sb = lhs.split(",")
-        gc = SymmetricTensor.from_flat(out_idx, ctx.out_keys, g.contiguous())
+        gc = SymmetricTensor.from_layout(out_idx, ctx.out_layout, g.contiguous())
         ga = gb = None
         if ctx.needs_input_grad[1]:
-            b = SymmetricTensor.from_flat(b_idx, b_keys, b_data)
-            ga = _onto_keys(blockwise_contract([gc, b], f"{so},{sb}->{sa}", a_idx, precision), a_keys)
+            b = SymmetricTensor.from_layout(b_idx, b_lay, b_data)
+            ga = _onto_keys(blockwise_contract([gc, b], f"{so},{sb}->{sa}", a_idx, precision), a_lay.keys)
         if ctx.needs_input_grad[2]:
-            a = SymmetricTensor.from_flat(a_idx, a_keys, a_data)
-            gb = _onto_keys(blockwise_contract([a, gc], f"{sa},{so}->{sb}", b_idx, precision), b_keys)
+            a = SymmetricTensor.from_layout(a_idx, a_lay, a_data)
+            gb = _onto_keys(blockwise_contract([a, gc], f"{sa},{so}->{sb}", b_idx, precision), b_lay.keys)
         return None, ga, gb
 
 
@@ -268,10 +273,9 @@ def contract_ad(a: SymmetricTensor, b: SymmetricTensor, output_labels=None, prec
     for s, other in ((sa, sb + so), (sb, sa + so)):
         if any(c not in other for c in s):
             raise TnxUnsupportedAD(f"'{subscripts}': a leg summed within one operand has no adjoint here")
-    spec = (a.indices, a.keys, b.indices, b.keys, subscripts, tuple(out_idx), True, precision)
+    spec = (a.indices, a._layout, b.indices, b._layout, subscripts, tuple(out_idx), True, precision)
     data = _SymContract.apply(spec, a.data, b.data)
-    probe = get_plan([a, b], [sa, sb], so, _capi.MATCH_FILTERED, tuple(out_idx))
-    return SymmetricTensor.from_flat(tuple(out_idx), probe.out_keys, data)
+    return get_plan([a, b], [sa, sb], so, _capi.MATCH_FILTERED, tuple(out_idx)).wrap(tuple(out_idx), data)
 
 
 class TnxUnsupportedAD(NotImplementedError):

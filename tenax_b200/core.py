@@ -223,7 +223,7 @@ class TensorIndex:
     def charge_dims(self) -> dict:
         """Multiplicity of each charge on this leg."""
         u, c = np.unique(self.charges, return_counts=True)
-        return {int(q): int(n) for q, n in zip(u, c)}
+        return dict(zip(u.tolist(), c.tolist()))
 
     def __eq__(self, other):
         if not isinstance(other, TensorIndex):

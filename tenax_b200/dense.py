@@ -50,14 +50,18 @@ class _DensePlan:
         self.precision = _capi.PRECISIONS[precision]
         self.flops = float(_capi.LIB.tnx_plan_flops(h))
         self.n_in = len(shapes)
+        self.ptr_array = C.c_void_p * self.n_in
 
     def __call__(self, *tensors):
-        out = torch.empty(self.out_shape, dtype=torch.float64, device=tensors[0].device)
+        dev = tensors[0].device
+        out = torch.empty(self.out_shape, dtype=torch.float64, device=dev)
         if out.numel() == 0:
             return out
-        ptrs = (C.c_void_p * self.n_in)(*[t.data_ptr() for t in tensors])
-        _capi.check(_capi.LIB.tnx_plan_execute(self.handle, ptrs, out.data_ptr(), self.precision, None, 0,
-                                               torch.cuda.current_stream(out.device).cuda_stream))
+        ptrs = self.ptr_array(*[t.data_ptr() for t in tensors])
+        st = _capi.LIB.tnx_plan_execute(self.handle, ptrs, out.data_ptr(), self.precision, None, 0,
+                                        torch._C._cuda_getCurrentRawStream(dev.index))
+        if st:
+            _capi.check(st)
         return out
 
     def __del__(self):

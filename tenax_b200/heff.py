@@ -25,6 +25,7 @@ import torch
 
 from tenax_b200 import _capi
 from tenax_b200.tensor import SymmetricTensor
+from tenax_b200.vector import _stream_ptr
 
 
 def _desc(t_indices, keys):
@@ -212,7 +213,7 @@ class HeffBatch:
     def apply(self, thetas, outs):
         tp = (C.c_void_p * len(thetas))(*[t.data_ptr() for t in thetas])
         op = (C.c_void_p * len(outs))(*[o.data_ptr() for o in outs])
-        _capi.check(_capi.LIB.tnx_heff_batch_apply(self.handle, tp, op, torch.cuda.current_stream().cuda_stream))
+        _capi.check(_capi.LIB.tnx_heff_batch_apply(self.handle, tp, op, _stream_ptr()))
 
     def route_stats(self) -> tuple:
         """(route records, largest window of records one epilogue warp scans

@@ -10,15 +10,18 @@ host-side key list and offset table; ``.blocks`` exposes per-key views.
 
 from __future__ import annotations
 
-from typing import Any
+import math
+from typing import Any, NamedTuple
 
 import numpy as np
 import torch
 
 from tenax_b200 import _capi
-from tenax_b200.core import TensorIndex
+from tenax_b200.core import FermionicU1, FermionParity, TensorIndex, U1Symmetry, ZnSymmetry
 
 BlockKey = tuple
+# symmetries whose charges fuse by addition, modulo n_values() where it is set
+_INTEGER_FUSE = (U1Symmetry, ZnSymmetry, FermionParity, FermionicU1)
 
 
 def _device() -> torch.device:
@@ -35,6 +38,28 @@ def block_shape(indices, key) -> tuple:
     return tuple(int(np.count_nonzero(idx.charges == q)) for idx, q in zip(indices, key))
 
 
+class Layout(NamedTuple):
+    """Where a tensor's blocks lie in its flat buffer.  Equal legs and keys
+    have equal layouts, so tensors of one structure share it (nothing writes
+    to one after it is built)."""
+
+    keys: tuple
+    offsets: np.ndarray
+    shapes: list
+    key_pos: dict
+
+
+def make_layout(indices, keys) -> Layout:
+    """Layout of the blocks ``keys`` (in this order): the multiplicities are
+    counted once per leg, not once per block and leg."""
+    dims = [idx.charge_dims() for idx in indices]
+    shapes = [tuple(d.get(q, 0) for d, q in zip(dims, k)) for k in keys]
+    offs = np.zeros(len(keys) + 1, dtype=np.int64)
+    if shapes:
+        offs[1:] = np.cumsum([math.prod(s) for s in shapes])
+    return Layout(tuple(keys), offs, shapes, {k: i for i, k in enumerate(keys)})
+
+
 def compute_valid_blocks(indices, target=None):
     """Valid keys in the reference's order (core/tensor.py:53-165), via the planner."""
     if not indices:
@@ -45,7 +70,7 @@ def compute_valid_blocks(indices, target=None):
 class SymmetricTensor:
     """Block-sparse tensor; blocks in one flat CUDA float64 buffer."""
 
-    __slots__ = ("_indices", "_keys", "_data", "_offsets", "_shapes", "_key_pos", "_blocks_cache")
+    __slots__ = ("_indices", "_keys", "_data", "_offsets", "_shapes", "_key_pos", "_blocks_cache", "_layout")
 
     def __init__(self, blocks: dict, indices, _validate: bool = True):
         indices = tuple(indices)
@@ -63,32 +88,45 @@ class SymmetricTensor:
 
     # ------------------------------------------------------------ construction
     def _init_flat(self, indices, keys, data):
+        self._init_layout(indices, make_layout(tuple(indices), keys), data)
+
+    def _init_layout(self, indices, layout: Layout, data):
+        if data.numel() != int(layout.offsets[-1]):
+            raise ValueError(f"flat buffer has {data.numel()} elements, blocks need {int(layout.offsets[-1])}")
         self._indices = tuple(indices)
-        self._keys = list(keys)
-        shapes = [block_shape(self._indices, k) for k in self._keys]
-        sizes = [int(np.prod(s)) if s else 1 for s in shapes]
-        offs = np.zeros(len(keys) + 1, dtype=np.int64)
-        if sizes:
-            offs[1:] = np.cumsum(sizes)
-        if data.numel() != int(offs[-1]):
-            raise ValueError(f"flat buffer has {data.numel()} elements, blocks need {int(offs[-1])}")
+        self._layout = layout
+        self._keys = list(layout.keys)
         self._data = data
-        self._offsets = offs
-        self._shapes = shapes
-        self._key_pos = {k: i for i, k in enumerate(self._keys)}
+        self._offsets = layout.offsets.copy()
+        self._shapes = layout.shapes
+        self._key_pos = layout.key_pos
         self._blocks_cache = None
 
     @classmethod
     def from_flat(cls, indices, keys, data: torch.Tensor) -> "SymmetricTensor":
         """Wrap an existing flat buffer (blocks in the given sorted key order)."""
         obj = object.__new__(cls)
-        obj._init_flat(indices, [tuple(int(q) for q in k) for k in keys], data)
+        obj._init_flat(indices, [tuple(map(int, k)) for k in keys], data)
+        return obj
+
+    @classmethod
+    def from_layout(cls, indices, layout: Layout, data: torch.Tensor) -> "SymmetricTensor":
+        """Wrap a flat buffer whose layout is known (``indices`` must have the
+        charges it was made for)."""
+        obj = object.__new__(cls)
+        obj._init_layout(indices, layout, data)
         return obj
 
     def _validate(self):
         if not self._indices:
             return
         sym = self._indices[0].symmetry
+        if type(sym) in _INTEGER_FUSE and self._keys and len(self._indices) > 1:
+            # charges that add (mod n): every block in one product
+            tot = np.array(self._keys, dtype=np.int64) @ np.array([int(i.flow) for i in self._indices], np.int64)
+            n = sym.n_values()
+            if not np.any(tot % n if n is not None else tot):
+                return
         for key in self._keys:
             eff = [int(i.flow) * int(q) for i, q in zip(self._indices, key)]
             fused = sym.fuse_many(eff)
@@ -238,7 +276,8 @@ class SymmetricTensor:
 
     # ------------------------------------------------------------ algebra
     def _like(self, data, indices=None) -> "SymmetricTensor":
-        return SymmetricTensor.from_flat(self._indices if indices is None else indices, self._keys, data)
+        # ``indices`` replaces labels or flows only: the layout stays
+        return SymmetricTensor.from_layout(self._indices if indices is None else indices, self._layout, data)
 
     def conj(self) -> "SymmetricTensor":
         return self._like(self._data)  # real float64 data

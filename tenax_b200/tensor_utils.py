@@ -18,7 +18,7 @@ import torch
 
 from tenax_b200 import _capi
 from tenax_b200.core import FlowDirection, TensorIndex
-from tenax_b200.tensor import SymmetricTensor
+from tenax_b200.tensor import SymmetricTensor, make_layout
 
 _PLANS: "OrderedDict[tuple, _FusePlan]" = OrderedDict()
 _PLAN_CACHE_SIZE = 256
@@ -43,6 +43,8 @@ class _FusePlan:
         self.fused_charges = self.fused_charges[: nf.value]
         self.out_keys = [tuple(int(q) for q in r) for r in keys[: nb.value * nl].reshape(-1, nl)]
         self.total = tot.value
+        # the result's layout, made with the first result's legs
+        self.layout = None
 
     def __del__(self):
         if getattr(self, "handle", None) and _capi is not None and _capi.LIB is not None:
@@ -89,8 +91,10 @@ def fuse_indices(tensor: SymmetricTensor, axis_a: int, axis_b: int, fused_label,
     out = torch.empty(max(1, plan.total), dtype=torch.float64, device=tensor.data.device)
     if plan.total:
         _capi.check(_capi.LIB.tnx_fuse_execute(plan.handle, tensor.data.data_ptr(), out.data_ptr(),
-                                               torch.cuda.current_stream(out.device).cuda_stream))
-    return SymmetricTensor.from_flat(new_indices, plan.out_keys, out[: plan.total])
+                                               torch._C._cuda_getCurrentRawStream(out.device.index)))
+    if plan.layout is None:
+        plan.layout = make_layout(new_indices, plan.out_keys)
+    return SymmetricTensor.from_layout(new_indices, plan.layout, out[: plan.total])
 
 
 def fused_charges(tensor: SymmetricTensor, axis_a: int, axis_b: int, fused_flow) -> np.ndarray:

@@ -10,7 +10,9 @@ _SCRATCH: dict = {}
 
 
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream, without building a Stream object
+    (4 us a call in a loop of small launches)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def scratch(device=None) -> torch.Tensor:

@@ -1,0 +1,47 @@
+"""Block layouts counted once per leg, and the conservation check of all blocks at once."""
+
+import itertools
+import math
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from tenax_b200.core import (FermionicU1, FermionParity, FlowDirection, TensorIndex, U1Symmetry,  # noqa: E402
+                             ZnSymmetry)
+from tenax_b200.tensor import SymmetricTensor, block_shape, make_layout  # noqa: E402
+
+SYMS = [U1Symmetry(), ZnSymmetry(2), ZnSymmetry(3), FermionParity(), FermionicU1()]
+
+
+def _legs(sym, n):
+    rng = np.random.default_rng(n)
+    hi = sym.n_values() or 3
+    return tuple(TensorIndex(sym, rng.integers(0, hi, 3 + 2 * i).astype(np.int32),
+                             FlowDirection.IN if i % 2 else FlowDirection.OUT, f"l{i}") for i in range(n))
+
+
+@pytest.mark.parametrize("sym", SYMS, ids=repr)
+@pytest.mark.parametrize("n", [0, 1, 2, 4])
+def test_layout_matches_block_shapes(sym, n):
+    idx = _legs(sym, n)
+    keys = list(itertools.product(range(-1, 3), repeat=n))  # charges that no state carries among them
+    lay = make_layout(idx, keys)
+    assert lay.shapes == [block_shape(idx, k) for k in keys]
+    assert lay.offsets.tolist() == np.concatenate([[0], np.cumsum([math.prod(s) for s in lay.shapes])]).tolist()
+    assert [lay.key_pos[k] for k in keys] == list(range(len(keys)))
+
+
+@pytest.mark.parametrize("sym", SYMS, ids=repr)
+@pytest.mark.parametrize("n", [1, 2, 3])
+def test_validate_agrees_with_fuse_many(sym, n):
+    idx = _legs(sym, n)
+    for key in itertools.product(range(3), repeat=n):
+        t = SymmetricTensor.from_flat(idx, [key], torch.zeros(math.prod(block_shape(idx, key)), dtype=torch.float64))
+        fused = sym.fuse_many([int(i.flow) * q for i, q in zip(idx, key)])
+        if fused == sym.identity():
+            t._validate()
+        else:
+            with pytest.raises(ValueError, match="charge conservation"):
+                t._validate()
