@@ -633,6 +633,31 @@ bool k_is_fast(const std::vector<std::pair<int64_t, int64_t>>& r, const std::vec
   return sk < sr;
 }
 
+// Whether elements 2i and 2i + 1 of an operand's fast axis are adjacent and
+// every such pair starts on an even element, for every block: the innermost
+// fast leg has stride 1 and an even extent (an axis of one leg may end on a
+// single), every other stride and the block's offset are even.
+bool pairs_ok(int64_t off, const std::vector<std::pair<int64_t, int64_t>>& fast,
+              const std::vector<std::pair<int64_t, int64_t>>& slow) {
+  if (off % 2) return false;
+  for (const auto& l : slow)
+    if (l.first > 1 && l.second % 2) return false;
+  int64_t legs = 0, inner = 0;
+  for (const auto& l : fast)
+    if (l.first > 1) {
+      ++legs;
+      inner = l.second == 1 ? l.first : inner;
+    }
+  if (legs == 0) return true;  // a single element a row: read alone
+  if (inner == 0 || (legs > 1 && inner % 2)) return false;
+  for (const auto& l : fast)
+    if (l.first > 1 && l.second != 1 && l.second % 2) return false;
+  // the innermost leg in the walking order must be the adjacent one
+  for (size_t i = fast.size(); i-- > 0;)
+    if (fast[i].first > 1) return fast[i].second == 1;
+  return true;
+}
+
 // Tables of the one-launch FP64 kernel for one step.  It serves every step
 // whose blocks hold fewer than 2^31 elements (its in-block offsets are 32-bit)
 // and carry no fermionic sign; the others keep the packed path, which negates
@@ -679,7 +704,8 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     }
     return legs;
   };
-  auto index = [&](const std::vector<PackSeg>& segs, const std::string& subs) {
+  auto index = [&](const std::vector<PackSeg>& segs, const std::string& subs, bool kfast, bool* vec) {
+    *vec = true;
     std::map<std::pair<int32_t, int32_t>, std::map<int32_t, Side>> by;  // (group, row0) -> k0 -> block
     for (const auto& s : segs) {
       Side x;
@@ -689,11 +715,13 @@ bool build_direct(const PairPlan& P, StepDev& d) {
       x.k = extent_of(k);
       T.add(r, &x.rt, &x.rs);
       T.add(k, &x.kt, &x.ks);
+      *vec = *vec && pairs_ok(s.src_off, kfast ? k : r, kfast ? r : k);
       by[{s.group, s.row0}][s.k0] = x;
     }
     return by;
   };
-  const auto A = index(P.packA, P.a_subs), B = index(P.packB, P.b_subs);
+  bool a_vec = false, b_vec = false;
+  const auto A = index(P.packA, P.a_subs, a_kfast, &a_vec), B = index(P.packB, P.b_subs, b_kfast, &b_vec);
   // rows are the longer side of a tile (128 x 16)
   int64_t sm = 0, sn = 0;
   for (const auto& sc : P.scatter) {
@@ -708,6 +736,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     if (sc.count == 0) continue;
     ContractTile t{};
     ContractBlk blk{};
+    t.scale = 1.0;
     const auto r = axis_legs(sc.nlegs, sc.dims, sc.rstr), c = axis_legs(sc.nlegs, sc.dims, sc.cstr);
     t.out_off = sc.dst_off;
     t.M = static_cast<int32_t>(extent_of(r));
@@ -748,6 +777,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
   }
   if (d.swapped) {
     std::swap(a_kfast, b_kfast);
+    std::swap(a_vec, b_vec);
     for (auto& g : spans) {
       std::swap(g.a_off, g.b_off);
       std::swap(g.ar_tab, g.br_tab);
@@ -757,28 +787,13 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     }
   }
   ContractLaunch& L = d.dl;
-  contract_choose(blks, device_sm_count(), &L.shape, &L.split, &L.parts);
+  contract_choose(blks, device_sm_count(), 1, 256, &L.shape, &L.split, &L.parts);
   L.a_kfast = a_kfast;
   L.b_kfast = b_kfast;
-  int bm, bn;
-  contract_tile_shape(L.shape, &bm, &bn);
-  // longest tiles first
-  std::vector<std::pair<int64_t, ContractTile>> tl;
-  for (size_t i = 0; i < proto.size(); ++i)
-    for (int64_t m0 = 0; m0 < proto[i].M; m0 += bm)
-      for (int64_t n0 = 0; n0 < proto[i].N; n0 += bn) {
-        ContractTile t = proto[i];
-        t.m0 = static_cast<int32_t>(m0);
-        t.n0 = static_cast<int32_t>(n0);
-        const int64_t cost = blks[i].k4 * cdiv(std::min<int64_t>(bm, t.M - m0), 8) *
-                             cdiv(std::min<int64_t>(bn, t.N - n0), 8);
-        tl.push_back({cost, t});
-      }
-  if (static_cast<int64_t>(tl.size()) * L.split * L.parts > INT32_MAX) return false;
-  std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-  std::vector<ContractTile> tiles;
-  tiles.reserve(tl.size());
-  for (const auto& x : tl) tiles.push_back(x.second);
+  L.a_vec = a_vec;
+  L.b_vec = b_vec;
+  const std::vector<ContractTile> tiles = contract_tiles(proto, blks, L.shape);
+  if (static_cast<int64_t>(tiles.size()) * L.split * L.parts > INT32_MAX) return false;
   L.n_tiles = static_cast<int>(tiles.size());
   // one buffer, one copy: spans, tiles, axis tables
   const size_t o_t = spans.size() * sizeof(ContractSpan), o_x = o_t + tiles.size() * sizeof(ContractTile);
@@ -1451,6 +1466,13 @@ struct tnx_heff {
   // routed stages 1-3 (mixed precisions): which output slots the epilogue writes
   bool routed = false;
   RoutedLayout rl;
+  // FP64: l_img holds L, r_img one copy of R per weight (weights[0] = 1), both
+  // divided by their powers of two; output slots with a single term of one of
+  // these weights are never formed, the others are when mpo_sum is set
+  std::vector<double> weights;
+  bool mpo_sum = false;
+  std::vector<int64_t> l_off, r_off;  // element offset of each block in its copy
+  int64_t l_total = 0, r_total = 0;   // elements of one copy
 };
 
 int tnx_heff_create(const tnx_tensor_desc* L, const tnx_tensor_desc* theta, const tnx_tensor_desc* Wl,
@@ -1526,6 +1548,84 @@ int tnx_heff_out_keys(const tnx_heff* h, int64_t* n_keys, int32_t* keys) {
 
 double tnx_heff_flops(const tnx_heff* h) { return h ? h->H.flops : 0.0; }
 
+}  // extern "C"
+
+namespace {
+// FP64 stage 4 sums one product per MPO term, A = the term's X1 slot and B =
+// R times the term's weight, instead of one per output slot of a formed X3.
+// An output slot with a single term costs the same either way and is never
+// formed; one with several costs a product more per extra term, which on small
+// operators is less than the launch that would sum them first.  The limit is
+// where both cost the same, about 8 us: extra products at 30 TFLOP/s against a
+// launch and the slots' traffic (chi = 64 chain: 1e6 extra FLOPs; chi = 1024
+// cylinder: 4e9).
+constexpr double kF64ExtraFlops = 2.5e8;
+constexpr size_t kF64Weights = 6;  // copies of R at most
+
+int64_t even(int64_t n) { return (n + 1) / 2 * 2; }
+
+// The FP64 copies of an environment T: blocks with their last leg padded to an
+// even extent (zeros), so that the products read it by 16 bytes; one copy per
+// scale, `total` elements each.  Returns once the copies are made.
+void padded_copies(const TensorStruct& T, const double* src, const double* scale, int nscale, DevMem& dst,
+                   std::vector<int64_t>& off, int64_t* total, cudaStream_t st) {
+  std::vector<DevPadSeg> segs;
+  std::vector<DevChunk> chunks;
+  off.clear();
+  *total = 0;
+  for (size_t k = 0; k < T.keys.size(); ++k) {
+    const auto& d = T.dims[k];
+    const int64_t n = d[0] * d[1] * d[2];
+    off.push_back(*total);
+    *total += d[0] * d[1] * even(d[2]);
+    if (n == 0) continue;
+    const int id = static_cast<int>(segs.size());
+    segs.push_back({T.offs[k], off.back(), static_cast<int32_t>(d[2]), static_cast<int32_t>(even(d[2]))});
+    for (int64_t e = 0; e < n; e += 4096) chunks.push_back({id, 0, e, std::min<int64_t>(4096, n - e)});
+  }
+  dst.alloc(std::max<int64_t>(2, *total) * sizeof(double) * nscale);
+  CUDA_OK(cudaMemsetAsync(dst.p, 0, dst.n, st));
+  DevMem ds, dc;
+  upload(ds, segs, st);
+  upload(dc, chunks, st);
+  launch_padded_copies(src, dst.as<double>(), ds.as<DevPadSeg>(), dc.as<DevChunk>(), static_cast<int>(chunks.size()),
+                       *total, scale, nscale, st);
+  CUDA_OK(cudaGetLastError());
+  CUDA_OK(cudaStreamSynchronize(st));
+}
+
+void choose_f64_weights(tnx_heff* h) {
+  const HeffPlan& H = h->H;
+  std::map<double, int64_t> single, all;
+  double extra = 0.0;
+  for (const MpoPair& mp : H.pairs) {
+    std::vector<int32_t> n(mp.n_out_slots, 0);
+    for (const MpoTerm& t : mp.terms) ++n[t.out_slot];
+    int64_t mg = 0;  // columns stage 4 gives this pair's slots
+    for (size_t b = 0; b < H.R.keys.size(); ++b)
+      if (H.R.keys[b][0] == mp.qd) mg = std::max(mg, H.R.dims[b][2]);
+    for (const MpoTerm& t : mp.terms) {
+      ++all[t.w];
+      if (n[t.out_slot] == 1) ++single[t.w];
+    }
+    for (int32_t k : n)
+      if (k > 1) extra += 2.0 * (k - 1) * static_cast<double>(mp.mc) * mp.md * static_cast<double>(mg);
+  }
+  h->mpo_sum = extra > kF64ExtraFlops || all.size() > kF64Weights;
+  std::vector<std::pair<int64_t, double>> by;
+  for (const auto& kv : h->mpo_sum ? single : all)
+    if (kv.first != 1.0) by.push_back({kv.second, kv.first});
+  std::sort(by.begin(), by.end(), [](const auto& x, const auto& y) {
+    return x.first != y.first ? x.first > y.first : x.second < y.second;
+  });
+  h->weights.assign(1, 1.0);
+  for (const auto& w : by)
+    if (h->weights.size() < kF64Weights) h->weights.push_back(w.second);
+}
+}  // namespace
+
+extern "C" {
+
 int tnx_heff_set_operators(tnx_heff* h, const double* L, const double* Wl, const double* Wr, const double* R,
                            int32_t precision, void* stream) {
   TNX_TRY({
@@ -1571,12 +1671,14 @@ int tnx_heff_set_operators(tnx_heff* h, const double* L, const double* Wl, const
     }
     // the stage-1 A image (L) serves the unfused and routed paths
     const bool plain = !h->fused;
-    h->l_img.alloc(plain ? std::max<int64_t>(1, h->g1.a_tiles) * ig.tile_bytes * split : 0);
-    h->r_img.alloc(std::max<int64_t>(1, h->g4.b_tiles) * ig.tile_bytes * split);
-    h->l_lo = h->g1.a_tiles * ig.tile_bytes;
-    h->r_lo = h->g4.b_tiles * ig.tile_bytes;
-    if (h->l_img.n) CUDA_OK(cudaMemsetAsync(h->l_img.p, 0, h->l_img.n, st));
-    CUDA_OK(cudaMemsetAsync(h->r_img.p, 0, h->r_img.n, st));
+    if (mode != IMG_F64) {
+      h->l_img.alloc(plain ? std::max<int64_t>(1, h->g1.a_tiles) * ig.tile_bytes * split : 0);
+      h->r_img.alloc(std::max<int64_t>(1, h->g4.b_tiles) * ig.tile_bytes * split);
+      h->l_lo = h->g1.a_tiles * ig.tile_bytes;
+      h->r_lo = h->g4.b_tiles * ig.tile_bytes;
+      if (h->l_img.n) CUDA_OK(cudaMemsetAsync(h->l_img.p, 0, h->l_img.n, st));
+      CUDA_OK(cudaMemsetAsync(h->r_img.p, 0, h->r_img.n, st));
+    }
     // Environments can sit far outside the FP32/BF16 range (a random MPS's
     // environments shrink geometrically with length): pack L and R divided by
     // powers of two near their max-abs and multiply 2^(eL+eR) back in the
@@ -1592,6 +1694,18 @@ int tnx_heff_set_operators(tnx_heff* h, const double* L, const double* Wl, const
     auto pow2_of = [](double m) { return (m > 0.0 && std::isfinite(m)) ? std::ldexp(1.0, std::ilogb(m)) : 1.0; };
     const double sL = pow2_of(mx[0]), sR = pow2_of(mx[1]);
     h->out_scale = sL * sR;
+    if (mode == IMG_F64) {
+      choose_f64_weights(h);
+      const int nw = static_cast<int>(h->weights.size());
+      std::vector<double> rs(nw);
+      for (int j = 0; j < nw; ++j) rs[j] = h->weights[j] / sR;
+      const double ls = 1.0 / sL;
+      padded_copies(H.L, L, &ls, 1, h->l_img, h->l_off, &h->l_total, st);
+      padded_copies(H.R, R, rs.data(), nw, h->r_img, h->r_off, &h->r_total, st);
+      h->lp_img.alloc(0);
+      h->prec = precision;
+      return TNX_OK;
+    }
     if (h->fused) {
       h->lp_img.alloc(std::max<int64_t>(1, h->fl.lp_bytes) * split);
       CUDA_OK(cudaMemsetAsync(h->lp_img.p, 0, h->lp_img.n, st));
@@ -1688,6 +1802,11 @@ struct tnx_heff_batch {
   int64_t n_routes = 0;
   int32_t route_win_max = 0;  // records in the largest (tile, lane quarter, chunk) window
   const int32_t* skip = nullptr;
+  // FP64: stage 1 (L . theta -> X1 slots), the sums of the multi-term slots
+  // (mpo_* tables, outputs in f64_oslots) and stage 4, all on plain blocks
+  DevMem f64_oslots;
+  std::vector<std::unique_ptr<DevMem>> f64_blobs;
+  std::vector<ContractLaunch> f64_s1, f64_s4;  // one launch per K split among the operators
   int n_launches = 0;
   std::vector<uint64_t> last_src, last_out;
   // host-resident streaming (tnx_heff_batch_apply_host): each problem's theta
@@ -1715,6 +1834,308 @@ struct tnx_heff_batch {
   }
 };
 
+}  // extern "C"
+
+namespace {
+// One operator's products of one stage.
+struct F64Stage {
+  std::vector<ContractSpan> spans;
+  std::vector<ContractTile> proto;
+  std::vector<ContractBlk> blks;
+  void close(ContractTile t, size_t first) {
+    ContractBlk k{};
+    t.span0 = static_cast<int32_t>(first);
+    t.nspan = static_cast<int32_t>(spans.size() - first);
+    for (size_t u = first; u < spans.size(); ++u) {
+      k.ktiles += cdiv(spans[u].K, 16);
+      k.k4 += cdiv(spans[u].K, 4);
+    }
+    t.ktiles = static_cast<int32_t>(k.ktiles);
+    k.M = t.M;
+    k.N = t.N;
+    proto.push_back(t);
+    blks.push_back(k);
+  }
+};
+
+// The launches of one stage.  Every operator's K split is chosen from its own
+// products, so that its sums are the same alone and in any batch; operators of
+// one split share a launch, whose tile shape suits them all.
+std::vector<ContractLaunch> f64_launches(const std::vector<F64Stage>& ops, bool a_kfast, bool b_vec,
+                                         std::vector<std::unique_ptr<DevMem>>& blobs) {
+  const int sms = device_sm_count();
+  std::map<int, F64Stage> by;
+  int shape = 0, split = 1, parts = 1;
+  for (const F64Stage& o : ops) {
+    contract_choose(o.blks, sms, 1, 8, &shape, &split, &parts);
+    F64Stage& g = by[split];
+    const int32_t s0 = static_cast<int32_t>(g.spans.size());
+    g.spans.insert(g.spans.end(), o.spans.begin(), o.spans.end());
+    g.blks.insert(g.blks.end(), o.blks.begin(), o.blks.end());
+    for (ContractTile t : o.proto) {
+      t.span0 += s0;
+      g.proto.push_back(t);
+    }
+  }
+  std::vector<ContractLaunch> out;
+  for (const auto& kv : by) {
+    ContractLaunch L{};
+    contract_choose(kv.second.blks, sms, kv.first, kv.first, &L.shape, &L.split, &L.parts);
+    const std::vector<ContractTile> tiles = contract_tiles(kv.second.proto, kv.second.blks, L.shape);
+    if (static_cast<int64_t>(tiles.size()) * L.split > INT32_MAX)
+      throw PlanError{TNX_ERR_UNSUPPORTED, "too many output tiles in one batch"};
+    L.n_tiles = static_cast<int>(tiles.size());
+    L.a_kfast = a_kfast;
+    L.b_kfast = false;
+    L.a_vec = true;  // padded copies and slots; bases are null, offsets absolute
+    L.b_vec = b_vec;
+    const size_t o_t = kv.second.spans.size() * sizeof(ContractSpan);
+    std::vector<uint8_t> h(std::max<size_t>(64, o_t + tiles.size() * sizeof(ContractTile)));
+    if (o_t) std::memcpy(h.data(), kv.second.spans.data(), o_t);
+    if (!tiles.empty()) std::memcpy(h.data() + o_t, tiles.data(), tiles.size() * sizeof(ContractTile));
+    blobs.push_back(std::make_unique<DevMem>());
+    upload(*blobs.back(), h);
+    L.spans = reinterpret_cast<const ContractSpan*>(blobs.back()->as<uint8_t>());
+    L.tiles = reinterpret_cast<const ContractTile*>(blobs.back()->as<uint8_t>() + o_t);
+    out.push_back(L);
+  }
+  return out;
+}
+
+int32_t stride32(int64_t s) {
+  // in-tile offsets (up to 128 rows) are formed in 32 bits
+  if (s >= (int64_t{1} << 24)) throw PlanError{TNX_ERR_UNSUPPORTED, "H_eff block stride exceeds 2^24 elements"};
+  return static_cast<int32_t>(s);
+}
+
+// FP64 tables.  X1 slots (b, p, q) of every MPO pair are c x d matrices; slots
+// no W_l W_r term reads are not computed (12 of the cylinder's 104), rows and
+// pitch padded to even for 16-byte reads (a pad row is L's zero row, a pad
+// column is never written nor read).  Stage 1
+// writes runs of consecutive b as one matrix; stage 4 adds, for each theta
+// block element (s, t), one product X1 slot x (w R[:, f, :]) per term.  theta
+// and the outputs are read and written in place (slots of the pointer tables),
+// and blocks that no term reaches are zeroed by tiles without products.
+void heff_batch_build_f64(tnx_heff_batch* b) {
+  const int n = static_cast<int>(b->hs.size());
+  // kept X1 slots, and slots formed by the sum kernel
+  std::vector<std::vector<std::vector<int64_t>>> x1(n), x3(n);  // [problem][pair][slot] -> element, -1
+  std::vector<std::vector<std::vector<char>>> formed(n);        // [problem][pair][out slot]
+  int64_t n1 = 0, n3 = 0;
+  for (int i = 0; i < n; ++i) {
+    const tnx_heff* h = b->hs[i];
+    const HeffPlan& H = h->H;
+    x1[i].resize(H.pairs.size());
+    x3[i].resize(H.pairs.size());
+    formed[i].resize(H.pairs.size());
+    for (size_t p = 0; p < H.pairs.size(); ++p) {
+      const MpoPair& mp = H.pairs[p];
+      const int64_t sz = even(mp.mc) * even(mp.md);  // pitch and rows even: 16-byte reads
+      std::vector<int32_t> cnt(mp.n_out_slots, 0);
+      std::vector<char> plain(mp.n_out_slots, 1), used(mp.n_in_slots, 0);
+      for (const MpoTerm& t : mp.terms) {
+        ++cnt[t.out_slot];
+        used[t.in_slot] = 1;
+        if (std::find(h->weights.begin(), h->weights.end(), t.w) == h->weights.end()) plain[t.out_slot] = 0;
+      }
+      formed[i][p].assign(mp.n_out_slots, 0);
+      x3[i][p].assign(mp.n_out_slots, -1);
+      for (int32_t o = 0; o < mp.n_out_slots; ++o)
+        if (cnt[o] > 0 && (!plain[o] || (h->mpo_sum && cnt[o] > 1))) {
+          formed[i][p][o] = 1;
+          x3[i][p][o] = n3;
+          n3 += sz;
+        }
+      x1[i][p].assign(mp.n_in_slots, -1);
+      // consecutive b of one (p, q) are consecutive matrices: one row axis (b, c)
+      for (size_t k = 0; k < mp.ins.size(); ++k) {
+        const MpoIn& in = mp.ins[k];
+        for (int32_t pq = 0; pq < in.mp * in.mq; ++pq)
+          for (int32_t bb = 0; bb < in.mb; ++bb) {
+            const int32_t sl = mp.in_slot0[k] + bb * in.mp * in.mq + pq;
+            if (!used[sl]) continue;
+            x1[i][p][sl] = n1;
+            n1 += sz;
+          }
+      }
+    }
+  }
+  b->x1.alloc(std::max<int64_t>(1, n1) * sizeof(double));
+  b->x3_img.alloc(std::max<int64_t>(1, n3) * sizeof(double));
+  const uint64_t x1_base = reinterpret_cast<uint64_t>(b->x1.p), x3_base = reinterpret_cast<uint64_t>(b->x3_img.p);
+  std::vector<F64Stage> s1(n), s4(n);
+  std::vector<DevMpoPair> MP;
+  std::vector<DevMpoSlot> MI, MO;
+  std::vector<DevMpoTerm> MT;
+  std::vector<int2> MC;
+  for (int i = 0; i < n; ++i) {
+    const tnx_heff* h = b->hs[i];
+    const HeffPlan& H = h->H;
+    const int64_t l0 = static_cast<int64_t>(reinterpret_cast<uint64_t>(h->l_img.p) / 8);
+    std::map<int64_t, size_t> l_blk;  // L block by its offset in the caller's buffer
+    for (size_t k = 0; k < H.L.keys.size(); ++k) l_blk[H.L.offs[k]] = k;
+    const int64_t r0 = static_cast<int64_t>(reinterpret_cast<uint64_t>(h->r_img.p) / 8);
+    // stage 1: (group, row or column origin) -> K origin -> block
+    std::map<std::pair<int32_t, int32_t>, std::map<int32_t, const PackSeg*>> lmap, tmap;
+    for (const PackSeg& s : H.s1.packA) lmap[{s.group, s.row0}][s.k0] = &s;
+    for (const PackSeg& s : H.s1.packB) tmap[{s.group, s.row0}][s.k0] = &s;
+    for (size_t p = 0; p < H.pairs.size(); ++p) {
+      const MpoPair& mp = H.pairs[p];
+      for (size_t k = 0; k < mp.ins.size(); ++k) {
+        const MpoIn& in = mp.ins[k];
+        const auto il = lmap.find({in.g1, in.row0});
+        const auto it = tmap.find({in.g1, in.col0});
+        if (il == lmap.end() || it == tmap.end()) throw PlanError{TNX_ERR_RUNTIME, "internal: X1 block without operands"};
+        for (int32_t pq = 0; pq < in.mp * in.mq; ++pq)
+          for (int32_t b0 = 0; b0 < in.mb;) {
+            auto at = [&](int32_t bb) { return x1[i][p][mp.in_slot0[k] + bb * in.mp * in.mq + pq]; };
+            if (at(b0) < 0) {
+              ++b0;
+              continue;
+            }
+            int32_t b1 = b0 + 1;
+            while (b1 < in.mb && at(b1) >= 0) ++b1;
+            const size_t first = s1[i].spans.size();
+            for (const auto& kv : il->second) {
+              const auto jt = it->second.find(kv.first);
+              if (jt == it->second.end()) continue;
+              const PackSeg &l = *kv.second, &t = *jt->second;  // L[a, b, c], theta[a, p, q, d]
+              ContractSpan g{};
+              g.a_off = l0 + h->l_off[l_blk.at(l.src_off)] + b0 * even(mp.mc);
+              g.b_off = t.src_off + static_cast<int64_t>(pq) * mp.md;
+              g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
+              g.ar_str = 1;
+              g.ak_str = stride32(l.dims[1] * even(l.dims[2]));
+              g.br_str = 1;
+              g.bk_str = stride32(static_cast<int64_t>(t.dims[1]) * t.dims[2] * t.dims[3]);
+              g.K = l.dims[0];
+              g.b_slot = i;
+              s1[i].spans.push_back(g);
+            }
+            ContractTile t{};
+            t.out_off = static_cast<int64_t>(x1_base / 8) + at(b0);
+            t.M = static_cast<int32_t>((b1 - b0) * even(mp.mc));
+            t.N = mp.md;
+            t.r_tab = t.c_tab = -1;
+            t.r_str = static_cast<int32_t>(even(mp.md));
+            t.c_str = 1;
+            t.scale = 1.0;
+            s1[i].close(t, first);
+            b0 = b1;
+          }
+      }
+      // the sums of this pair's formed slots
+      DevMpoPair dp{};
+      dp.mc = mp.mc;
+      dp.md = mp.md;
+      dp.in0 = static_cast<int32_t>(MI.size());
+      dp.out0 = static_cast<int32_t>(MO.size());
+      dp.term0 = static_cast<int32_t>(MT.size());
+      for (const MpoTerm& t : mp.terms)
+        if (formed[i][p][t.out_slot]) MT.push_back({t.out_slot, t.in_slot, t.w});
+      dp.n_terms = static_cast<int32_t>(MT.size()) - dp.term0;
+      if (dp.n_terms > 0) {
+        for (int64_t e : x1[i][p]) MI.push_back({x1_base + static_cast<uint64_t>(std::max<int64_t>(0, e)) * 8, even(mp.md)});
+        for (int64_t e : x3[i][p])
+          MO.push_back({x3_base + static_cast<uint64_t>(std::max<int64_t>(0, e)) * 8, even(mp.md)});
+        const int id = static_cast<int>(MP.size());
+        MP.push_back(dp);
+        const int64_t pts = static_cast<int64_t>(mp.mc) * mp.md;
+        if (pts > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "an MPO pair has more than 2^31 points"};
+        for (int64_t p0 = 0; p0 < pts; p0 += mpo_points_per_cta()) MC.push_back(make_int2(id, static_cast<int>(p0)));
+      }
+    }
+    // stage 4: products by theta block and (s, t)
+    std::map<Key, size_t> th_idx;
+    for (size_t k = 0; k < H.th.keys.size(); ++k) th_idx[H.th.keys[k]] = k;
+    std::vector<std::vector<std::vector<ContractSpan>>> prod(H.th.keys.size());
+    for (size_t k = 0; k < H.th.keys.size(); ++k) prod[k].resize(H.th.dims[k][1] * H.th.dims[k][2]);
+    std::map<std::pair<int32_t, int32_t>, std::vector<size_t>> r_by;  // (q_d, q_f) -> R blocks
+    for (size_t k = 0; k < H.R.keys.size(); ++k) r_by[{H.R.keys[k][0], H.R.keys[k][1]}].push_back(k);
+    for (size_t p = 0; p < H.pairs.size(); ++p) {
+      const MpoPair& mp = H.pairs[p];
+      size_t u = 0;  // terms are sorted by output slot
+      for (size_t k = 0; k < mp.outs.size(); ++k) {
+        const MpoOut& o = mp.outs[k];
+        const Key& ok = H.mpo_out_keys[p][k];  // (q_s, q_t, q_f)
+        const auto rb = r_by.find({mp.qd, ok[2]});
+        for (int32_t e = 0; e < o.ms * o.mt * o.mf; ++e) {
+          const int32_t slot = mp.out_slot0[k] + e, st = e / o.mf, f = e % o.mf;
+          size_t u1 = u;
+          while (u1 < mp.terms.size() && mp.terms[u1].out_slot == slot) ++u1;
+          if (u1 > u && rb != r_by.end())
+            for (size_t rk : rb->second) {
+              const auto& rd = H.R.dims[rk];
+              if (rd[0] != mp.md || rd[1] != o.mf || rd[2] == 0) continue;
+              const auto ti = th_idx.find(Key{mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
+              if (ti == th_idx.end()) continue;
+              auto& dst = prod[ti->second].at(st);
+              ContractSpan g{};
+              g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
+              g.ar_str = static_cast<int32_t>(even(mp.md));
+              g.ak_str = 1;
+              g.br_str = 1;
+              g.bk_str = stride32(rd[1] * even(rd[2]));
+              g.K = mp.md;
+              const int64_t r = r0 + h->r_off[rk] + f * even(rd[2]);
+              if (formed[i][p][slot]) {
+                g.a_off = static_cast<int64_t>(x3_base / 8) + x3[i][p][slot];
+                g.b_off = r;
+                dst.push_back(g);
+              } else {
+                for (size_t v = u; v < u1; ++v) {
+                  const auto w = std::find(h->weights.begin(), h->weights.end(), mp.terms[v].w);
+                  if (w == h->weights.end()) throw PlanError{TNX_ERR_RUNTIME, "internal: MPO weight without its R copy"};
+                  g.a_off = static_cast<int64_t>(x1_base / 8) + x1[i][p][mp.terms[v].in_slot];
+                  g.b_off = r + static_cast<int64_t>(w - h->weights.begin()) * h->r_total;
+                  dst.push_back(g);
+                }
+              }
+            }
+          u = u1;
+        }
+      }
+    }
+    for (size_t k = 0; k < H.th.keys.size(); ++k) {
+      const auto& td = H.th.dims[k];
+      if (td[0] == 0 || td[3] == 0) continue;
+      for (size_t st = 0; st < prod[k].size(); ++st) {
+        const size_t first = s4[i].spans.size();
+        s4[i].spans.insert(s4[i].spans.end(), prod[k][st].begin(), prod[k][st].end());
+        ContractTile t{};
+        t.out_off = H.th.offs[k] + static_cast<int64_t>(st) * td[3];
+        t.M = static_cast<int32_t>(td[0]);
+        t.N = static_cast<int32_t>(td[3]);
+        t.r_tab = t.c_tab = -1;
+        t.r_str = stride32(td[1] * td[2] * td[3]);
+        t.c_str = 1;
+        t.out_slot = 1 + i;
+        t.scale = h->out_scale;  // undoes the power-of-two scaling of L and R
+        s4[i].close(t, first);
+      }
+    }
+  }
+  // stage 1: L[a, (b, c)] padded, theta[a, .., d] as the caller laid it out
+  b->f64_s1 = f64_launches(s1, false, false, b->f64_blobs);
+  // stage 4: X1 slots [c, d] and R[d, f, g], both padded
+  b->f64_s4 = f64_launches(s4, true, true, b->f64_blobs);
+  upload(b->mpo_pairs, MP);
+  upload(b->mpo_slots, MI);
+  upload(b->f64_oslots, MO);
+  upload(b->mpo_terms, MT);
+  upload(b->mpo_chunks, MC);
+  b->n_mpo_chunks = static_cast<int>(MC.size());
+  b->err.alloc(sizeof(int32_t));
+  CUDA_OK(cudaMemset(b->err.p, 0, sizeof(int32_t)));
+  b->src_tab.alloc(sizeof(PtrTab));
+  b->out_tab4.alloc(sizeof(PtrTab));
+  CUDA_OK(cudaDeviceSynchronize());
+  b->n_launches = static_cast<int>(b->f64_s1.size() + b->f64_s4.size()) + (b->n_mpo_chunks > 0 ? 1 : 0);
+}
+}  // namespace
+
+extern "C" {
+
 int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx_heff_batch** out) {
   TNX_TRY({
     if (n < 1 || n > kMaxSlots - 1) return set_err(TNX_ERR_VALUE, "batch size must be in [1, 255]");
@@ -1724,7 +2145,6 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     const int mode = b->mode;
     const ImgGeom ig = img_geom(mode);
     const int split = mode == IMG_BF16 ? 2 : 1;
-    const bool f32 = mode != IMG_F64;
     for (int i = 0; i < n; ++i) {
       if (hs[i]->prec != precision) return set_err(TNX_ERR_VALUE, "operators were packed for another precision");
       if (hs[i]->fused != hs[0]->fused)
@@ -1739,6 +2159,11 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     for (int i = 0; i < n; ++i) {
       b->th_off.push_back(b->th_total);
       b->th_total += hs[i]->H.th.total;
+    }
+    if (mode == IMG_F64) {
+      heff_batch_build_f64(b.get());
+      *out = b.release();
+      return TNX_OK;
     }
     // sizes: theta images (stage-1 B), X1 results, X3 images (stage-4 A)
     const bool fz = b->fused, rt = b->routed;
@@ -1768,7 +2193,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     b->x3_img.alloc(std::max<int64_t>(1, x3_tiles) * ig.tile_bytes * split);
     b->th_lo = th_tiles * ig.tile_bytes;
     b->x3_lo = x3_tiles * ig.tile_bytes;
-    b->x1.alloc(fz ? 16 : std::max<int64_t>(1, x1_elems) * (f32 ? 4 : 8));
+    b->x1.alloc(fz ? 16 : std::max<int64_t>(1, x1_elems) * 4);
     CUDA_OK(cudaMemset(b->th_img.p, 0, b->th_img.n));
     CUDA_OK(cudaMemset(b->x3_img.p, 0, b->x3_img.n));
     std::vector<int64_t> thp_t0(n, 0);
@@ -1793,7 +2218,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     const uint64_t th_base = reinterpret_cast<uint64_t>(b->th_img.p);
     const uint64_t x3_base = reinterpret_cast<uint64_t>(b->x3_img.p);
     const uint64_t x1_base = reinterpret_cast<uint64_t>(b->x1.p);
-    const int esz = f32 ? 4 : 8;
+    constexpr int esz = 4;  // X1 is FP32
     std::vector<DevPackSeg> tp;
     std::vector<DevChunk> tc;
     std::vector<DevRowPackSeg> trs;
@@ -1993,7 +2418,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
                                         esz;
                 sl.ld = ld;
                 // the FP32 MPO kernel loads 8 consecutive d (padding included) with 16-byte loads
-                if (f32 && !fz && (H.x1_align != kMpoKAlign || sl.base % 32 != 0 || ld % 8 != 0))
+                if (!fz && (H.x1_align != kMpoKAlign || sl.base % 32 != 0 || ld % 8 != 0))
                   return set_err(TNX_ERR_RUNTIME, "internal: X1 slot not aligned for the vector MPO loads");
                 MI.push_back(sl);
               }
@@ -2123,8 +2548,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
               FTL.push_back({work, DevFTile{fpair, static_cast<int32_t>(ct), static_cast<int32_t>(dt), 0}});
         }
         const int ppc = mpo_points_per_cta();
-        const int dpt = mpo_d_per_thread(b->mode);
-        const int npts = mp.mc * ((mp.md + dpt - 1) / dpt);
+        const int npts = mp.mc * ((mp.md + kMpoKAlign - 1) / kMpoKAlign);  // one thread forms kMpoKAlign consecutive d
         for (int p0 = 0; p0 < npts && dp.n_terms > 0; p0 += ppc) MC.push_back(make_int2(pair_id, p0));
       }
       if (rti) {
@@ -2355,7 +2779,20 @@ int tnx_heff_batch_route_stats(const tnx_heff_batch* b, int64_t* n_routes, int32
 // src_tab / out_tab4: device pointer tables of the inputs (problem i) and outputs (slot 1 + i)
 static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, const uint64_t* src_tab,
                              const uint64_t* out_tab4) {
-  const bool f32 = b->mode != IMG_F64;
+  if (b->mode == IMG_F64) {
+    // theta is read in place (stage 0 has nothing to pack)
+    if (stage == 1 || stage == 3) {
+      for (ContractLaunch L : stage == 1 ? b->f64_s1 : b->f64_s4) {
+        (stage == 1 ? L.b_ptrs : L.c_ptrs) = stage == 1 ? src_tab : out_tab4;
+        L.skip = b->skip;
+        CUDA_OK(launch_contract_f64(L, st));
+      }
+    } else if (stage == 2) {
+      launch_mpo_sum(b->mpo_pairs.as<DevMpoPair>(), b->mpo_slots.as<DevMpoSlot>(), b->f64_oslots.as<DevMpoSlot>(),
+                     b->mpo_terms.as<DevMpoTerm>(), b->mpo_chunks.as<int2>(), b->n_mpo_chunks, b->skip, st);
+    }
+    return;
+  }
   if (b->fused && stage < 3) {
     // 0: theta panels; 1: fused stages 1-3 (X3 image); 2: nothing (the MPO ran inside stage 1)
     if (stage == 0)
@@ -2377,28 +2814,20 @@ static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, cons
                     b->n_th_chunks, b->mode, b->skip, st);
       break;
     case 1:
-      if (b->mode == IMG_F64)
-        launch_gemm_f64(b->g1.as<DevGroup>(), b->t1.as<DevTile>(), b->n_t1, b->ro1.as<int64_t>(),
-                        b->out_tab1.as<uint64_t>(), b->skip, st);
-      else
-        launch_gemm_tc(b->mode, b->g1.as<DevGroup>(), b->t1.as<DevTile>(), b->n_t1, b->ro1.as<int64_t>(),
+      launch_gemm_tc(b->mode, b->g1.as<DevGroup>(), b->t1.as<DevTile>(), b->n_t1, b->ro1.as<int64_t>(),
                        b->out_tab1.as<uint64_t>(), false, b->err.as<int32_t>(), b->skip, st,
                        b->routed ? DevRouteTabs{b->x3_lo, b->routes.as<DevRoute>(), b->route_win.as<int2>(),
                                                 b->route_rows.as<int2>(), b->route_cols.as<int2>()}
                                  : DevRouteTabs{});
       break;
     case 2:
-      launch_mpo_apply(f32, b->mode, b->mpo_pairs.as<DevMpoPair>(), b->mpo_slots.as<DevMpoSlot>(),
+      launch_mpo_apply(b->mode, b->mpo_pairs.as<DevMpoPair>(), b->mpo_slots.as<DevMpoSlot>(),
                        b->mpo_oslots.as<DevMpoOutSlot>(), b->mpo_terms.as<DevMpoTerm>(), b->mpo_chunks.as<int2>(),
                        b->n_mpo_chunks, b->mpo_smem, b->skip, st);
       break;
     default:
       launch_zero_ranges(out_tab4, b->zero_chunks.as<DevChunk>(), b->n_zero_chunks, b->skip, st);
-      if (b->mode == IMG_F64)
-        launch_gemm_f64(b->g4.as<DevGroup>(), b->t4.as<DevTile>(), b->n_t4, b->ro4.as<int64_t>(),
-                        out_tab4, b->skip, st);
-      else
-        launch_gemm_tc(b->mode, b->g4.as<DevGroup>(), b->t4.as<DevTile>(), b->n_t4, b->ro4.as<int64_t>(),
+      launch_gemm_tc(b->mode, b->g4.as<DevGroup>(), b->t4.as<DevTile>(), b->n_t4, b->ro4.as<int64_t>(),
                        out_tab4, true, b->err.as<int32_t>(), b->skip, st);
   }
 }

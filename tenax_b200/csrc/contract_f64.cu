@@ -38,18 +38,20 @@ namespace tnx {
 namespace {
 constexpr int BK = 16;
 constexpr int STAGES = 4;
-constexpr int THREADS = 128;
-constexpr int kSmemSpans = 16;  // span records kept in shared memory; the rest are read from global
+constexpr int kSmemSpans = 32;  // span records kept in shared memory; the rest are read from global
 
-__device__ __forceinline__ int axis_off(const int32_t* __restrict__ tab, int32_t t, int32_t str, int i) {
-  return t < 0 ? i * str : __ldg(tab + t + i);
+__device__ __forceinline__ int64_t axis_off(const int32_t* __restrict__ tab, int32_t t, int32_t str, int i) {
+  return t < 0 ? static_cast<int64_t>(i) * str : __ldg(tab + t + i);
 }
 
-// 8-byte asynchronous copy; ok = false writes a zero without reading.  No
-// memory clobber: it fills a stage that no fragment load touches before the
-// next barrier, so the two may be interleaved.
-__device__ __forceinline__ void cp8(double* dst, const double* src, bool ok) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 8 : 0));
+// Asynchronous copies of 8 or 16 bytes, of which the first `bytes` are read and
+// the rest is zero.  No memory clobber: they fill a stage that no fragment load
+// touches before the next barrier, so the two may be interleaved.
+__device__ __forceinline__ void cp8(uint32_t dst, const double* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const double* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -77,59 +79,76 @@ __device__ __forceinline__ double ld_peer(uint32_t saddr, uint32_t rank) {
 // loads over all banks, and 16 lanes fetch one row's 16 consecutive K.
 // Otherwise rows are the fast axis: the tile is stored K-major with a row
 // pitch of R + 4 (bank-free fragment loads), consecutive lanes fetch
-// consecutive rows.
-template <int R, bool KF>
+// consecutive rows.  VEC: elements 2i and 2i + 1 of the fast axis are adjacent
+// and every pair starts on 16 bytes, so a lane fetches a pair: the copies' issue
+// is what holds the tensor pipe below its rate.
+template <int R, bool KF, bool VEC, int THREADS>
 struct Operand {
-  static constexpr int kPer = R * BK / THREADS;                 // elements per thread and K tile
+  static constexpr int W = VEC ? 2 : 1;                         // elements a copy
+  static constexpr int kPer = R * BK / W / THREADS;             // copies per thread and K tile
+  static constexpr int kLanes = (KF ? BK : R) / W;              // lanes along the fast axis
   static constexpr int kRows = KF ? kPer : 1;                   // distinct rows per thread
   static constexpr int kTile = KF ? R * BK : BK * (R + 4);      // doubles per stage
-  const double* base;
+  static_assert(kPer >= 1 && THREADS % kLanes == 0, "whole copies");
+  const double* base;  // affine axes: the tile's own origin, so that 32-bit offsets span one tile
   int32_t kt, ks;
+  int32_t rbytes;      // rows fast: bytes of this lane's copy that lie inside the block
   int32_t off[kRows];
 
   __device__ __forceinline__ void set_span(const double* p, const int32_t* tab, int32_t rt, int32_t rs, int32_t kt_,
                                            int32_t ks_, int row0, int rows) {
-    base = p;
+    base = rt < 0 ? p + static_cast<int64_t>(row0) * rs : p;
     kt = kt_;
     ks = ks_;
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
-      const int r = KF ? (static_cast<int>(threadIdx.x) >> 4) + 8 * i : static_cast<int>(threadIdx.x) % R;
-      off[i] = r < rows ? axis_off(tab, rt, rs, row0 + r) : -1;  // -1: past the block, not loaded
+      const int r = KF ? static_cast<int>(threadIdx.x) / kLanes + THREADS / kLanes * i
+                       : static_cast<int>(threadIdx.x) % kLanes * W;
+      off[i] = r < rows ? (rt < 0 ? r * rs : __ldg(tab + rt + row0 + r)) : -1;  // -1: past the block, not loaded
+      if (!KF) rbytes = 8 * min(W, rows - r);
     }
   }
-  // quarter Q of the tile's elements (Q = 4: all of them)
   // TAB: the K axis is a table (several legs that do not merge), else a stride
-  template <bool TAB, int Q>
+  template <bool TAB>
   __device__ __forceinline__ void load_as(double* s, const int32_t* tab, int k0, int K) const {
+    const double* b0 = TAB ? base : base + static_cast<int64_t>(k0) * ks;
     if constexpr (KF) {
-      const int kk = threadIdx.x & 15;
-      const bool ok = k0 + kk < K;
-      const int ko = ok ? (TAB ? __ldg(tab + kt + k0 + kk) : (k0 + kk) * ks) : 0;
-      double* d = s + (threadIdx.x >> 4) * BK + (kk ^ (((threadIdx.x >> 4) & 3) << 2));
-#pragma unroll
-      for (int i = 0; i < kPer; ++i)
-        if ((Q == 4 || (i & 3) == Q) && off[i] >= 0) cp8(d + i * 8 * BK, base + (off[i] + ko), ok);
-    } else {
-      const int r = static_cast<int>(threadIdx.x) % R, q = static_cast<int>(threadIdx.x) / R;
-      if (off[0] < 0) return;
-      double* d = s + q * (R + 4) + r;
+      const int kk = static_cast<int>(threadIdx.x) % kLanes * W, r0 = static_cast<int>(threadIdx.x) / kLanes;
+      const int bytes = 8 * max(0, min(W, K - k0 - kk));
+      const double* p = b0 + (bytes ? (TAB ? __ldg(tab + kt + k0 + kk) : kk * ks) : 0);
+      const uint32_t d = smem_u32(s) + 8 * (r0 * BK + (kk ^ ((r0 & 3) << 2)));
 #pragma unroll
       for (int i = 0; i < kPer; ++i) {
-        if (Q != 4 && (i & 3) != Q) continue;
-        const int kk = k0 + q + i * (THREADS / R);
-        const bool ok = kk < K;
-        const int ko = ok ? (TAB ? __ldg(tab + kt + kk) : kk * ks) : 0;
-        cp8(d + i * (THREADS / R) * (R + 4), base + (off[0] + ko), ok);
+        // rows r0 + i * THREADS / kLanes: a multiple of 4 apart, so one swizzle
+        static_assert(THREADS / kLanes % 4 == 0, "rows of a thread share their swizzle");
+        if (off[i] < 0) continue;
+        if constexpr (VEC)
+          cp16(d + 8 * i * (THREADS / kLanes) * BK, p + off[i], bytes);
+        else
+          cp8(d + 8 * i * (THREADS / kLanes) * BK, p + off[i], bytes);
+      }
+    } else {
+      const int r = static_cast<int>(threadIdx.x) % kLanes * W, q = static_cast<int>(threadIdx.x) / kLanes;
+      if (off[0] < 0) return;
+      const double* p = b0 + off[0];
+      const uint32_t d = smem_u32(s) + 8 * (q * (R + 4) + r);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int kk = q + i * (THREADS / kLanes);
+        const bool ok = k0 + kk < K;
+        const int ko = ok ? (TAB ? __ldg(tab + kt + k0 + kk) : kk * ks) : 0;
+        if constexpr (VEC)
+          cp16(d + 8 * i * (THREADS / kLanes) * (R + 4), p + ko, ok ? rbytes : 0);
+        else
+          cp8(d + 8 * i * (THREADS / kLanes) * (R + 4), p + ko, ok ? 8 : 0);
       }
     }
   }
-  template <int Q>
   __device__ __forceinline__ void load(double* s, const int32_t* tab, int k0, int K) const {
     if (kt < 0)
-      load_as<false, Q>(s, tab, k0, K);
+      load_as<false>(s, tab, k0, K);
     else
-      load_as<true, Q>(s, tab, k0, K);
+      load_as<true>(s, tab, k0, K);
   }
   static __device__ __forceinline__ double frag(const double* s, int r, int kk) {
     return KF ? s[r * BK + (kk ^ ((r & 3) << 2))] : s[kk * (R + 4) + r];
@@ -173,20 +192,23 @@ __device__ __forceinline__ void products_n(double (&acc)[MI][NI][2], const doubl
 
 template <int BM, int BN, bool AK, bool BKF>
 constexpr int smem_doubles() {
-  constexpr int ring = STAGES * (Operand<BM, AK>::kTile + Operand<BN, BKF>::kTile);
+  constexpr int ring = STAGES * (Operand<BM, AK, false, 128>::kTile + Operand<BN, BKF, false, 128>::kTile);
   constexpr int part = BM * (BN + 1);  // a split's partial tile reuses the ring
   return ring > part ? ring : part;
 }
 
-template <int BM, int BN, int WM, int WN, bool AK, bool BKF>
-__global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
+template <int BM, int BN, int WM, int WN, bool AK, bool BKF, bool AV, bool BV>
+__global__ void __launch_bounds__(32 * WM * WN, (BM * BN >= 4096) ? 3 : 4)
     contract_f64_kernel(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
                         const ContractTile* __restrict__ tiles, const ContractSpan* __restrict__ spans,
-                        const int32_t* __restrict__ tab, int split, int parts, double* __restrict__ ws) {
-  static_assert(WM * WN == 4, "four warps");
+                        const int32_t* __restrict__ tab, int split, int parts, double* __restrict__ ws,
+                        const uint64_t* __restrict__ a_ptrs, const uint64_t* __restrict__ b_ptrs,
+                        const uint64_t* __restrict__ c_ptrs, const int32_t* __restrict__ skip_flag) {
+  constexpr int THREADS = 32 * WM * WN;
+  if (skip_flag && *skip_flag) return;  // the whole cluster
   constexpr int MI = BM / 8 / WM, NI = BN / 8 / WN;
-  using OpA = Operand<BM, AK>;
-  using OpB = Operand<BN, BKF>;
+  using OpA = Operand<BM, AK, AV, THREADS>;
+  using OpB = Operand<BN, BKF, BV, THREADS>;
   extern __shared__ __align__(16) double ring[];
   __shared__ ContractSpan sspan[kSmemSpans];
   double* As = ring;
@@ -231,8 +253,10 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     if (fresh) {
       const ContractSpan g = sp < kSmemSpans ? sspan[sp] : spans[t.span0 + sp];
       K = g.K;
-      oa.set_span(A + g.a_off, tab, g.ar_tab, g.ar_str, g.ak_tab, g.ak_str, t.m0, rows);
-      ob.set_span(B + g.b_off, tab, g.br_tab, g.br_str, g.bk_tab, g.bk_str, t.n0, cols);
+      const double* pa = a_ptrs ? reinterpret_cast<const double*>(a_ptrs[g.a_slot]) : A;
+      const double* pb = b_ptrs ? reinterpret_cast<const double*>(b_ptrs[g.b_slot]) : B;
+      oa.set_span(pa + g.a_off, tab, g.ar_tab, g.ar_str, g.ak_tab, g.ak_str, t.m0, rows);
+      ob.set_span(pb + g.b_off, tab, g.br_tab, g.br_str, g.bk_tab, g.bk_str, t.n0, cols);
       fresh = false;
     }
     const uint32_t n4 = static_cast<uint32_t>((min(BK, K - k0) + 3) / 4);
@@ -248,8 +272,8 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
   };
   auto issue = [&](int s) {
     begin(s);
-    oa.template load<4>(As + s * OpA::kTile, tab, k0, K);
-    ob.template load<4>(Bs + s * OpB::kTile, tab, k0, K);
+    oa.load(As + s * OpA::kTile, tab, k0, K);
+    ob.load(Bs + s * OpB::kTile, tab, k0, K);
     finish();
   };
 #pragma unroll
@@ -281,18 +305,24 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     }
   }
   cp_wait<0>();
-  double* out = C + t.out_off;
+  double* out = (c_ptrs ? reinterpret_cast<double*>(c_ptrs[t.out_slot]) : C) + t.out_off;
   if (split == 1) {
+    int64_t co[NI][2];
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        co[j][h] = axis_off(tab, t.c_tab, t.c_str, t.n0 + min(cols - 1, (j * WN + wn) * 8 + (lane & 3) * 2 + h));
 #pragma unroll
     for (int i = 0; i < MI; ++i) {
       const int r = (i * WM + wm) * 8 + (lane >> 2);
       if (r >= rows) continue;
-      const int ro = axis_off(tab, t.r_tab, t.r_str, t.m0 + r);
+      double* row = out + axis_off(tab, t.r_tab, t.r_str, t.m0 + r);
 #pragma unroll
       for (int j = 0; j < NI; ++j) {
         const int c = (j * WN + wn) * 8 + (lane & 3) * 2;
-        if (c < cols) out[ro + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = acc[i][j][0];
-        if (c + 1 < cols) out[ro + axis_off(tab, t.c_tab, t.c_str, t.n0 + c + 1)] = acc[i][j][1];
+        if (c < cols) row[co[j][0]] = acc[i][j][0] * t.scale;
+        if (c + 1 < cols) row[co[j][1]] = acc[i][j][1] * t.scale;
       }
     }
     return;
@@ -325,7 +355,7 @@ __global__ void __launch_bounds__(THREADS, (BM * BN >= 4096) ? 3 : 4)
     if (parts > 1)
       wpart[r * BN + c] = v;
     else
-      out[axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v;
+      out[axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v * t.scale;
   }
   cluster_sync();  // no CTA leaves while a peer reads its shared memory
 }
@@ -341,19 +371,19 @@ __global__ void __launch_bounds__(256)
     const int r = e / cols, c = e - r * cols;
     double v = 0.0;
     for (int p = 0; p < parts; ++p) v += w[static_cast<int64_t>(p) * bm * bn + r * bn + c];
-    C[t.out_off + axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v;
+    C[t.out_off + axis_off(tab, t.r_tab, t.r_str, t.m0 + r) + axis_off(tab, t.c_tab, t.c_str, t.n0 + c)] = v * t.scale;
   }
 }
 
-template <int BM, int BN, int WM, int WN, bool AK, bool BKF>
+template <int BM, int BN, int WM, int WN, bool AK, bool BKF, bool AV, bool BV>
 cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
   constexpr int smem = smem_doubles<BM, BN, AK, BKF>() * static_cast<int>(sizeof(double));
-  auto kernel = contract_f64_kernel<BM, BN, WM, WN, AK, BKF>;
+  auto kernel = contract_f64_kernel<BM, BN, WM, WN, AK, BKF, AV, BV>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(L.n_tiles) * L.split * L.parts);
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(32 * WM * WN);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -372,7 +402,8 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
     e = cudaMallocAsync(&ws, sizeof(double) * BM * BN * static_cast<size_t>(L.n_tiles) * L.parts, st);
     if (e != cudaSuccess) return e;
   }
-  e = cudaLaunchKernelEx(&cfg, kernel, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws);
+  e = cudaLaunchKernelEx(&cfg, kernel, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws,
+                         L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
   if (L.parts > 1) {
     if (e == cudaSuccess) {
       contract_parts_kernel<<<dim3(L.n_tiles, (BM * BN + 255) / 256), 256, 0, st>>>(ws, L.c, L.tiles, L.tab, L.parts,
@@ -385,38 +416,52 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
   return e;
 }
 
+// 16-byte copies of A alone or of both operands (a step where only B could
+// have them reads both by 8 bytes)
+template <int BM, int BN, int WM, int WN, bool AK, bool BKF>
+cudaError_t go_vec(const ContractLaunch& L, cudaStream_t st) {
+  const bool av = L.a_vec && reinterpret_cast<uintptr_t>(L.a) % 16 == 0;
+  const bool bv = L.b_vec && reinterpret_cast<uintptr_t>(L.b) % 16 == 0;
+  if (av && bv) return go<BM, BN, WM, WN, AK, BKF, true, true>(L, st);
+  if (av) return go<BM, BN, WM, WN, AK, BKF, true, false>(L, st);
+  return go<BM, BN, WM, WN, AK, BKF, false, false>(L, st);
+}
 template <int BM, int BN, int WM, int WN>
 cudaError_t go_layout(const ContractLaunch& L, cudaStream_t st) {
-  if (L.a_kfast) return L.b_kfast ? go<BM, BN, WM, WN, true, true>(L, st) : go<BM, BN, WM, WN, true, false>(L, st);
-  return L.b_kfast ? go<BM, BN, WM, WN, false, true>(L, st) : go<BM, BN, WM, WN, false, false>(L, st);
+  if (L.a_kfast)
+    return L.b_kfast ? go_vec<BM, BN, WM, WN, true, true>(L, st) : go_vec<BM, BN, WM, WN, true, false>(L, st);
+  return L.b_kfast ? go_vec<BM, BN, WM, WN, false, true>(L, st) : go_vec<BM, BN, WM, WN, false, false>(L, st);
 }
 
 struct Shape {
   int bm, bn, wm, wn, resident;
+  double eff;  // tensor-pipe rate against 64 x 64 tiles (2000^3: 29.1, 25.4, 21.8, 26.7 TFLOP/s)
 };
 // 64 x 64: the DMMA-bound shape; 64 x 32 and 32 x 32: few tiles or small
 // blocks; 128 x 16: narrow column blocks (an MPO leg), whose rows are many
-constexpr Shape kShapes[kContractShapes] = {{64, 64, 2, 2, 3}, {32, 32, 2, 2, 4}, {128, 16, 4, 1, 3}, {64, 32, 2, 2, 4}};
+constexpr Shape kShapes[kContractShapes] = {
+    {64, 64, 2, 2, 3, 1.0}, {32, 32, 2, 2, 4, 0.87}, {128, 16, 4, 1, 3, 0.75}, {64, 32, 2, 2, 4, 0.95}};
 }  // namespace
-
-void contract_tile_shape(int shape, int* bm, int* bn) {
-  *bm = kShapes[shape].bm;
-  *bn = kShapes[shape].bn;
-}
 
 // Estimated clocks of a step for every tile shape and number of K shares (up
 // to 8 in one cluster, beyond that parts of 8 summed by a second launch); the
-// smallest wins.  Per CTA: the longest warp's DMMA chain (16 clocks each), its
-// operand loads (about 48 bytes a clock and SM), and at least 270 clocks a K
-// tile (the latency of a load over the ring's depth).  One CTA on an SM keeps
-// about 0.6 of its tensor pipes busy, three 0.9.
-void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape, int* split, int* parts) {
+// smallest wins.  A CTA's work is its longest warp's DMMA chain (16 clocks
+// each) or its operand loads (about 48 bytes a clock and SM).  The step takes
+// an even spread of that over the SMs, whose pipes are 0.6 busy with one CTA
+// and 0.9 with three, plus what the longest share overhangs it by; at least the
+// longest share alone (700 to 1000 clocks a K tile of latency and issue); and the
+// prologues and epilogues, where a split writes and reads back every partial.
+// Against both sides measured on 20 dense products of 0.02 to 16 GFLOP (every
+// shape, 1 to 16 shares) the choice is within 12 % of the best.
+void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_split, int max_split, int* shape,
+                     int* split, int* parts) {
   double best = -1.0;
   *shape = 0;
-  *split = *parts = 1;
+  *split = std::min(min_split, 8);
+  *parts = min_split / *split;
   for (int s : {1, 3, 2, 0}) {  // the smallest tile of equal estimates
     const Shape& h = kShapes[s];
-    double sum = 0.0, longest = 0.0;
+    double sum = 0.0, work_max = 0.0, cells = 0.0;
     int64_t n = 0, kmax = 0;
     for (const ContractBlk& b : blks) {
       kmax = std::max(kmax, b.ktiles);
@@ -429,7 +474,8 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape,
         const double mem = static_cast<double>((r + c) * b.ktiles) * 16.0 * 8.0 / 48.0;
         const double x = std::max(mma, mem);
         sum += static_cast<double>(count) * x;
-        longest = std::max(longest, std::max(x / 0.6, 270.0 * static_cast<double>(b.ktiles)));
+        work_max = std::max(work_max, x);
+        cells += static_cast<double>(count * r * c);
         n += count;
       };
       add(fm * fn, h.bm, h.bn);
@@ -437,14 +483,18 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape,
       add(fm, h.bm, en);
       add(em > 0 && en > 0 ? 1 : 0, em, en);
     }
-    for (int sp = 1; sp <= 256; sp *= 2) {
-      if (sp > 1 && kmax < 2 * sp) break;
-      const double ctas = static_cast<double>(n * sp);
+    if (n == 0) continue;
+    const double cell = cells / static_cast<double>(n);
+    for (int sp = min_split; sp <= max_split; sp *= 2) {
+      if (sp > min_split && kmax < 2 * sp) break;
+      const double ctas = static_cast<double>(n) * sp;
       const double per_sm = std::min(static_cast<double>(h.resident), std::max(1.0, ctas / n_sm));
-      const double eff = std::min(0.9, 0.45 + 0.15 * per_sm);
-      const double over = 2500.0 + (sp > 1 ? 1500.0 : 0.0);
+      const double eff = std::min(0.9, 0.45 + 0.15 * per_sm) * h.eff;
+      const double over = sp == 1 ? 2500.0 + 0.8 * cell : 4500.0 + (0.8 / sp + 1.5) * cell;
       const double waves = std::max(1.0, ctas / (static_cast<double>(n_sm) * h.resident));
-      const double est = std::max(sum / n_sm / eff, longest / sp) + over * waves + (sp > 8 ? 6000.0 : 0.0);
+      const double alone = std::max(work_max / (0.6 * h.eff), (400.0 + 4.6 * (h.bm + h.bn)) * static_cast<double>(kmax)) / sp;
+      const double est = std::max(sum / n_sm / eff + 0.6 * work_max / sp, alone) + over * waves +
+                         (sp > 8 ? 6000.0 : 0.0);
       if (best < 0.0 || est < best) {
         best = est;
         *shape = s;
@@ -453,6 +503,26 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int* shape,
       }
     }
   }
+}
+
+std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks,
+                                         int shape) {
+  const Shape& h = kShapes[shape];
+  std::vector<std::pair<int64_t, ContractTile>> tl;
+  for (size_t i = 0; i < proto.size(); ++i)
+    for (int64_t m0 = 0; m0 < proto[i].M; m0 += h.bm)
+      for (int64_t n0 = 0; n0 < proto[i].N; n0 += h.bn) {
+        ContractTile t = proto[i];
+        t.m0 = static_cast<int32_t>(m0);
+        t.n0 = static_cast<int32_t>(n0);
+        const int64_t fm = (std::min<int64_t>(h.bm, t.M - m0) + 7) / 8, fn = (std::min<int64_t>(h.bn, t.N - n0) + 7) / 8;
+        tl.push_back({blks[i].k4 * fm * fn, t});
+      }
+  std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  std::vector<ContractTile> out;
+  out.reserve(tl.size());
+  for (const auto& x : tl) out.push_back(x.second);
+  return out;
 }
 
 cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st) {

@@ -1,7 +1,5 @@
 // HBM-bound kernels: operand-image packing, result scatter, the fused MPO
 // application of the two-site H_eff, and FP64 vector primitives.
-#include <type_traits>
-
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -150,7 +148,7 @@ void launch_zero_ranges(const uint64_t* out_tab, const DevChunk* chunks, int n_c
 // outputs of one slot form one aligned K chunk -- a single 16-byte swizzle
 // unit of a BF16 image row (two for TF32) -- and the table reads and image
 // addressing are paid once per chunk instead of once per element.  kMpoTerms
-// terms' loads are kept in flight per thread.  FP64 uses the per-point kernel.
+// terms' loads are kept in flight per thread.  FP64 has its own (mpo_sum_kernel).
 // ---------------------------------------------------------------------------
 constexpr int kMpoThreads = 256;
 constexpr int kMpoTerms = 4;
@@ -225,60 +223,83 @@ __global__ void __launch_bounds__(kMpoThreads) mpo_apply_kernel(
                         o.row0 + c * o.rows_per_c + o.row_add, o.k0 + o.k_add + d0, acc);
 }
 
-// FP64 images: one thread per point (c, d) writes single doubles.  An
-// 8-wide chunk of doubles per thread holds too many registers to beat this
-// (3.78 vs 3.17 ms on the 64-problem batch); the padded K layout is the same.
-__global__ void __launch_bounds__(kMpoThreads) mpo_apply_point_kernel(
-    const DevMpoPair* __restrict__ pairs, const DevMpoSlot* __restrict__ islots,
-    const DevMpoOutSlot* __restrict__ oslots, const DevMpoTerm* __restrict__ terms,
-    const int2* __restrict__ chunks, const int32_t* __restrict__ skip) {
+// FP64: stage 4 reads X1 itself wherever an output slot has a single term (see
+// the FP64 tables of the batch), so only the few slots that sum several terms
+// are formed here, one thread a point (c, d), consecutive threads along d.
+// Reads one X1 slot a term and writes one slot an output: 36 of the cylinder
+// MPO's 104 slots move instead of 104 + 92.
+__global__ void __launch_bounds__(kMpoThreads)
+    mpo_sum_kernel(const DevMpoPair* __restrict__ pairs, const DevMpoSlot* __restrict__ islots,
+                   const DevMpoSlot* __restrict__ oslots, const DevMpoTerm* __restrict__ terms,
+                   const int2* __restrict__ chunks, const int32_t* __restrict__ skip) {
   constexpr int kLoads = 8;
   if (skip && *skip) return;
-  extern __shared__ __align__(16) unsigned char mpo_smem[];
   const int2 ch = chunks[blockIdx.x];
   const DevMpoPair pr = pairs[ch.x];
-  DevMpoTerm* st = reinterpret_cast<DevMpoTerm*>(mpo_smem);
-  DevMpoSlot* si = reinterpret_cast<DevMpoSlot*>(st + pr.n_terms);
-  DevMpoOutSlot* so = reinterpret_cast<DevMpoOutSlot*>(si + pr.n_in_slots);
-  for (int i = threadIdx.x; i < pr.n_terms; i += blockDim.x) st[i] = terms[pr.term0 + i];
-  for (int i = threadIdx.x; i < pr.n_in_slots; i += blockDim.x) si[i] = islots[pr.in0 + i];
-  for (int i = threadIdx.x; i < pr.n_out_slots; i += blockDim.x) so[i] = oslots[pr.out0 + i];
-  __syncthreads();
-  const int p = ch.y + threadIdx.x;
+  const int p = ch.y + static_cast<int>(threadIdx.x);
   if (p >= pr.mc * pr.md || pr.n_terms == 0) return;
   const int64_t c = p / pr.md;
   const int d = p - static_cast<int>(c) * pr.md;
+  const DevMpoTerm* tm = terms + pr.term0;
   double acc = 0.0;
-  int cur = st[0].out_slot;
+  int cur = tm[0].out_slot;
   for (int t0 = 0; t0 < pr.n_terms; t0 += kLoads) {
     double xv[kLoads];
 #pragma unroll
     for (int u = 0; u < kLoads; ++u) {
       xv[u] = 0.0;
       if (t0 + u < pr.n_terms) {
-        const DevMpoSlot sl = si[st[t0 + u].in_slot];
+        const DevMpoSlot sl = islots[pr.in0 + tm[t0 + u].in_slot];
         xv[u] = reinterpret_cast<const double*>(sl.base)[c * sl.ld + d];
       }
     }
 #pragma unroll
     for (int u = 0; u < kLoads; ++u) {
       if (t0 + u >= pr.n_terms) break;
-      const DevMpoTerm tm = st[t0 + u];
-      if (tm.out_slot != cur) {
-        const DevMpoOutSlot o = so[cur];
-        *reinterpret_cast<double*>(reinterpret_cast<uint8_t*>(o.img_addr) +
-                                   img_byte_offset(IMG_F64, 0, o.nKt, o.row0 + c * o.rows_per_c + o.row_add,
-                                                   o.k0 + o.k_add + d)) = acc;
-        cur = tm.out_slot;
+      const DevMpoTerm t = tm[t0 + u];
+      if (t.out_slot != cur) {
+        const DevMpoSlot o = oslots[pr.out0 + cur];
+        reinterpret_cast<double*>(o.base)[c * o.ld + d] = acc;
+        cur = t.out_slot;
         acc = 0.0;
       }
-      acc += tm.w * xv[u];
+      acc += t.w * xv[u];
     }
   }
-  const DevMpoOutSlot o = so[cur];
-  *reinterpret_cast<double*>(reinterpret_cast<uint8_t*>(o.img_addr) +
-                             img_byte_offset(IMG_F64, 0, o.nKt, o.row0 + c * o.rows_per_c + o.row_add,
-                                             o.k0 + o.k_add + d)) = acc;
+  const DevMpoSlot o = oslots[pr.out0 + cur];
+  reinterpret_cast<double*>(o.base)[c * o.ld + d] = acc;
+}
+
+void launch_mpo_sum(const DevMpoPair* pairs, const DevMpoSlot* islots, const DevMpoSlot* oslots,
+                    const DevMpoTerm* terms, const int2* chunks, int n_chunks, const int32_t* skip, cudaStream_t st) {
+  if (n_chunks <= 0) return;
+  mpo_sum_kernel<<<n_chunks, kMpoThreads, 0, st>>>(pairs, islots, oslots, terms, chunks, skip);
+}
+
+// Copies of a block-sparse operand with padded rows (the FP64 H_eff reads its
+// environments by 16 bytes), one per scale; once per operator.
+struct Scales {
+  double s[kMaxScales];
+};
+__global__ void padded_copies_kernel(const double* __restrict__ src, double* __restrict__ dst,
+                                     const DevPadSeg* __restrict__ segs, const DevChunk* __restrict__ chunks,
+                                     int64_t stride, Scales sc, int nscale) {
+  const DevChunk ch = chunks[blockIdx.x];
+  const DevPadSeg s = segs[ch.seg];
+  for (int64_t e = ch.start + threadIdx.x; e < ch.start + ch.count; e += blockDim.x) {
+    const int64_t row = e / s.inner;
+    const double v = src[s.src_off + e];
+    double* d = dst + s.dst_off + row * s.pitch + (e - row * s.inner);
+    for (int j = 0; j < nscale; ++j) d[j * stride] = v * sc.s[j];
+  }
+}
+
+void launch_padded_copies(const double* src, double* dst, const DevPadSeg* segs, const DevChunk* chunks, int n_chunks,
+                          int64_t stride, const double* scale, int nscale, cudaStream_t st) {
+  if (n_chunks <= 0 || nscale <= 0) return;
+  Scales sc{};
+  for (int j = 0; j < nscale && j < kMaxScales; ++j) sc.s[j] = scale[j];
+  padded_copies_kernel<<<n_chunks, 256, 0, st>>>(src, dst, segs, chunks, stride, sc, nscale);
 }
 
 // ---------------------------------------------------------------------------
@@ -293,33 +314,27 @@ __global__ void __launch_bounds__(kPackRows) pack_rows_kernel(const uint64_t* __
                                                         const DevRowPackSeg* __restrict__ segs,
                                                         const int4* __restrict__ chunks,
                                                         const int32_t* __restrict__ skip) {
-  using ValT = typename std::conditional<MODE == IMG_F64, double, float>::type;
   constexpr int kChunks = 4;  // K chunks of 8 per thread, all loads issued before the stores
   if (skip && *skip) return;
   const int4 ch = chunks[blockIdx.x];  // (segment, first row, first K chunk, -)
   const DevRowPackSeg s = segs[ch.x];
   const int r = ch.y + static_cast<int>(threadIdx.x);
-  // BF16 / TF32 CTAs all reach the shared-memory exchange below: a row past
-  // the segment loads zeros and is not stored
-  if (MODE == IMG_F64 && r >= s.rows) return;
+  // every thread reaches the shared-memory exchange below: a row past the
+  // segment loads zeros and is not stored
   const int rr = r < s.rows ? r : s.rows - 1;
   const double* src = reinterpret_cast<const double*>(src_tab[s.src_slot]) + s.src_off + rr;
   uint8_t* img = reinterpret_cast<uint8_t*>(s.img_addr);
   const int nkc = (s.kval + kMpoVec - 1) / kMpoVec;
-  ValT v[kChunks][kMpoVec];
+  float v[kChunks][kMpoVec];
 #pragma unroll
   for (int j = 0; j < kChunks; ++j)
 #pragma unroll
     for (int u = 0; u < kMpoVec; ++u) {
       const int a = (ch.z + j) * kMpoVec + u;
-      v[j][u] = (a < s.kval && r < s.rows) ? static_cast<ValT>(src[static_cast<int64_t>(a) * s.kstride] * s.scale)
-                                           : ValT(0);
+      v[j][u] = (a < s.kval && r < s.rows) ? static_cast<float>(src[static_cast<int64_t>(a) * s.kstride] * s.scale)
+                                           : 0.0f;
     }
-  if constexpr (MODE == IMG_F64) {
-#pragma unroll
-    for (int j = 0; j < kChunks; ++j)
-      if (ch.z + j < nkc) img_store_chunk<MODE>(img, s.lo_off, s.nKt, s.row0 + r, s.k0 + (ch.z + j) * kMpoVec, v[j]);
-  } else {
+  {
     // BF16 / TF32: each row's 4 chunks in their image form go through shared
     // memory, so that the four lanes of a quad then write one row's 64 bytes
     // (of each plane) and a store instruction fills whole sectors of 8 rows
@@ -370,15 +385,13 @@ __global__ void __launch_bounds__(kPackRows) pack_rows_kernel(const uint64_t* __
 void launch_pack_rows(const uint64_t* src_tab, const DevRowPackSeg* segs, const int4* chunks, int n_chunks, int mode,
                       const int32_t* skip, cudaStream_t st) {
   if (n_chunks <= 0) return;
-  if (mode == IMG_F64)
-    pack_rows_kernel<IMG_F64><<<n_chunks, kPackRows, 0, st>>>(src_tab, segs, chunks, skip);
-  else if (mode == IMG_BF16)
+  if (mode == IMG_BF16)
     pack_rows_kernel<IMG_BF16><<<n_chunks, kPackRows, 0, st>>>(src_tab, segs, chunks, skip);
   else
     pack_rows_kernel<IMG_TF32><<<n_chunks, kPackRows, 0, st>>>(src_tab, segs, chunks, skip);
 }
 
-void launch_mpo_apply(bool x1_f32, int mode, const DevMpoPair* pairs, const DevMpoSlot* islots,
+void launch_mpo_apply(int mode, const DevMpoPair* pairs, const DevMpoSlot* islots,
                       const DevMpoOutSlot* oslots, const DevMpoTerm* terms, const int2* chunks, int n_chunks,
                       size_t smem_bytes, const int32_t* skip, cudaStream_t st) {
   if (n_chunks <= 0) return;
@@ -388,9 +401,7 @@ void launch_mpo_apply(bool x1_f32, int mode, const DevMpoPair* pairs, const DevM
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return;
     kernel<<<n_chunks, kMpoThreads, smem, st>>>(pairs, islots, oslots, terms, chunks, skip);
   };
-  if (!x1_f32)
-    go(mpo_apply_point_kernel);
-  else if (mode == IMG_BF16)
+  if (mode == IMG_BF16)
     go(mpo_apply_kernel<IMG_BF16>);
   else
     go(mpo_apply_kernel<IMG_TF32>);
@@ -400,7 +411,6 @@ int mpo_points_per_cta() { return kMpoThreads; }
 int pack_rows_per_cta() { return kPackRows; }
 
 int pack_rows_chunks_per_thread() { return 4; }
-int mpo_d_per_thread(int mode) { return mode == IMG_F64 ? 1 : kMpoVec; }
 
 // ---------------------------------------------------------------------------
 // FP64 vector primitives: deterministic two-pass reductions

@@ -21,12 +21,21 @@ void launch_zero_ranges(const uint64_t* out_tab, const DevChunk* chunks, int n_c
                         cudaStream_t st);
 void launch_scatter(const void* res, bool res_f32, double* out, const DevScatSeg* segs, const DevChunk* chunks,
                     int n_chunks, cudaStream_t st);
-void launch_mpo_apply(bool x1_f32, int mode, const DevMpoPair* pairs, const DevMpoSlot* islots,
+void launch_mpo_apply(int mode, const DevMpoPair* pairs, const DevMpoSlot* islots,
                       const DevMpoOutSlot* oslots, const DevMpoTerm* terms, const int2* chunks, int n_chunks,
                       size_t smem_bytes, const int32_t* skip, cudaStream_t st);
+// FP64 H_eff: the multi-term outputs, y[c,d] = sum of w * x[c,d] (slots: base address and c stride)
+void launch_mpo_sum(const DevMpoPair* pairs, const DevMpoSlot* islots, const DevMpoSlot* oslots,
+                    const DevMpoTerm* terms, const int2* chunks, int n_chunks, const int32_t* skip, cudaStream_t st);
 int mpo_points_per_cta();
-// consecutive d one MPO thread produces: the stage-4 d padding for the mixed images, 1 for FP64
-int mpo_d_per_thread(int mode);
+// blocks as rows of `inner` elements -> rows of `pitch`, nscale copies each times its scale, copy j at j * stride
+constexpr int kMaxScales = 8;
+struct DevPadSeg {
+  int64_t src_off, dst_off;
+  int32_t inner, pitch;
+};
+void launch_padded_copies(const double* src, double* dst, const DevPadSeg* segs, const DevChunk* chunks, int n_chunks,
+                          int64_t stride, const double* scale, int nscale, cudaStream_t st);
 // dst[seg.dst_off + sum idx_l dstr_l] = src[seg.src_off + e] for each chunk's range of elements e
 void launch_strided_copy(const double* src, double* dst, const DevCopySeg* segs, const DevChunk* chunks, int n_chunks,
                          cudaStream_t st);
