@@ -327,6 +327,15 @@ int tnx_svd_batch(int32_t n, const int64_t* m, const int64_t* k, const double* c
 int tnx_lanczos_step(double* w, const double* v, const double* v_prev, double* v_next, int64_t n, double* alpha,
                      double* beta, int32_t k, double tol, double tol_rel, int32_t* done, double* scratch,
                      void* stream);
+
+/* Issue a whole Krylov loop of a one-operator batch (dmrg.py:993-1019) on
+ * `stream`: basis[0] = x0 / (||x0|| + 1e-15), then num_steps times w = H_eff
+ * basis[k] and the step above.  basis holds num_steps + 1 vectors `ld`
+ * elements apart, n elements each; alpha num_steps, beta num_steps + 1 values;
+ * norm one double.  The batch's skip flag should be `done`. */
+int tnx_krylov_issue(tnx_heff_batch* b, const double* x0, double* basis, int64_t ld, int64_t n, int32_t num_steps,
+                     double* w, double* alpha, double* beta, double tol, double tol_rel, int32_t* done, double* norm,
+                     double* scratch, void* stream);
 /* out = sum_k coefs[k] * basis[k], summed left to right as the reference's
  * eigenvector reconstruction (dmrg.py:1038-1040); device pointer table and
  * device coefficients. */

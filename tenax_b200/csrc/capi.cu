@@ -1555,11 +1555,11 @@ namespace {
 // R times the term's weight, instead of one per output slot of a formed X3.
 // An output slot with a single term costs the same either way and is never
 // formed; one with several costs a product more per extra term, which on small
-// operators is less than the launch that would sum them first.  The limit is
-// where both cost the same, about 8 us: extra products at 30 TFLOP/s against a
-// launch and the slots' traffic (chi = 64 chain: 1e6 extra FLOPs; chi = 1024
-// cylinder: 4e9).
-constexpr double kF64ExtraFlops = 2.5e8;
+// operators is less than the launch that would sum them first.  Measured on
+// the cylinder, products against the summing launch: chi = 60 15.5 / 22.6 us,
+// 200 30.9 / 35.0, 300 54.0 / 55.4 (7e7 extra FLOPs), 400 95.5 / 90.1 (1.4e8),
+// 600 211 / 190.
+constexpr double kF64ExtraFlops = 1e8;
 constexpr size_t kF64Weights = 6;  // copies of R at most
 
 int64_t even(int64_t n) { return (n + 1) / 2 * 2; }
@@ -1807,6 +1807,11 @@ struct tnx_heff_batch {
   DevMem f64_oslots;
   std::vector<std::unique_ptr<DevMem>> f64_blobs;
   std::vector<ContractLaunch> f64_s1, f64_s4;  // one launch per K split among the operators
+  // FP64 of one operator: theta and the output travel as kernel arguments, so an
+  // apply with new buffers uploads nothing
+  const double* one_in = nullptr;
+  double* one_out = nullptr;
+  bool one() const { return mode == IMG_F64 && hs.size() == 1; }
   int n_launches = 0;
   std::vector<uint64_t> last_src, last_out;
   // host-resident streaming (tnx_heff_batch_apply_host): each problem's theta
@@ -1961,7 +1966,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
     }
   }
   b->x1.alloc(std::max<int64_t>(1, n1) * sizeof(double));
-  b->x3_img.alloc(std::max<int64_t>(1, n3) * sizeof(double));
+  b->x3_img.alloc(n3 * sizeof(double));
   const uint64_t x1_base = reinterpret_cast<uint64_t>(b->x1.p), x3_base = reinterpret_cast<uint64_t>(b->x3_img.p);
   std::vector<F64Stage> s1(n), s4(n);
   std::vector<DevMpoPair> MP;
@@ -2125,11 +2130,12 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
   upload(b->mpo_terms, MT);
   upload(b->mpo_chunks, MC);
   b->n_mpo_chunks = static_cast<int>(MC.size());
-  b->err.alloc(sizeof(int32_t));
-  CUDA_OK(cudaMemset(b->err.p, 0, sizeof(int32_t)));
-  b->src_tab.alloc(sizeof(PtrTab));
-  b->out_tab4.alloc(sizeof(PtrTab));
-  CUDA_OK(cudaDeviceSynchronize());
+  if (!b->one()) {
+    b->src_tab.alloc(sizeof(PtrTab));
+    b->out_tab4.alloc(sizeof(PtrTab));
+  }
+  // the tables were uploaded in the legacy stream; callers may use any other
+  CUDA_OK(cudaStreamSynchronize(nullptr));
   b->n_launches = static_cast<int>(b->f64_s1.size() + b->f64_s4.size()) + (b->n_mpo_chunks > 0 ? 1 : 0);
 }
 }  // namespace
@@ -2776,14 +2782,20 @@ int tnx_heff_batch_route_stats(const tnx_heff_batch* b, int64_t* n_routes, int32
 }
 
 // stage 0: pack theta; 1: stage-1 GEMM; 2: fused MPO; 3: stage-4 GEMM into theta layout.
-// src_tab / out_tab4: device pointer tables of the inputs (problem i) and outputs (slot 1 + i)
+// src_tab / out_tab4: device pointer tables of the inputs (problem i) and outputs (slot 1 + i); both null:
+// the single FP64 problem's one_in and one_out
 static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, const uint64_t* src_tab,
                              const uint64_t* out_tab4) {
   if (b->mode == IMG_F64) {
     // theta is read in place (stage 0 has nothing to pack)
     if (stage == 1 || stage == 3) {
       for (ContractLaunch L : stage == 1 ? b->f64_s1 : b->f64_s4) {
-        (stage == 1 ? L.b_ptrs : L.c_ptrs) = stage == 1 ? src_tab : out_tab4;
+        if (!src_tab) {
+          L.b = stage == 1 ? b->one_in : nullptr;
+          L.c = stage == 1 ? nullptr : b->one_out;
+        } else {
+          (stage == 1 ? L.b_ptrs : L.c_ptrs) = stage == 1 ? src_tab : out_tab4;
+        }
         L.skip = b->skip;
         CUDA_OK(launch_contract_f64(L, st));
       }
@@ -2832,6 +2844,13 @@ static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, cons
   }
 }
 
+static void heff_apply_one(tnx_heff_batch* b, const double* theta, double* out, cudaStream_t st) {
+  b->one_in = theta;
+  b->one_out = out;
+  for (int stage = 1; stage < 4; ++stage) heff_batch_stage(b, stage, st, nullptr, nullptr);
+  CUDA_OK(cudaGetLastError());
+}
+
 int tnx_heff_batch_apply(tnx_heff_batch* b, const double* const* thetas, double* const* outs, void* stream) {
   TNX_TRY({
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -2840,6 +2859,11 @@ int tnx_heff_batch_apply(tnx_heff_batch* b, const double* const* thetas, double*
     for (int i = 0; i < n; ++i) {
       src[i] = reinterpret_cast<uint64_t>(thetas[i]);
       o4[1 + i] = reinterpret_cast<uint64_t>(outs[i]);
+    }
+    if (b->one()) {
+      heff_apply_one(b, thetas[0], outs[0], st);
+      b->last_src = src;
+      return TNX_OK;
     }
     // pointer tables are re-uploaded only when they change, so an apply with
     // the same buffers issues kernels only (and can be captured in a graph)
@@ -2923,8 +2947,8 @@ int tnx_heff_batch_apply_stage(tnx_heff_batch* b, int32_t stage, void* stream) {
   TNX_TRY({
     if (stage < 0 || stage > 3) return set_err(TNX_ERR_VALUE, "stage must be 0..3");
     if (b->last_src.empty()) return set_err(TNX_ERR_VALUE, "call tnx_heff_batch_apply once first");
-    heff_batch_stage(b, stage, static_cast<cudaStream_t>(stream), b->src_tab.as<uint64_t>(),
-                     b->out_tab4.as<uint64_t>());
+    heff_batch_stage(b, stage, static_cast<cudaStream_t>(stream), b->one() ? nullptr : b->src_tab.as<uint64_t>(),
+                     b->one() ? nullptr : b->out_tab4.as<uint64_t>());
     CUDA_OK(cudaGetLastError());
     return TNX_OK;
   })
@@ -2941,7 +2965,8 @@ void tnx_heff_batch_destroy(tnx_heff_batch* b) { delete b; }
 
 int tnx_heff_batch_error(tnx_heff_batch* b, int32_t* err) {
   TNX_TRY({
-    CUDA_OK(cudaMemcpy(err, b->err.p, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    *err = 0;  // the FP64 kernels have no device-side wait to give up
+    if (b->err.p) CUDA_OK(cudaMemcpy(err, b->err.p, sizeof(int32_t), cudaMemcpyDeviceToHost));
     return TNX_OK;
   })
 }
@@ -3304,6 +3329,36 @@ int tnx_lanczos_step(double* w, const double* v, const double* v_prev, double* v
     launch_lanczos_step(w, v, k > 0 ? v_prev : nullptr, v_next, n, alpha + k, beta + k + 1, beta + k, tol, tol_rel,
                         done, scratch, static_cast<cudaStream_t>(stream));
     CUDA_OK(cudaGetLastError());
+    return TNX_OK;
+  })
+}
+
+int tnx_krylov_issue(tnx_heff_batch* b, const double* x0, double* basis, int64_t ld, int64_t n, int32_t num_steps,
+                     double* w, double* alpha, double* beta, double tol, double tol_rel, int32_t* done, double* norm,
+                     double* scratch, void* stream) {
+  TNX_TRY({
+    if (!b || !x0 || !basis || !w || !alpha || !beta || !done || !norm || !scratch)
+      return set_err(TNX_ERR_VALUE, "tnx_krylov_issue: null argument");
+    if (b->hs.size() != 1) return set_err(TNX_ERR_VALUE, "tnx_krylov_issue takes a batch of one operator");
+    if (n != b->th_total || ld < n || num_steps < 0)
+      return set_err(TNX_ERR_VALUE, "tnx_krylov_issue: vectors do not match the operator");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    launch_dot(x0, x0, n, 1, norm, scratch, nullptr, st);
+    launch_scale(x0, basis, n, norm, 2, nullptr, st);
+    for (int32_t k = 0; k < num_steps; ++k) {
+      const double* v = basis + k * ld;
+      if (b->one()) {
+        heff_apply_one(b, v, w, st);
+        b->last_src.assign(1, reinterpret_cast<uint64_t>(v));
+      } else {
+        double* o = w;
+        const int rc = tnx_heff_batch_apply(b, &v, &o, stream);
+        if (rc != TNX_OK) return rc;
+      }
+      launch_lanczos_step(w, v, k > 0 ? v - ld : nullptr, basis + (k + 1) * ld, n, alpha + k, beta + k + 1, beta + k,
+                          tol, tol_rel, done, scratch, st);
+      CUDA_OK(cudaGetLastError());
+    }
     return TNX_OK;
   })
 }

@@ -535,19 +535,167 @@ __global__ void finish_sum_kernel(const double* __restrict__ partials, int np, d
   if (threadIdx.x == 0) *result = op == 1 ? sqrt(acc) : acc;
 }
 
+// ---------------------------------------------------------------------------
+// One Lanczos step.  Vectors of up to kStepMax elements are worked in one
+// launch: one cluster holds w and v in registers (8 elements a thread), both
+// reductions go through distributed shared memory in rank order and nothing is
+// read twice.  On theta of the chi = 64 chain (1.7k elements) the step is
+// bound by launches: five kernels 11 us of device time and 15 us to issue, one
+// 3 us.  Longer vectors take three launches whose blocks each reduce
+// the previous launch's partial sums themselves (592 values from L2) instead of
+// waiting for a single-block kernel.
+// ---------------------------------------------------------------------------
+constexpr int kStepThreads = 1024;
+constexpr int kStepElems = 8;  // per thread
+constexpr int kStepCluster = 8;
+constexpr int64_t kStepMax = static_cast<int64_t>(kStepThreads) * kStepElems * kStepCluster;
+
+// total over the cluster's CTAs, in rank order, returned to every thread;
+// `slot` is a shared double no other reduction of this kernel uses
+__device__ __forceinline__ double cluster_total(double v, double* slot) {
+  v = block_sum(v);
+  if (threadIdx.x == 0) *slot = v;
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  double t = 0.0;
+  for (uint32_t r = 0; r < n; ++r) {
+    uint32_t a;
+    double p;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(slot)), "r"(r));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(p) : "r"(a) : "memory");
+    t = r == 0 ? p : t + p;
+  }
+  return t;
+}
+
+__device__ __forceinline__ void cluster_leave() {  // no CTA ends while a peer reads its shared memory
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kStepThreads)
+    lanczos_cluster_kernel(double* w, const double* v, const double* vp, double* vnext, int64_t n, double* alpha,
+                           double* beta_next, const double* beta_prev, double tol, double tol_rel, int32_t* done) {
+  if (*done) return;  // set by an earlier launch only, or by this one after every CTA has passed here
+  __shared__ double slots[2];
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kStepThreads;
+  const int64_t i0 = blockIdx.x * static_cast<int64_t>(kStepThreads) + threadIdx.x;
+  double wr[kStepElems], vr[kStepElems];
+  double acc = 0.0;
+#pragma unroll
+  for (int u = 0; u < kStepElems; ++u) {
+    const int64_t i = i0 + u * stride;
+    wr[u] = i < n ? w[i] : 0.0;
+    vr[u] = i < n ? v[i] : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < kStepElems; ++u) acc += vr[u] * wr[u];
+  const double a = cluster_total(acc, &slots[0]);
+  const double b = vp ? *beta_prev : 0.0;
+  acc = 0.0;
+#pragma unroll
+  for (int u = 0; u < kStepElems; ++u) {
+    const int64_t i = i0 + u * stride;
+    if (i >= n) continue;
+    double x = wr[u] - vr[u] * a;
+    if (vp) x = x - vp[i] * b;
+    wr[u] = x;
+    w[i] = x;
+    acc += x * x;
+  }
+  __syncthreads();  // block_sum's scratch is reused
+  const double bn = sqrt(cluster_total(acc, &slots[1]));
+  // beta < tol is the reference's absolute test; with an inexact matvec, also
+  // beta < tol_rel * |alpha| (below the matvec's noise)
+  const bool stop = bn < tol || bn < tol_rel * fabs(a);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *alpha = a;
+    *beta_next = bn;
+    if (stop) *done = 1;
+  }
+  if (vnext && !stop) {
+    const double f = 1.0 / bn;
+#pragma unroll
+    for (int u = 0; u < kStepElems; ++u) {
+      const int64_t i = i0 + u * stride;
+      if (i < n) vnext[i] = wr[u] * f;
+    }
+  }
+  cluster_leave();
+}
+
+// sum x*y (kind 0) or sqrt(sum x*x) (kind 1) of up to kStepMax elements
+__global__ void __launch_bounds__(kStepThreads)
+    dot_cluster_kernel(const double* __restrict__ x, const double* __restrict__ y, int64_t n, int kind,
+                       double* __restrict__ result, const int32_t* __restrict__ skip) {
+  if (skip && *skip) return;
+  __shared__ double slot;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kStepThreads;
+  double acc = 0.0;
+#pragma unroll
+  for (int u = 0; u < kStepElems; ++u) {
+    const int64_t i = blockIdx.x * static_cast<int64_t>(kStepThreads) + threadIdx.x + u * stride;
+    if (i < n) acc += x[i] * (kind ? x[i] : y[i]);
+  }
+  const double t = cluster_total(acc, &slot);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *result = kind == 1 ? sqrt(t) : t;
+  cluster_leave();
+}
+
+// CTAs of the cluster: about 2 elements a thread, then up to 8 (1.7k elements:
+// 6.3 us with 1 CTA, 7.2 with 8; 8k: 8.5 with 1, 6.9 with 4; 64k: 10.1 with 8)
+static int step_ctas(int64_t n) {
+  int c = 1;
+  while (c < kStepCluster && static_cast<int64_t>(c) * kStepThreads * 2 < n) c *= 2;
+  return c;
+}
+
+template <typename K, typename... Args>
+static void launch_cluster(K kernel, int ctas, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kStepThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  // a failure is the thread's last CUDA error, checked by every caller
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 void launch_dot(const double* x, const double* y, int64_t n, int kind, double* result, double* partials,
                 const int32_t* skip, cudaStream_t st) {
+  if (n <= kStepMax) {
+    launch_cluster(dot_cluster_kernel, step_ctas(n), st, x, y, n, kind, result, skip);
+    return;
+  }
   partial_dot_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(x, y, n, kind, partials, skip);
   finish_sum_kernel<<<1, 1024, 0, st>>>(partials, kRedBlocks, result, kind, skip);
 }
 
-// w -= alpha v (+ beta v_prev); partial sums of w*w
+// the sum of kRedBlocks partials, in the same order in every block
+__device__ __forceinline__ double partials_total(const double* __restrict__ p) {
+  __shared__ double tot;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < kRedBlocks; i += kRedThreads) acc += p[i];
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) tot = acc;
+  __syncthreads();
+  return tot;
+}
+
+// alpha from the partial products, w -= alpha v (+ beta v_prev), partial sums of w*w
 __global__ void lanczos_axpy_kernel(double* __restrict__ w, const double* __restrict__ v,
-                                    const double* __restrict__ vp, int64_t n, const double* __restrict__ alpha,
-                                    const double* __restrict__ beta, double* __restrict__ partials,
-                                    const int32_t* __restrict__ skip) {
+                                    const double* __restrict__ vp, int64_t n, double* __restrict__ alpha,
+                                    const double* __restrict__ beta, const double* __restrict__ pdot,
+                                    double* __restrict__ pnorm, const int32_t* __restrict__ skip) {
   if (skip && *skip) return;
-  const double a = *alpha;
+  const double a = partials_total(pdot);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *alpha = a;
   const double b = vp ? *beta : 0.0;
   double acc = 0.0;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -558,23 +706,29 @@ __global__ void lanczos_axpy_kernel(double* __restrict__ w, const double* __rest
     acc += x * x;
   }
   acc = block_sum(acc);
-  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+  if (threadIdx.x == 0) pnorm[blockIdx.x] = acc;
 }
 
-// beta = ||w||; stop when beta < tol (the reference's absolute test) or, with
-// an inexact matvec, when beta < tol_rel * |alpha| (below the matvec's noise)
-__global__ void lanczos_beta_kernel(const double* __restrict__ partials, int np, double* __restrict__ beta_out,
-                                    const double* __restrict__ alpha, double tol, double tol_rel,
-                                    int32_t* __restrict__ done) {
+// beta = ||w|| from the partial sums; stop when beta < tol (the reference's
+// absolute test) or, with an inexact matvec, when beta < tol_rel * |alpha|
+// (below the matvec's noise); otherwise v_next = w / beta.  A block that finds
+// *done set by block 0 of this launch has nothing to write: every block makes
+// the same decision.
+__global__ void lanczos_next_kernel(const double* w, double* vnext, int64_t n, const double* __restrict__ pnorm,
+                                    double* __restrict__ beta_out, const double* __restrict__ alpha, double tol,
+                                    double tol_rel, int32_t* done) {
   if (*done) return;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) acc += partials[i];
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) {
-    double b = sqrt(acc);
+  const double b = sqrt(partials_total(pnorm));
+  const bool stop = b < tol || b < tol_rel * fabs(*alpha);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     *beta_out = b;
-    if (b < tol || b < tol_rel * fabs(*alpha)) *done = 1;
+    if (stop) *done = 1;
   }
+  if (stop || !vnext) return;
+  const double f = 1.0 / b;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    vnext[i] = w[i] * f;
 }
 
 __global__ void scale_into_kernel(const double* __restrict__ w, double* __restrict__ out, int64_t n,
@@ -591,12 +745,16 @@ __global__ void scale_into_kernel(const double* __restrict__ w, double* __restri
 void launch_lanczos_step(double* w, const double* v, const double* vp, double* vnext, int64_t n, double* alpha,
                          double* beta_next, const double* beta_prev, double tol, double tol_rel, int32_t* done,
                          double* partials, cudaStream_t st) {
-  // alpha = <v, w>
+  if (n <= kStepMax) {
+    launch_cluster(lanczos_cluster_kernel, step_ctas(n), st, w, v, vp, vnext, n, alpha, beta_next, beta_prev, tol,
+                   tol_rel, done);
+    return;
+  }
   partial_dot_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(v, w, n, 0, partials, done);
-  finish_sum_kernel<<<1, 1024, 0, st>>>(partials, kRedBlocks, alpha, 0, done);
-  lanczos_axpy_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, v, vp, n, alpha, beta_prev, partials, done);
-  lanczos_beta_kernel<<<1, 1024, 0, st>>>(partials, kRedBlocks, beta_next, alpha, tol, tol_rel, done);
-  if (vnext) scale_into_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, vnext, n, beta_next, 1, done);
+  lanczos_axpy_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, v, vp, n, alpha, beta_prev, partials,
+                                                          partials + kRedBlocks, done);
+  lanczos_next_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, vnext, n, partials + kRedBlocks, beta_next, alpha, tol,
+                                                          tol_rel, done);
 }
 
 void launch_scale(const double* w, double* out, int64_t n, const double* s, int mode, const int32_t* skip,
@@ -620,7 +778,7 @@ void launch_combine(const double* const* basis, const double* coefs, int nv, int
   combine_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(basis, coefs, nv, n, out);
 }
 
-int reduce_partials_count() { return kRedBlocks; }
+int reduce_partials_count() { return 2 * kRedBlocks; }  // a step's two reductions
 
 // ---------------------------------------------------------------------------
 // Max-abs renormalisation of a batch of tensors and its adjoint.

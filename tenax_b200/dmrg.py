@@ -186,7 +186,7 @@ def lanczos(op: HeffOperator, theta: SymmetricTensor, num_steps: int, tol: float
         # Rayleigh quotient of the Ritz vector with the FP64 operator
         hv = fp64_op.apply(vec)
         energy = float(vector.dot(vec, hv)) / float(vector.dot(vec, vec))
-    full = SymmetricTensor.from_flat(theta.indices, op.keys, vec)
+    full = theta._like(vec) if theta.keys == op.keys else SymmetricTensor.from_flat(theta.indices, op.keys, vec)
     result = restrict_to_keys(full, keys)
     return energy, result, LanczosStats(m, a[:m], b[1:m + 1], time.perf_counter() - t0)
 
@@ -231,16 +231,20 @@ def _krylov(op: HeffOperator, x0: torch.Tensor, num_steps: int, tol: float, tol_
 
     def issue(x_in, scr, nrm):
         st = torch.cuda.current_stream().cuda_stream
+        if batch is not None and x_in is None:
+            # every launch of the loop from one native call
+            _capi.check(_capi.LIB.tnx_krylov_issue(
+                batch.handle, x0.data_ptr(), basis.data_ptr(), basis.stride(0), n, num_steps, w.data_ptr(),
+                alpha.data_ptr(), beta.data_ptr(), float(tol), float(tol_rel), done.data_ptr(), nrm.data_ptr(),
+                scr.data_ptr(), st))
+            return
         _capi.check(_capi.LIB.tnx_nrm2(x0.data_ptr(), n, nrm.data_ptr(), scr.data_ptr(), st))
         _capi.check(_capi.LIB.tnx_scale(x0.data_ptr(), basis[0].data_ptr(), n, nrm.data_ptr(), 2, st))
         for k in range(num_steps):
             if batch is not None:
-                if x_in is not None:
-                    # fixed matvec input: the batch's pointer tables never change inside a graph
-                    x_in[:n].copy_(basis[k, :n])
-                    batch.apply([x_in[:n]], [w[:n]])
-                else:
-                    batch.apply([basis[k, :n]], [w[:n]])
+                # fixed matvec input: the batch's pointer tables never change inside a graph
+                x_in[:n].copy_(basis[k, :n])
+                batch.apply([x_in[:n]], [w[:n]])
             else:
                 if k > 0 and k % _GENERAL_DONE_POLL == 0 and int(done.item()) != 0:
                     break
