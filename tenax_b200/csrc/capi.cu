@@ -207,6 +207,31 @@ void build_tiles(const PairPlan& P, const PairGeom& G, int group_base, std::vect
       for (int nt = 0; nt < G.nNt[g]; ++nt) tl.push_back({G.nKt[g], DevTile{group_base + static_cast<int>(g), mt, nt, 0}});
 }
 
+// A tcgen05 launch of fewer 128-column tiles than SMs, cut to 64 or 32 columns
+// until they cover the SMs.  Every element keeps its own accumulation order, so
+// the results are the same bits.  H_eff stage 4 in TF32 at chi = 512 (about 70
+// tiles of up to 92 K slabs): 34.4 us in 128 columns, 31.3 in 32.
+// Returns the tiles' width.
+int narrow_tiles(std::vector<std::pair<int64_t, DevTile>>& tl, const std::vector<DevGroup>& groups) {
+  const size_t sms = static_cast<size_t>(device_sm_count());
+  if (tl.size() >= sms) return 128;
+  int last = 128;
+  std::vector<std::pair<int64_t, DevTile>> out;
+  for (int width : {64, 32}) {
+    out.clear();
+    last = width;
+    for (const auto& t : tl)
+      for (int sub = 0; sub < 128 && t.second.nt * 128 + sub < groups[t.second.g].N; sub += width) {
+        DevTile d = t.second;
+        d.sub = width << 16 | sub;
+        out.push_back({t.first, d});
+      }
+    if (out.size() >= sms) break;
+  }
+  tl.swap(out);
+  return last;
+}
+
 std::vector<DevTile> sorted_tiles(std::vector<std::pair<int64_t, DevTile>>& tl) {
   std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
   std::vector<DevTile> out;
@@ -215,7 +240,7 @@ std::vector<DevTile> sorted_tiles(std::vector<std::pair<int64_t, DevTile>>& tl) 
   return out;
 }
 
-void gemm_launch(int mode, const DevMem& groups, const DevMem& tiles, int n_tiles, const DevMem& rowoff,
+void gemm_launch(int mode, const DevMem& groups, const DevMem& tiles, int n_tiles, int width, const DevMem& rowoff,
                  const PtrTab& out_tab, bool out_f64, int32_t* err, const int32_t* skip, cudaStream_t st,
                  DevMem& out_tab_dev) {
   // out_tab travels through a small device array (kernels index it per group)
@@ -225,7 +250,7 @@ void gemm_launch(int mode, const DevMem& groups, const DevMem& tiles, int n_tile
                     out_tab_dev.as<uint64_t>(), skip, st);
   else
     launch_gemm_tc(mode, groups.as<DevGroup>(), tiles.as<DevTile>(), n_tiles, rowoff.as<int64_t>(),
-                   out_tab_dev.as<uint64_t>(), out_f64, err, skip, st);
+                   out_tab_dev.as<uint64_t>(), out_f64, err, skip, st, width);
 }
 }  // namespace
 
@@ -238,7 +263,7 @@ struct StepDev {
   DevMem a_img, b_img, c_res;  // images and result matrices
   int64_t a_lo = 0, b_lo = 0;
   DevMem packA, chunksA, packB, chunksB, groups, tiles, rowoff, scat, chunksS, out_tab;
-  int nA = 0, nB = 0, nT = 0, nS = 0;
+  int nA = 0, nB = 0, nT = 0, nS = 0, width = 128;
   bool res_f32 = false;
   // FP64 in one launch (contract_f64.cu): tables of the step in one buffer
   bool direct = false, swapped = false;
@@ -918,6 +943,7 @@ static void plan_build_device(tnx_plan* p, int precision) {
     upload(d->rowoff, ro);
     std::vector<std::pair<int64_t, DevTile>> tl;
     build_tiles(P, d->G, 0, tl);
+    if (mode != IMG_F64) d->width = narrow_tiles(tl, gr);
     auto tiles = sorted_tiles(tl);
     upload(d->tiles, tiles);
     d->nT = static_cast<int>(tiles.size());
@@ -993,7 +1019,7 @@ int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, i
                   st);
       PtrTab ot{};
       ot.p[0] = reinterpret_cast<uint64_t>(d.c_res.p);
-      gemm_launch(d.mode, d.groups, d.tiles, d.nT, d.rowoff, ot, false, plan->err_flag.as<int32_t>(), nullptr, st,
+      gemm_launch(d.mode, d.groups, d.tiles, d.nT, d.width, d.rowoff, ot, false, plan->err_flag.as<int32_t>(), nullptr, st,
                   d.out_tab);
       if (P.out.total > 0)
         CUDA_OK(cudaMemsetAsync(o_ptr, 0, P.out.total * sizeof(double), st));
@@ -1782,7 +1808,7 @@ struct tnx_heff_batch {
   int n_th_row_chunks = 0;
   bool th_by_rows = false;
   DevMem g1, t1, ro1, g4, t4, ro4;
-  int n_t1 = 0, n_t4 = 0;
+  int n_t1 = 0, n_t4 = 0, width1 = 128, width4 = 128;
   DevMem mpo_pairs, mpo_slots, mpo_oslots, mpo_terms, mpo_chunks;
   int n_mpo_chunks = 0;
   size_t mpo_smem = 16;
@@ -2640,6 +2666,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     }
     upload(b->g1, G1);
     upload(b->ro1, R1);
+    if (!rt) b->width1 = narrow_tiles(T1, G1);  // the routed epilogue's windows are per 128-column tile
     auto t1 = sorted_tiles(T1);
     upload(b->t1, t1);
     if (rt) {
@@ -2678,6 +2705,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     b->n_t1 = static_cast<int>(t1.size());
     upload(b->g4, G4);
     upload(b->ro4, R4);
+    b->width4 = narrow_tiles(T4, G4);
     auto t4 = sorted_tiles(T4);
     upload(b->t4, t4);
     b->n_t4 = static_cast<int>(t4.size());
@@ -2827,7 +2855,7 @@ static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, cons
       break;
     case 1:
       launch_gemm_tc(b->mode, b->g1.as<DevGroup>(), b->t1.as<DevTile>(), b->n_t1, b->ro1.as<int64_t>(),
-                       b->out_tab1.as<uint64_t>(), false, b->err.as<int32_t>(), b->skip, st,
+                       b->out_tab1.as<uint64_t>(), false, b->err.as<int32_t>(), b->skip, st, b->width1,
                        b->routed ? DevRouteTabs{b->x3_lo, b->routes.as<DevRoute>(), b->route_win.as<int2>(),
                                                 b->route_rows.as<int2>(), b->route_cols.as<int2>()}
                                  : DevRouteTabs{});
@@ -2840,7 +2868,7 @@ static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, cons
     default:
       launch_zero_ranges(out_tab4, b->zero_chunks.as<DevChunk>(), b->n_zero_chunks, b->skip, st);
       launch_gemm_tc(b->mode, b->g4.as<DevGroup>(), b->t4.as<DevTile>(), b->n_t4, b->ro4.as<int64_t>(),
-                       out_tab4, true, b->err.as<int32_t>(), b->skip, st);
+                       out_tab4, true, b->err.as<int32_t>(), b->skip, st, b->width4);
   }
 }
 

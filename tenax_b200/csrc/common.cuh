@@ -158,7 +158,8 @@ struct DevRouteTabs {
 };
 
 struct DevTile {
-  int32_t g, mt, nt, pad;
+  int32_t g, mt, nt;
+  int32_t sub;  // tcgen05: columns of a narrow tile << 16 | its first column inside the 128-column tile; 0: all 128
 };
 
 struct DevMpoPair {

@@ -40,6 +40,23 @@ constexpr int THREADS = 64 + 32 * EPI_WARPS;
 #endif
 constexpr int NACC = TNX_TMEM_ACC;
 static_assert(NACC == 2 || NACC == 4, "TMEM accumulators: 2 or 4 (512 columns)");
+// The columns and operand rows a tile works on.  Loads are trimmed to the rows
+// the group has (whole 8-row swizzle atoms of A, the MMA's N of B): rows of the
+// stage past them hold older bytes, which reach only result rows and columns
+// that are not stored.  A launch of fewer tiles than SMs leaves SMs idle; the
+// host then cuts tiles to 64 or 32 columns (narrow_tiles).
+struct TileCols {
+  int col0, ncols, width;  // first column, valid columns, columns of the tile
+  uint32_t a_bytes, b_bytes;
+  __device__ __forceinline__ TileCols(const DevTile& tl, const DevGroup& g) {
+    width = tl.sub ? tl.sub >> 16 : 128;
+    col0 = tl.nt * 128 + (tl.sub & 0xffff);
+    ncols = min(g.N - col0, width);
+    a_bytes = static_cast<uint32_t>((min(128, g.M - tl.mt * 128) + 7) & ~7) * 128u;
+    b_bytes = static_cast<uint32_t>((ncols + 15) & ~15) * 128u;
+  }
+};
+
 // The persistent loop over a CTA's tiles with the descriptors of the next
 // tiles in flight: the group record of tile t+1 and the tile record of t+2
 // are requested while tile t is processed, so no role waits on the
@@ -175,9 +192,12 @@ template <bool TF32, typename OutT, bool ROUTED>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_tc_kernel(const DevGroup* __restrict__ groups, const DevTile* __restrict__ tiles, int n_tiles,
                    const int64_t* __restrict__ rowoff, const uint64_t* __restrict__ out_tab, int32_t* err_flag,
-                   const int32_t* __restrict__ skip, const DevRouteTabs rt) {
+                   const int32_t* __restrict__ skip, const DevRouteTabs rt, const int width_) {
   constexpr int NT = TF32 ? 2 : 4;          // operand tiles per stage
   constexpr int STAGES = gemm_tc_stages<TF32, ROUTED>();  // 192 KB of operand ring (128 KB routed)
+  // narrow tiles (one width a launch) take smaller stages, so more of them: a
+  // tile's K chain runs at (stages in flight) / (latency of a copy)
+  constexpr int MAXS = ROUTED ? STAGES : (TF32 ? 9 : 4);
   constexpr int KSUB = 4;                   // MMAs per 128-byte K slab (32 B each)
   // TMEM accumulators: the routed instance runs 4 (all 512 columns), so the
   // MMAs run up to three tiles ahead of its longer epilogue
@@ -189,24 +209,28 @@ __global__ void __launch_bounds__(THREADS, 1)
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * NT * TILE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;
+  uint64_t* empty = full + MAXS;
+  uint64_t* tfull = empty + MAXS;
   uint64_t* tempty = tfull + NACC;
   uint64_t* drain = tempty + NACC;
   // split BF16: each stage lands in two halves, the hi planes of A and B on
   // full[s] and the lo planes on full2[s], so the hi x hi products start
   // while the lo planes are still in flight
   uint64_t* full2 = drain + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(full2 + (TF32 ? 0 : STAGES));
-  static_assert((2 * STAGES + 2 * NACC + 1 + (TF32 ? 0 : STAGES)) * 8 + 8 <= 256,
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(full2 + (TF32 ? 0 : MAXS));
+  static_assert((2 * MAXS + 2 * NACC + 1 + (TF32 ? 0 : MAXS)) * 8 + 8 <= 256,
                 "barriers, TMEM address and abort flag fit the 256 bytes before the epilogue staging");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   // epilogue staging: one 32 x 33 fp32 buffer per epilogue warp, after 256 B of barriers
   float* epi_stage = reinterpret_cast<float*>(smem + STAGES * NT * TILE_BYTES + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int width = ROUTED ? TBN : width_;  // columns of this launch's tiles
+  const uint32_t b_tile = static_cast<uint32_t>(width) * 128u;               // bytes of one B plane of a stage
+  const uint32_t stage_bytes = static_cast<uint32_t>(NT / 2) * (TILE_BYTES + b_tile);
+  const int nst = width == TBN ? STAGES : min(MAXS, STAGES * NT * TILE_BYTES / static_cast<int>(stage_bytes));
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < nst; ++s) {
       mbar_init(&full[s], 1);
       if (!TF32) mbar_init(&full2[s], 1);
       mbar_init(&empty[s], 1);
@@ -232,48 +256,54 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    {
+      const uint32_t lead = elect_one();
+      const uint32_t ring0 = smem_u32(smem), full0 = smem_u32(full), full20 = smem_u32(full2);
       int s = 0;
       uint32_t ph = 0;
-      int last_par[STAGES];
-      for (int i = 0; i < STAGES; ++i) last_par[i] = -1;
+      int last_par[MAXS];
+      for (int i = 0; i < MAXS; ++i) last_par[i] = -1;
       bool ok = true;
       for (TileIter it(tiles, groups, n_tiles, blockIdx.x); it.t < n_tiles && ok; it.advance()) {
         it.prefetch();
-        const DevTile tl = it.tl;
-        const DevGroup g = it.g;
-        const uint8_t* ga = reinterpret_cast<const uint8_t*>(g.a_addr) + static_cast<int64_t>(tl.mt) * g.nKt * TILE_BYTES;
-        const uint8_t* gb = reinterpret_cast<const uint8_t*>(g.b_addr) + static_cast<int64_t>(tl.nt) * g.nKt * TILE_BYTES;
-        for (int kt = 0; kt < g.nKt; ++kt) {
-          if (!wait_or_abort(&empty[s], ph ^ 1u, abort_flag, err_flag)) {
+        const TileCols tc(it.tl, it.g);
+        const uint8_t* ga =
+            reinterpret_cast<const uint8_t*>(it.g.a_addr) + static_cast<int64_t>(it.tl.mt) * it.g.nKt * TILE_BYTES;
+        const uint8_t* gb = reinterpret_cast<const uint8_t*>(it.g.b_addr) +
+                            static_cast<int64_t>(it.tl.nt) * it.g.nKt * TILE_BYTES + (tc.col0 - it.tl.nt * TBN) * 128;
+        const int64_t a_lo = it.g.a_lo, b_lo = it.g.b_lo;
+        const uint32_t ab = warp_uniform(tc.a_bytes), bb = warp_uniform(tc.b_bytes);
+        const int nKt = static_cast<int>(warp_uniform(it.g.nKt));
+        for (int kt = 0; kt < nKt; ++kt) {
+          if (!warp_wait_or_abort(&empty[s], ph ^ 1u, abort_flag, err_flag)) {
             ok = false;
             break;
           }
-          uint8_t* st = smem + s * NT * TILE_BYTES;
+          const uint32_t st = ring0 + s * stage_bytes, fb = full0 + 8 * s, fb2 = full20 + 8 * s;
           const int64_t ko = static_cast<int64_t>(kt) * TILE_BYTES;
           if (TF32) {
-            mbar_expect_tx(&full[s], NT * TILE_BYTES);
-            bulk_g2s(st, ga + ko, TILE_BYTES, &full[s]);
-            bulk_g2s(st + TILE_BYTES, gb + ko, TILE_BYTES, &full[s]);
+            mbar_expect_tx_on(lead, fb, ab + bb);
+            bulk_g2s_on(lead, st, ga + ko, ab, fb);
+            bulk_g2s_on(lead, st + TILE_BYTES, gb + ko, bb, fb);
           } else {
             // stage layout [A hi][A lo][B hi][B lo]; hi planes first
-            mbar_expect_tx(&full[s], 2 * TILE_BYTES);
-            bulk_g2s(st, ga + ko, TILE_BYTES, &full[s]);
-            bulk_g2s(st + 2 * TILE_BYTES, gb + ko, TILE_BYTES, &full[s]);
-            mbar_expect_tx(&full2[s], 2 * TILE_BYTES);
-            bulk_g2s(st + TILE_BYTES, ga + g.a_lo + ko, TILE_BYTES, &full2[s]);
-            bulk_g2s(st + 3 * TILE_BYTES, gb + g.b_lo + ko, TILE_BYTES, &full2[s]);
+            mbar_expect_tx_on(lead, fb, ab + bb);
+            bulk_g2s_on(lead, st, ga + ko, ab, fb);
+            bulk_g2s_on(lead, st + 2 * TILE_BYTES, gb + ko, bb, fb);
+            mbar_expect_tx_on(lead, fb2, ab + bb);
+            bulk_g2s_on(lead, st + TILE_BYTES, ga + a_lo + ko, ab, fb2);
+            bulk_g2s_on(lead, st + 2 * TILE_BYTES + b_tile, gb + b_lo + ko, bb, fb2);
           }
           last_par[s] = static_cast<int>(ph);
-          if (++s == STAGES) {
+          if (++s == nst) {
             s = 0;
             ph ^= 1u;
           }
         }
       }
       if (!ok) {
-        // let every copy this thread issued land before the CTA exits
-        for (int i = 0; i < STAGES; ++i) {
+        // let every copy this warp issued land before the CTA exits
+        for (int i = 0; i < MAXS; ++i) {
           if (last_par[i] < 0) continue;
           uint64_t t0 = gtimer();
           while (!mbar_try_wait(&full[i], static_cast<uint32_t>(last_par[i])) && gtimer() - t0 < kTimeoutNs) {
@@ -287,10 +317,18 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // The whole warp walks the loop and one elected lane issues, from 32-bit
+    // descriptor words and without a branch per MMA.  Inside a lane == 0 branch
+    // a split-BF16 slab of 12 MMAs took 1090 clocks and a TF32 slab of 4 took 520
+    // whatever N was; now 810 and 370 (128 columns of split BF16 need 768).  K =
+    // 8192, one tile: split BF16 78.8 -> 57.4 us, TF32 75.4 -> 51.7 us.
+    {
+      const uint32_t lead = elect_one();
       // instruction descriptor without N: FP32 accumulate, operand kinds, M = 128
       const uint32_t idesc0 = (1u << 4) | ((TF32 ? 2u : 1u) << 7) | ((TF32 ? 2u : 1u) << 10) |
                               (static_cast<uint32_t>(TBM >> 4) << 24);
+      const uint32_t tmem0 = warp_uniform(tmem_base);
+      const uint32_t ring0 = smem_u32(smem);
       int s = 0;
       uint32_t ph = 0;
       int acc = 0;
@@ -299,76 +337,77 @@ __global__ void __launch_bounds__(THREADS, 1)
       bool issued = false;
       for (TileIter it(tiles, groups, n_tiles, blockIdx.x); it.t < n_tiles && ok; it.advance()) {
         it.prefetch();
-        const DevTile tl = it.tl;
-        const DevGroup g = it.g;
         // MMA extent trimmed to the tile's valid columns (rounded to 16) and
         // the last slab's valid K steps: the operand images are zero beyond
         // both, so the skipped products are exact zeros
-        int ncols = g.N - tl.nt * TBN;
-        ncols = ncols > TBN ? TBN : ncols;
-        const uint32_t n_mma = static_cast<uint32_t>((ncols + 15) / 16 * 16);
+        const uint32_t n_mma = warp_uniform((TileCols(it.tl, it.g).ncols + 15) / 16 * 16);
         const uint32_t idesc = idesc0 | ((n_mma >> 3) << 17);
-        const int ksub_last = g.kk_last > 0 ? g.kk_last : KSUB;
-        if (!wait_or_abort(&tempty[acc], aph ^ 1u, abort_flag, err_flag)) {
+        const int nKt = static_cast<int>(warp_uniform(it.g.nKt));
+        const int ksub_last = static_cast<int>(warp_uniform(it.g.kk_last > 0 ? it.g.kk_last : KSUB));
+        if (!warp_wait_or_abort(&tempty[acc], aph ^ 1u, abort_flag, err_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * TBN);
-        for (int kt = 0; kt < g.nKt; ++kt) {
-          if (!wait_or_abort(&full[s], ph, abort_flag, err_flag)) {
+        const uint32_t d_tmem = tmem0 + static_cast<uint32_t>(acc * TBN);
+        for (int kt = 0; kt < nKt; ++kt) {
+          if (!warp_wait_or_abort(&full[s], ph, abort_flag, err_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * NT * TILE_BYTES);
-          const uint64_t da = sw128_desc(sa);
-          const int nk = kt + 1 == g.nKt ? ksub_last : KSUB;
+          const uint32_t sa = ring0 + s * stage_bytes;
+          const uint32_t da = sw128_lo(sa);
+          const int nk = kt + 1 == nKt ? ksub_last : KSUB;
           if (TF32) {
-            const uint64_t db = sw128_desc(sa + TILE_BYTES);
-#pragma unroll
-            for (int kk = 0; kk < KSUB; ++kk)
-              if (kk < nk) mma_issue<TF32>(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kt | kk) ? 1u : 0u);
-          } else {
-            const uint64_t dal = sw128_desc(sa + TILE_BYTES);
-            const uint64_t db = sw128_desc(sa + 2 * TILE_BYTES);
-            const uint64_t dbl = sw128_desc(sa + 3 * TILE_BYTES);
-            // hi x hi on the hi planes, then hi x lo and lo x hi once the lo planes land
-#pragma unroll
-            for (int kk = 0; kk < KSUB; ++kk) {
-              if (kk >= nk) break;
-              mma_issue<TF32>(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kt | kk) ? 1u : 0u);
+            if (lead) {
+              mma_slab<TF32>(d_tmem, da, sw128_lo(sa + TILE_BYTES), idesc, kt ? 1u : 0u, nk);
+              mma_commit(&empty[s]);
             }
+          } else {
+            const uint32_t dal = sw128_lo(sa + TILE_BYTES);
+            const uint32_t db = sw128_lo(sa + 2 * TILE_BYTES);
+            const uint32_t dbl = sw128_lo(sa + 2 * TILE_BYTES + b_tile);
+            // hi x hi on the hi planes, then hi x lo and lo x hi once the lo planes land
+            if (lead) mma_slab<TF32>(d_tmem, da, db, idesc, kt ? 1u : 0u, nk);
             issued = true;  // an abort below still waits for these MMAs before TMEM is freed
-            if (!wait_or_abort(&full2[s], ph, abort_flag, err_flag)) {
+            if (!warp_wait_or_abort(&full2[s], ph, abort_flag, err_flag)) {
               ok = false;
               break;
             }
             tc_fence_after();
+            if (lead) {
+              if (nk == KSUB) {
 #pragma unroll
-            for (int kk = 0; kk < KSUB; ++kk) {
-              if (kk >= nk) break;
-              mma_issue<TF32>(d_tmem, da + 2 * kk, dbl + 2 * kk, idesc, 1u);
-              mma_issue<TF32>(d_tmem, dal + 2 * kk, db + 2 * kk, idesc, 1u);
+                for (int kk = 0; kk < KSUB; ++kk) {
+                  mma_issue_lo<TF32>(d_tmem, da + 2 * kk, dbl + 2 * kk, idesc, 1u);
+                  mma_issue_lo<TF32>(d_tmem, dal + 2 * kk, db + 2 * kk, idesc, 1u);
+                }
+              } else {
+                for (int kk = 0; kk < nk; ++kk) {
+                  mma_issue_lo<TF32>(d_tmem, da + 2 * kk, dbl + 2 * kk, idesc, 1u);
+                  mma_issue_lo<TF32>(d_tmem, dal + 2 * kk, db + 2 * kk, idesc, 1u);
+                }
+              }
+              mma_commit(&empty[s]);
             }
           }
           issued = true;
-          mma_commit(&empty[s]);
-          if (++s == STAGES) {
+          if (++s == nst) {
             s = 0;
             ph ^= 1u;
           }
         }
         if (!ok) break;
-        mma_commit(&tfull[acc]);
+        if (lead) mma_commit(&tfull[acc]);
         if (++acc == NACC) {
           acc = 0;
           aph ^= 1u;
         }
       }
       if (!ok && issued) {
-        // wait for every MMA this thread issued before TMEM is freed
-        mma_commit(drain);
+        // wait for every MMA this warp issued before TMEM is freed
+        if (lead) mma_commit(drain);
         uint64_t t0 = gtimer();
         while (!mbar_try_wait(drain, 0) && gtimer() - t0 < kTimeoutNs) {
         }
@@ -567,8 +606,10 @@ __global__ void __launch_bounds__(THREADS, 1)
       // fragments; otherwise each lane holds one row (32x32b) and 32x32
       // chunks are staged through shared memory so that every store
       // instruction writes 32 consecutive columns of one row.
+      const TileCols tc(tl, g);
+      const int c_end = min(tc.width, (sizeof(OutT) == 4 && g.vec_ld > 0 ? g.vec_ld : g.N) - tc.col0);  // columns to store
 #pragma unroll 1
-      for (int c0 = c_begin; c0 < c_begin + kColsPerWarp; c0 += 32) {
+      for (int c0 = c_begin; c0 < c_begin + kColsPerWarp && c0 < c_end; c0 += 32) {
         bool done = false;
         if constexpr (sizeof(OutT) == 4) {
           if (g.vec_ld > 0) {
@@ -581,7 +622,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             tmem_ld16x256b_x4(tbase + (16u << 16) + c0, v1);
             tmem_wait_ld();
             const float fs = static_cast<float>(scale);
-            const int cl = tl.nt * TBN + c0 + 2 * (lane & 3);
+            const int cl = tc.col0 + c0 + 2 * (lane & 3);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               const uint32_t(&v)[16] = h ? v1 : v0;
@@ -610,7 +651,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) stg[lane * kStagePitch + j] = __uint_as_float(v[j]);
           __syncwarp();
-          const int col = tl.nt * TBN + c0 + lane;
+          const int col = tc.col0 + c0 + lane;
           const bool col_ok = col < g.N;
 #pragma unroll 4
           for (int r = 0; r < 32; ++r) {
@@ -642,7 +683,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 template <bool TF32, typename OutT, bool ROUTED>
 void launch_tc_impl(const DevGroup* groups, const DevTile* tiles, int n_tiles, const int64_t* rowoff,
                     const uint64_t* out_tab, int32_t* err_flag, const int32_t* skip, cudaStream_t st,
-                    const DevRouteTabs& rt) {
+                    const DevRouteTabs& rt, int width) {
   constexpr int smem = gemm_tc_smem<TF32, ROUTED>();
   if (cudaFuncSetAttribute(gemm_tc_kernel<TF32, OutT, ROUTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
@@ -650,29 +691,29 @@ void launch_tc_impl(const DevGroup* groups, const DevTile* tiles, int n_tiles, c
   int grid = device_sm_count();
   if (grid > n_tiles) grid = n_tiles;
   gemm_tc_kernel<TF32, OutT, ROUTED>
-      <<<grid, THREADS, smem, st>>>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, rt);
+      <<<grid, THREADS, smem, st>>>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, rt, width);
 }
 }  // namespace
 
 void launch_gemm_tc(int mode, const DevGroup* groups, const DevTile* tiles, int n_tiles, const int64_t* rowoff,
                     const uint64_t* out_tab, bool out_f64, int32_t* err_flag, const int32_t* skip, cudaStream_t st,
-                    const DevRouteTabs& rt) {
+                    int width, const DevRouteTabs& rt) {
   if (n_tiles <= 0) return;
   const bool routed = rt.win != nullptr;  // every group routed, FP32 results
   if (mode == IMG_TF32) {
     if (out_f64)
-      launch_tc_impl<true, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<true, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
     else if (routed)
-      launch_tc_impl<true, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<true, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
     else
-      launch_tc_impl<true, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<true, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
   } else {
     if (out_f64)
-      launch_tc_impl<false, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<false, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
     else if (routed)
-      launch_tc_impl<false, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<false, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
     else
-      launch_tc_impl<false, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt);
+      launch_tc_impl<false, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
   }
 }
 

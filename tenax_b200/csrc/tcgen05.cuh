@@ -34,6 +34,25 @@ static __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t par
   }
 }
 
+// One lane of a converged warp, always the same one.  The roles' loops run in
+// all lanes of their warp and only the instruction itself is predicated on the
+// elected lane (the `on` arguments below), so that addresses and descriptors are
+// formed in warp-uniform code.
+static __device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p;
+}
+
+// wait_or_abort by a whole converged warp, with one answer for all its lanes
+static __device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                          int32_t* err_flag) {
+  return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, err_flag)) != 0;
+}
+
+// a value every lane of the warp holds, marked as such
+static __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 static __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);  // start address
@@ -59,6 +78,56 @@ static __device__ __forceinline__ void mma_issue(uint32_t d_tmem, uint64_t a, ui
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
   }
+}
+
+// the same from the low words of SWIZZLE_128B descriptors (sw128_lo), whose high word is fixed
+constexpr uint32_t kSw128Hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+static __device__ __forceinline__ uint32_t sw128_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+template <bool TF32>
+static __device__ __forceinline__ void mma_issue_lo(uint32_t d_tmem, uint32_t a, uint32_t b, uint32_t idesc,
+                                                    uint32_t acc) {
+  if constexpr (TF32) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 da, db;\nsetp.ne.b32 p, %4, 0;\n"
+        "mov.b64 da, {%1, %5};\nmov.b64 db, {%2, %5};\n"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a), "r"(b), "r"(idesc), "r"(acc), "n"(kSw128Hi));
+  } else {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 da, db;\nsetp.ne.b32 p, %4, 0;\n"
+        "mov.b64 da, {%1, %5};\nmov.b64 db, {%2, %5};\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a), "r"(b), "r"(idesc), "r"(acc), "n"(kSw128Hi));
+  }
+}
+// one slab's n K steps of A x B, 32 bytes each; acc0: whether the first one accumulates
+template <bool TF32>
+static __device__ __forceinline__ void mma_slab(uint32_t d_tmem, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc0,
+                                                int n) {
+  mma_issue_lo<TF32>(d_tmem, a, b, idesc, acc0);
+  if (n == 4) {
+    mma_issue_lo<TF32>(d_tmem, a + 2, b + 2, idesc, 1u);
+    mma_issue_lo<TF32>(d_tmem, a + 4, b + 4, idesc, 1u);
+    mma_issue_lo<TF32>(d_tmem, a + 6, b + 6, idesc, 1u);
+  } else {
+    for (int k = 1; k < n; ++k) mma_issue_lo<TF32>(d_tmem, a + 2 * k, b + 2 * k, idesc, 1u);
+  }
+}
+
+// expect `bytes` on the barrier at shared address bar, and one bulk copy counted on it
+static __device__ __forceinline__ void mbar_expect_tx_on(uint32_t on, uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(bar), "r"(bytes), "r"(on)
+      : "memory");
+}
+static __device__ __forceinline__ void bulk_g2s_on(uint32_t on, uint32_t dst, const void* src, uint32_t bytes,
+                                                   uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}\n" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar), "r"(on)
+      : "memory");
 }
 
 static __device__ __forceinline__ void mma_commit(uint64_t* bar) {
