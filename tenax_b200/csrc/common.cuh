@@ -263,6 +263,16 @@ static __device__ __forceinline__ void img_store_chunk(uint8_t* img, int64_t lo_
 // PTX wrappers (sm_100a)
 // ---------------------------------------------------------------------------
 
+// Programmatic dependent launch.  A kernel launched by launch_pdl may start
+// while its predecessor in the stream still runs; it reads only tables written
+// before the plan or batch was first used until pdl_wait(), which returns once
+// the predecessor has completed and its writes are visible.  pdl_trigger() lets
+// the successor start likewise.  Every kernel launched this way waits before its
+// first dependent access (the skip flag included), so completion stays in stream
+// order; what overlaps is the launch and the prologue.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * WM * WN, (BM * BN >= 4096) ? 3 : 4)
                         const uint64_t* __restrict__ a_ptrs, const uint64_t* __restrict__ b_ptrs,
                         const uint64_t* __restrict__ c_ptrs, const int32_t* __restrict__ skip_flag) {
   constexpr int THREADS = 32 * WM * WN;
-  if (skip_flag && *skip_flag) return;  // the whole cluster
+  pdl_trigger();
   constexpr int MI = BM / 8 / WM, NI = BN / 8 / WN;
   using OpA = Operand<BM, AK, AV, THREADS>;
   using OpB = Operand<BN, BKF, BV, THREADS>;
@@ -219,6 +219,8 @@ __global__ void __launch_bounds__(32 * WM * WN, (BM * BN >= 4096) ? 3 : 4)
   const ContractTile t = tiles[blockIdx.x / (split * parts)];
   for (int i = tid; i < t.nspan * 4 && i < kSmemSpans * 4; i += THREADS)
     reinterpret_cast<int4*>(sspan)[i] = __ldg(reinterpret_cast<const int4*>(spans + t.span0) + i);
+  pdl_wait();  // the tables are the plan's; operands, pointers and the skip flag are not
+  if (skip_flag && *skip_flag) return;  // the whole cluster
   __syncthreads();
   const int rows = min(BM, t.M - t.m0), cols = min(BN, t.N - t.n0);
   // this CTA's K tiles: an even share of the output tile's
@@ -381,20 +383,6 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
   auto kernel = contract_f64_kernel<BM, BN, WM, WN, AK, BKF, AV, BV>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(L.n_tiles) * L.split * L.parts);
-  cfg.blockDim = dim3(32 * WM * WN);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  if (L.split > 1) {
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = L.split;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-  }
   double* ws = nullptr;
   if (L.parts > 1) {
     // partial tiles of this call, from the stream-ordered pool: safe with any
@@ -402,8 +390,8 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
     e = cudaMallocAsync(&ws, sizeof(double) * BM * BN * static_cast<size_t>(L.n_tiles) * L.parts, st);
     if (e != cudaSuccess) return e;
   }
-  e = cudaLaunchKernelEx(&cfg, kernel, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws,
-                         L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
+  e = launch_pdl(kernel, static_cast<unsigned>(L.n_tiles) * L.split * L.parts, 32 * WM * WN, smem, st, L.split,
+                 L.n_tiles, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws, L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
   if (L.parts > 1) {
     if (e == cudaSuccess) {
       contract_parts_kernel<<<dim3(L.n_tiles, (BM * BN + 255) / 256), 256, 0, st>>>(ws, L.c, L.tiles, L.tab, L.parts,

@@ -190,7 +190,7 @@ static __device__ __forceinline__ void route_store(uint8_t* img, int64_t lo_off,
 // route windows in shared memory.
 template <bool TF32, typename OutT, bool ROUTED>
 __global__ void __launch_bounds__(THREADS, 1)
-    gemm_tc_kernel(const DevGroup* __restrict__ groups, const DevTile* __restrict__ tiles, int n_tiles,
+    gemm_tc_kernel(const DevGroup* __restrict__ groups, const DevTile* __restrict__ tiles, const int n_all,
                    const int64_t* __restrict__ rowoff, const uint64_t* __restrict__ out_tab, int32_t* err_flag,
                    const int32_t* __restrict__ skip, const DevRouteTabs rt, const int width_) {
   constexpr int NT = TF32 ? 2 : 4;          // operand tiles per stage
@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(THREADS, 1)
   // MMAs run up to three tiles ahead of its longer epilogue
   constexpr int NACC = ROUTED ? 4 : ::tnx::NACC;
   constexpr int TMEM_COLS = NACC * TBN;
-  if (skip && *skip) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -253,6 +252,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_wait();  // the tables are the plan's; operands, pointers and the skip flag are not
+  const int n_tiles = skip && *skip ? 0 : n_all;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -690,8 +691,8 @@ void launch_tc_impl(const DevGroup* groups, const DevTile* tiles, int n_tiles, c
     return;  // the thread's last CUDA error, checked by every caller
   int grid = device_sm_count();
   if (grid > n_tiles) grid = n_tiles;
-  gemm_tc_kernel<TF32, OutT, ROUTED>
-      <<<grid, THREADS, smem, st>>>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, rt, width);
+  launch_pdl(gemm_tc_kernel<TF32, OutT, ROUTED>, grid, THREADS, smem, st, 1, n_tiles, groups, tiles, n_tiles, rowoff,
+             out_tab, err_flag, skip, rt, width);
 }
 }  // namespace
 

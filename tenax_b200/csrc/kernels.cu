@@ -123,6 +123,8 @@ void launch_strided_copy(const double* src, double* dst, const DevCopySeg* segs,
 // ---------------------------------------------------------------------------
 __global__ void zero_ranges_kernel(const uint64_t* __restrict__ out_tab, const DevChunk* __restrict__ chunks,
                                    const int32_t* __restrict__ skip) {
+  pdl_trigger();
+  pdl_wait();
   if (skip && *skip) return;
   const DevChunk ch = chunks[blockIdx.x];  // seg = pointer slot, start = element offset
   double* out = reinterpret_cast<double*>(out_tab[ch.seg]) + ch.start;
@@ -132,7 +134,7 @@ __global__ void zero_ranges_kernel(const uint64_t* __restrict__ out_tab, const D
 void launch_zero_ranges(const uint64_t* out_tab, const DevChunk* chunks, int n_chunks, const int32_t* skip,
                         cudaStream_t st) {
   if (n_chunks <= 0) return;
-  zero_ranges_kernel<<<n_chunks, 256, 0, st>>>(out_tab, chunks, skip);
+  launch_pdl(zero_ranges_kernel, n_chunks, 256, 0, st, 1, n_chunks, out_tab, chunks, skip);
 }
 
 // ---------------------------------------------------------------------------
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(kMpoThreads) mpo_apply_kernel(
   // boundary and is padded to a multiple of kMpoVec with zero columns (the
   // planner's N padding), so a thread's 8 d of one term are two aligned
   // 16-byte loads and need no bounds mask
-  if (skip && *skip) return;
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char mpo_smem[];
   const int2 ch = chunks[blockIdx.x];
   const DevMpoPair pr = pairs[ch.x];
@@ -172,6 +174,8 @@ __global__ void __launch_bounds__(kMpoThreads) mpo_apply_kernel(
   for (int i = threadIdx.x; i < pr.n_terms; i += blockDim.x) st[i] = terms[pr.term0 + i];
   for (int i = threadIdx.x; i < pr.n_in_slots; i += blockDim.x) si[i] = islots[pr.in0 + i];
   for (int i = threadIdx.x; i < pr.n_out_slots; i += blockDim.x) so[i] = oslots[pr.out0 + i];
+  pdl_wait();  // the tables are the batch's; X1 and the skip flag are not
+  if (skip && *skip) return;
   __syncthreads();
   const int nchunk = (pr.md + kMpoVec - 1) / kMpoVec;
   const int p = ch.y + threadIdx.x;
@@ -233,6 +237,8 @@ __global__ void __launch_bounds__(kMpoThreads)
                    const DevMpoSlot* __restrict__ oslots, const DevMpoTerm* __restrict__ terms,
                    const int2* __restrict__ chunks, const int32_t* __restrict__ skip) {
   constexpr int kLoads = 8;
+  pdl_trigger();
+  pdl_wait();
   if (skip && *skip) return;
   const int2 ch = chunks[blockIdx.x];
   const DevMpoPair pr = pairs[ch.x];
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(kMpoThreads)
 void launch_mpo_sum(const DevMpoPair* pairs, const DevMpoSlot* islots, const DevMpoSlot* oslots,
                     const DevMpoTerm* terms, const int2* chunks, int n_chunks, const int32_t* skip, cudaStream_t st) {
   if (n_chunks <= 0) return;
-  mpo_sum_kernel<<<n_chunks, kMpoThreads, 0, st>>>(pairs, islots, oslots, terms, chunks, skip);
+  launch_pdl(mpo_sum_kernel, n_chunks, kMpoThreads, 0, st, 1, n_chunks, pairs, islots, oslots, terms, chunks, skip);
 }
 
 // Copies of a block-sparse operand with padded rows (the FP64 H_eff reads its
@@ -315,9 +321,11 @@ __global__ void __launch_bounds__(kPackRows) pack_rows_kernel(const uint64_t* __
                                                         const int4* __restrict__ chunks,
                                                         const int32_t* __restrict__ skip) {
   constexpr int kChunks = 4;  // K chunks of 8 per thread, all loads issued before the stores
-  if (skip && *skip) return;
+  pdl_trigger();
   const int4 ch = chunks[blockIdx.x];  // (segment, first row, first K chunk, -)
   const DevRowPackSeg s = segs[ch.x];
+  pdl_wait();
+  if (skip && *skip) return;
   const int r = ch.y + static_cast<int>(threadIdx.x);
   // every thread reaches the shared-memory exchange below: a row past the
   // segment loads zeros and is not stored
@@ -386,9 +394,9 @@ void launch_pack_rows(const uint64_t* src_tab, const DevRowPackSeg* segs, const 
                       const int32_t* skip, cudaStream_t st) {
   if (n_chunks <= 0) return;
   if (mode == IMG_BF16)
-    pack_rows_kernel<IMG_BF16><<<n_chunks, kPackRows, 0, st>>>(src_tab, segs, chunks, skip);
+    launch_pdl(pack_rows_kernel<IMG_BF16>, n_chunks, kPackRows, 0, st, 1, n_chunks, src_tab, segs, chunks, skip);
   else
-    pack_rows_kernel<IMG_TF32><<<n_chunks, kPackRows, 0, st>>>(src_tab, segs, chunks, skip);
+    launch_pdl(pack_rows_kernel<IMG_TF32>, n_chunks, kPackRows, 0, st, 1, n_chunks, src_tab, segs, chunks, skip);
 }
 
 void launch_mpo_apply(int mode, const DevMpoPair* pairs, const DevMpoSlot* islots,
@@ -399,7 +407,7 @@ void launch_mpo_apply(int mode, const DevMpoPair* pairs, const DevMpoSlot* islot
   auto go = [&](auto kernel) {
     // a failure here is the thread's last CUDA error, checked by every caller
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return;
-    kernel<<<n_chunks, kMpoThreads, smem, st>>>(pairs, islots, oslots, terms, chunks, skip);
+    launch_pdl(kernel, n_chunks, kMpoThreads, smem, st, 1, n_chunks, pairs, islots, oslots, terms, chunks, skip);
   };
   if (mode == IMG_BF16)
     go(mpo_apply_kernel<IMG_BF16>);
@@ -576,6 +584,8 @@ __device__ __forceinline__ void cluster_leave() {  // no CTA ends while a peer r
 __global__ void __launch_bounds__(kStepThreads)
     lanczos_cluster_kernel(double* w, const double* v, const double* vp, double* vnext, int64_t n, double* alpha,
                            double* beta_next, const double* beta_prev, double tol, double tol_rel, int32_t* done) {
+  pdl_trigger();
+  pdl_wait();
   if (*done) return;  // set by an earlier launch only, or by this one after every CTA has passed here
   __shared__ double slots[2];
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kStepThreads;
@@ -628,6 +638,8 @@ __global__ void __launch_bounds__(kStepThreads)
 __global__ void __launch_bounds__(kStepThreads)
     dot_cluster_kernel(const double* __restrict__ x, const double* __restrict__ y, int64_t n, int kind,
                        double* __restrict__ result, const int32_t* __restrict__ skip) {
+  pdl_trigger();
+  pdl_wait();
   if (skip && *skip) return;
   __shared__ double slot;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kStepThreads;
@@ -650,27 +662,10 @@ static int step_ctas(int64_t n) {
   return c;
 }
 
-template <typename K, typename... Args>
-static void launch_cluster(K kernel, int ctas, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kStepThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ctas;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  // a failure is the thread's last CUDA error, checked by every caller
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 void launch_dot(const double* x, const double* y, int64_t n, int kind, double* result, double* partials,
                 const int32_t* skip, cudaStream_t st) {
   if (n <= kStepMax) {
-    launch_cluster(dot_cluster_kernel, step_ctas(n), st, x, y, n, kind, result, skip);
+    launch_pdl(dot_cluster_kernel, step_ctas(n), kStepThreads, 0, st, step_ctas(n), 0, x, y, n, kind, result, skip);
     return;
   }
   partial_dot_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(x, y, n, kind, partials, skip);
@@ -746,8 +741,8 @@ void launch_lanczos_step(double* w, const double* v, const double* vp, double* v
                          double* beta_next, const double* beta_prev, double tol, double tol_rel, int32_t* done,
                          double* partials, cudaStream_t st) {
   if (n <= kStepMax) {
-    launch_cluster(lanczos_cluster_kernel, step_ctas(n), st, w, v, vp, vnext, n, alpha, beta_next, beta_prev, tol,
-                   tol_rel, done);
+    launch_pdl(lanczos_cluster_kernel, step_ctas(n), kStepThreads, 0, st, step_ctas(n), 0, w, v, vp, vnext, n, alpha,
+               beta_next, beta_prev, tol, tol_rel, done);
     return;
   }
   partial_dot_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(v, w, n, 0, partials, done);

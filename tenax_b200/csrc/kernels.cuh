@@ -8,6 +8,41 @@
 
 namespace tnx {
 
+// Launch of a kernel that calls pdl_wait() (see common.cuh), in a cluster of
+// `cluster` CTAs where that is above 1.  A failure is also the thread's last
+// CUDA error.  What the overlap saves is a launch gap of 1 to 2 us a kernel:
+// H_eff in TF32 at chi = 512, four launches, 58.8 -> 52.4 us; the FP64 chain at
+// chi = 64, two, 12.3 -> 9.4 us.  Launches of more than kPdlWork units run for
+// hundreds of us and go without (a 16-problem batch: within 2 % either way).
+// The tcgen05 GEMM does not trigger its successor early: CTAs of the MPO kernel
+// resident beside it keep the SM's carve-out, so that kernel would run with its
+// L1 at a few KB (TF32 chi = 512: 85 us).
+constexpr int64_t kPdlWork = 600;
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
+                              int64_t work, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (work <= kPdlWork) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = static_cast<unsigned>(cluster);
+    at[n].val.clusterDim.y = 1;
+    at[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 void launch_pack(const uint64_t* src_tab, const DevPackSeg* segs, const DevChunk* chunks, int n_chunks, int mode,
                  const int32_t* skip, cudaStream_t st);
 // chunks: (segment, first row, first 8-wide K chunk, -): pack_rows_per_cta() rows x pack_rows_chunks_per_thread()
