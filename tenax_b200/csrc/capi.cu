@@ -241,16 +241,13 @@ std::vector<DevTile> sorted_tiles(std::vector<std::pair<int64_t, DevTile>>& tl) 
 }
 
 void gemm_launch(int mode, const DevMem& groups, const DevMem& tiles, int n_tiles, int width, const DevMem& rowoff,
-                 const PtrTab& out_tab, bool out_f64, int32_t* err, const int32_t* skip, cudaStream_t st,
-                 DevMem& out_tab_dev) {
-  // out_tab travels through a small device array (kernels index it per group)
-  CUDA_OK(cudaMemcpyAsync(out_tab_dev.p, out_tab.p, sizeof(PtrTab), cudaMemcpyHostToDevice, st));
+                 const DevMem& out_tab, int32_t* err, cudaStream_t st) {
   if (mode == IMG_F64)
-    launch_gemm_f64(groups.as<DevGroup>(), tiles.as<DevTile>(), n_tiles, rowoff.as<int64_t>(),
-                    out_tab_dev.as<uint64_t>(), skip, st);
+    launch_gemm_f64(groups.as<DevGroup>(), tiles.as<DevTile>(), n_tiles, rowoff.as<int64_t>(), out_tab.as<uint64_t>(),
+                    nullptr, st);
   else
     launch_gemm_tc(mode, groups.as<DevGroup>(), tiles.as<DevTile>(), n_tiles, rowoff.as<int64_t>(),
-                   out_tab_dev.as<uint64_t>(), out_f64, err, skip, st, width);
+                   out_tab.as<uint64_t>(), false, err, nullptr, st, width);
 }
 }  // namespace
 
@@ -262,8 +259,8 @@ struct StepDev {
   PairGeom G;
   DevMem a_img, b_img, c_res;  // images and result matrices
   int64_t a_lo = 0, b_lo = 0;
-  DevMem packA, chunksA, packB, chunksB, groups, tiles, rowoff, scat, chunksS, out_tab;
-  int nA = 0, nB = 0, nT = 0, nS = 0, width = 128;
+  DevMem pack, chunksP, groups, tiles, rowoff, scat, chunksS, out_tab;
+  int nP = 0, nT = 0, nS = 0, width = 128;
   bool res_f32 = false;
   // FP64 in one launch (contract_f64.cu): tables of the step in one buffer
   bool direct = false, swapped = false;
@@ -291,7 +288,7 @@ struct tnx_plan {
   std::vector<std::unique_ptr<StepDev>> dev;
   std::vector<std::unique_ptr<DevMem>> inter;  // intermediate block buffers (fp64)
   DevMem scalar_one;                           // operand for single-tensor plans
-  DevMem err_flag, src_tab;
+  DevMem err_flag;
 };
 
 static void finalize_plan_out(tnx_plan* p) {
@@ -900,6 +897,9 @@ static void plan_build_device(tnx_plan* p, int precision) {
     const int split = mode == IMG_BF16 ? 2 : 1;
     d->a_img.alloc(std::max<int64_t>(1, d->G.a_tiles) * ig.tile_bytes * split);
     d->b_img.alloc(std::max<int64_t>(1, d->G.b_tiles) * ig.tile_bytes * split);
+    // cleared once: every pack writes the same elements, so the padding stays zero
+    CUDA_OK(cudaMemsetAsync(d->a_img.p, 0, d->a_img.n, nullptr));
+    CUDA_OK(cudaMemsetAsync(d->b_img.p, 0, d->b_img.n, nullptr));
     d->a_lo = d->G.a_tiles * ig.tile_bytes;
     d->b_lo = d->G.b_tiles * ig.tile_bytes;
     d->res_f32 = mode != IMG_F64;
@@ -911,16 +911,14 @@ static void plan_build_device(tnx_plan* p, int precision) {
       roff += g.M * g.N;
     }
     d->c_res.alloc(std::max<int64_t>(1, roff) * (d->res_f32 ? 4 : 8));
-    std::vector<DevPackSeg> pa, pb;
-    std::vector<DevChunk> ca, cb;
-    build_pack(P.packA, d->G, true, reinterpret_cast<uint64_t>(d->a_img.p), d->a_lo, ig.tile_bytes, 0, pa, ca);
-    build_pack(P.packB, d->G, false, reinterpret_cast<uint64_t>(d->b_img.p), d->b_lo, ig.tile_bytes, 1, pb, cb);
-    upload(d->packA, pa);
-    upload(d->chunksA, ca);
-    upload(d->packB, pb);
-    upload(d->chunksB, cb);
-    d->nA = static_cast<int>(ca.size());
-    d->nB = static_cast<int>(cb.size());
+    // both operands in one list: build_pack numbers its chunks by the segments so far
+    std::vector<DevPackSeg> pk;
+    std::vector<DevChunk> ck;
+    build_pack(P.packA, d->G, true, reinterpret_cast<uint64_t>(d->a_img.p), d->a_lo, ig.tile_bytes, 0, pk, ck);
+    build_pack(P.packB, d->G, false, reinterpret_cast<uint64_t>(d->b_img.p), d->b_lo, ig.tile_bytes, 1, pk, ck);
+    upload(d->pack, pk);
+    upload(d->chunksP, ck);
+    d->nP = static_cast<int>(ck.size());
     std::vector<DevGroup> gr;
     std::vector<int64_t> ro;
     for (size_t g = 0; g < P.groups.size(); ++g) {
@@ -968,7 +966,8 @@ static void plan_build_device(tnx_plan* p, int precision) {
     upload(d->scat, ss);
     upload(d->chunksS, cs);
     d->nS = static_cast<int>(cs.size());
-    d->out_tab.alloc(sizeof(PtrTab));
+    // the GEMM's output is the plan's own result buffer
+    upload(d->out_tab, std::vector<uint64_t>{reinterpret_cast<uint64_t>(d->c_res.p)});
     p->dev.push_back(std::move(d));
   }
   CUDA_OK(cudaDeviceSynchronize());
@@ -983,11 +982,8 @@ int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, i
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (plan->empty_result) return TNX_OK;
     if (plan->dev_prec != precision) plan_build_device(plan, precision);
-    const ImgGeom ig = img_geom(img_mode_of(precision));
-    const int split = precision == TNX_PREC_BF16X3 ? 2 : 1;
     for (size_t s = 0; s < plan->steps.size(); ++s) {
       StepDev& d = *plan->dev[s];
-      const PairPlan& P = plan->steps[s];
       const double* a_ptr = plan->a_src[s] >= 0 ? inputs[plan->a_src[s]] : plan->inter[s - 1]->as<double>();
       const double* b_ptr = plan->has_scalar ? plan->scalar_one.as<double>() : inputs[plan->b_src[s]];
       double* o_ptr = (s + 1 == plan->steps.size()) ? out : plan->inter[s]->as<double>();
@@ -1004,25 +1000,10 @@ int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, i
         CUDA_OK(cudaGetLastError());
         continue;
       }
-      PtrTab src{};
-      src.p[0] = reinterpret_cast<uint64_t>(a_ptr);
-      src.p[1] = reinterpret_cast<uint64_t>(b_ptr);
-      // the pack kernels read operand pointers from a device table
-      DevMem& srcdev = plan->src_tab;
-      if (!srcdev.p) srcdev.alloc(sizeof(PtrTab));
-      CUDA_OK(cudaMemcpyAsync(srcdev.p, &src, 2 * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-      CUDA_OK(cudaMemsetAsync(d.a_img.p, 0, std::max<int64_t>(1, d.G.a_tiles) * ig.tile_bytes * split, st));
-      CUDA_OK(cudaMemsetAsync(d.b_img.p, 0, std::max<int64_t>(1, d.G.b_tiles) * ig.tile_bytes * split, st));
-      launch_pack(srcdev.as<uint64_t>(), d.packA.as<DevPackSeg>(), d.chunksA.as<DevChunk>(), d.nA, d.mode, nullptr,
-                  st);
-      launch_pack(srcdev.as<uint64_t>(), d.packB.as<DevPackSeg>(), d.chunksB.as<DevChunk>(), d.nB, d.mode, nullptr,
-                  st);
-      PtrTab ot{};
-      ot.p[0] = reinterpret_cast<uint64_t>(d.c_res.p);
-      gemm_launch(d.mode, d.groups, d.tiles, d.nT, d.width, d.rowoff, ot, false, plan->err_flag.as<int32_t>(), nullptr, st,
-                  d.out_tab);
-      if (P.out.total > 0)
-        CUDA_OK(cudaMemsetAsync(o_ptr, 0, P.out.total * sizeof(double), st));
+      // three launches: the images' padding was cleared with the plan, and the
+      // scatter writes every element of every output block
+      launch_pack_two(a_ptr, b_ptr, d.pack.as<DevPackSeg>(), d.chunksP.as<DevChunk>(), d.nP, d.mode, st);
+      gemm_launch(d.mode, d.groups, d.tiles, d.nT, d.width, d.rowoff, d.out_tab, plan->err_flag.as<int32_t>(), st);
       launch_scatter(d.c_res.p, d.res_f32, o_ptr, d.scat.as<DevScatSeg>(), d.chunksS.as<DevChunk>(), d.nS, st);
       CUDA_OK(cudaGetLastError());
     }
@@ -1039,6 +1020,7 @@ struct tnx_fuse_plan {
   FusePlan F;
   DevMem segs, chunks;
   int n_chunks = 0;
+  int64_t covered = 0;  // output elements the copies write (each once); the rest is cleared first
   bool on_device = false;
 };
 
@@ -1092,6 +1074,7 @@ int tnx_fuse_execute(tnx_fuse_plan* p, const double* in, double* out, void* stre
         }
         const int id = static_cast<int>(segs.size());
         segs.push_back(d);
+        p->covered += c.count;
         for (int64_t s = 0; s < c.count; s += 2048) chunks.push_back({id, 0, s, std::min<int64_t>(2048, c.count - s)});
       }
       upload(p->segs, segs);
@@ -1100,7 +1083,7 @@ int tnx_fuse_execute(tnx_fuse_plan* p, const double* in, double* out, void* stre
       CUDA_OK(cudaDeviceSynchronize());
       p->on_device = true;
     }
-    if (p->F.out.total > 0) CUDA_OK(cudaMemsetAsync(out, 0, p->F.out.total * sizeof(double), st));
+    if (p->covered < p->F.out.total) CUDA_OK(cudaMemsetAsync(out, 0, p->F.out.total * sizeof(double), st));
     launch_strided_copy(in, out, p->segs.as<DevCopySeg>(), p->chunks.as<DevChunk>(), p->n_chunks, st);
     CUDA_OK(cudaGetLastError());
     return TNX_OK;

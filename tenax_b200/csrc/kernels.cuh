@@ -45,6 +45,9 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
 
 void launch_pack(const uint64_t* src_tab, const DevPackSeg* segs, const DevChunk* chunks, int n_chunks, int mode,
                  const int32_t* skip, cudaStream_t st);
+// the same for two operands, slots 0 and 1, given as arguments
+void launch_pack_two(const double* p0, const double* p1, const DevPackSeg* segs, const DevChunk* chunks, int n_chunks,
+                     int mode, cudaStream_t st);
 // chunks: (segment, first row, first 8-wide K chunk, -): pack_rows_per_cta() rows x pack_rows_chunks_per_thread()
 // K chunks each; K blocks of the image start at multiples of 8
 void launch_pack_rows(const uint64_t* src_tab, const DevRowPackSeg* segs, const int4* chunks, int n_chunks, int mode,

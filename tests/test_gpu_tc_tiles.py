@@ -30,3 +30,17 @@ def test_few_tiles_equal_many(precision, eps, m, n, k):
     assert torch.equal(few, big[:m])
     ref, mag = a[:m] @ b.T, a[:m].abs() @ b.abs().T
     assert bool(((few - ref).abs() <= (eps + (k + 4) * 2.0 ** -24) * mag).all())
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "tf32"])
+def test_plan_buffers_hold_nothing_of_the_last_call(precision):
+    """A plan's operand images are cleared once and refilled by every call: a
+    call after one with NaN and other values equals a fresh plan's."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(37, 5, 9, generator=g, dtype=torch.float64, device="cuda")
+    b = torch.randn(9, 21, 5, generator=g, dtype=torch.float64, device="cuda")
+    dense._PLANS.clear()
+    fresh = dense.einsum("mak,kna->nm", a, b, precision=precision)
+    dense._PLANS.clear()
+    dense.einsum("mak,kna->nm", torch.full_like(a, float("nan")), b * 1e30, precision=precision)
+    assert torch.equal(dense.einsum("mak,kna->nm", a, b, precision=precision), fresh)
