@@ -211,12 +211,25 @@ void build_tiles(const PairPlan& P, const PairGeom& G, int group_base, std::vect
 // until they cover the SMs.  Every element keeps its own accumulation order, so
 // the results are the same bits.  H_eff stage 4 in TF32 at chi = 512 (about 70
 // tiles of up to 92 K slabs): 34.4 us in 128 columns, 31.3 in 32.
-// Returns the tiles' width.
-int narrow_tiles(std::vector<std::pair<int64_t, DevTile>>& tl, const std::vector<DevGroup>& groups) {
+// A launch of many tiles is bound by what the L2 hands the SMs (16-problem batch,
+// stage 4: 4.7 GB of operands at 12 TB/s): 256 columns read each A panel once for
+// twice the columns (3.6 GB; 389 -> 371 us).  Returns the tiles' width.
+constexpr size_t kWideTiles = 4;
+int fit_tiles(std::vector<std::pair<int64_t, DevTile>>& tl, const std::vector<DevGroup>& groups) {
   const size_t sms = static_cast<size_t>(device_sm_count());
-  if (tl.size() >= sms) return 128;
-  int last = 128;
   std::vector<std::pair<int64_t, DevTile>> out;
+  if (tl.size() >= sms) {
+    // many tiles: 256 columns where they still leave four tiles an SM
+    for (const auto& t : tl)
+      if (t.second.nt % 2 == 0) {
+        out.push_back(t);
+        out.back().second.nt /= 2;
+      }
+    if (out.size() == tl.size() || out.size() < kWideTiles * sms) return 128;
+    tl.swap(out);
+    return 256;
+  }
+  int last = 128;
   for (int width : {64, 32}) {
     out.clear();
     last = width;
@@ -941,7 +954,7 @@ static void plan_build_device(tnx_plan* p, int precision) {
     upload(d->rowoff, ro);
     std::vector<std::pair<int64_t, DevTile>> tl;
     build_tiles(P, d->G, 0, tl);
-    if (mode != IMG_F64) d->width = narrow_tiles(tl, gr);
+    if (mode != IMG_F64) d->width = fit_tiles(tl, gr);
     auto tiles = sorted_tiles(tl);
     upload(d->tiles, tiles);
     d->nT = static_cast<int>(tiles.size());
@@ -2649,7 +2662,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     }
     upload(b->g1, G1);
     upload(b->ro1, R1);
-    if (!rt) b->width1 = narrow_tiles(T1, G1);  // the routed epilogue's windows are per 128-column tile
+    if (!rt) b->width1 = fit_tiles(T1, G1);  // the routed epilogue's windows are per 128-column tile
     auto t1 = sorted_tiles(T1);
     upload(b->t1, t1);
     if (rt) {
@@ -2688,7 +2701,7 @@ int tnx_heff_batch_create(tnx_heff* const* hs, int32_t n, int32_t precision, tnx
     b->n_t1 = static_cast<int>(t1.size());
     upload(b->g4, G4);
     upload(b->ro4, R4);
-    b->width4 = narrow_tiles(T4, G4);
+    b->width4 = fit_tiles(T4, G4);
     auto t4 = sorted_tiles(T4);
     upload(b->t4, t4);
     b->n_t4 = static_cast<int>(t4.size());

@@ -1,7 +1,8 @@
 // Persistent grouped GEMM on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
 // C_g[row, col] = sum_k A_g[row, k] * B_g[col, k] over every sector group g,
-// one work-list entry per 128x128 output tile.  Operands are pre-swizzled
+// one work-list entry per output tile of 128 rows and 128 columns (256 in launches
+// of many tiles, 64 or 32 in launches of few: fit_tiles picks).  Operands are pre-swizzled
 // SWIZZLE_128B K-major image tiles (16 KB each) moved by 1-D bulk async copies
 // (cp.async.bulk, no tensor map; every CTA fetches its own tiles) into a
 // STAGES-deep ring.
@@ -44,13 +45,14 @@ static_assert(NACC == 2 || NACC == 4, "TMEM accumulators: 2 or 4 (512 columns)")
 // the group has (whole 8-row swizzle atoms of A, the MMA's N of B): rows of the
 // stage past them hold older bytes, which reach only result rows and columns
 // that are not stored.  A launch of fewer tiles than SMs leaves SMs idle; the
-// host then cuts tiles to 64 or 32 columns (narrow_tiles).
+// host then cuts tiles to 64 or 32 columns (fit_tiles).
+template <int TN>
 struct TileCols {
   int col0, ncols, width;  // first column, valid columns, columns of the tile
   uint32_t a_bytes, b_bytes;
   __device__ __forceinline__ TileCols(const DevTile& tl, const DevGroup& g) {
-    width = tl.sub ? tl.sub >> 16 : 128;
-    col0 = tl.nt * 128 + (tl.sub & 0xffff);
+    width = tl.sub ? tl.sub >> 16 : TN;
+    col0 = tl.nt * TN + (tl.sub & 0xffff);
     ncols = min(g.N - col0, width);
     a_bytes = static_cast<uint32_t>((min(128, g.M - tl.mt * 128) + 7) & ~7) * 128u;
     b_bytes = static_cast<uint32_t>((ncols + 15) & ~15) * 128u;
@@ -188,7 +190,7 @@ static __device__ __forceinline__ void route_store(uint8_t* img, int64_t lo_off,
 // row class (DevRouteTabs); it runs a 2-stage operand ring (stage 1 is
 // short-K) so that each epilogue warp also holds a transpose buffer and two
 // route windows in shared memory.
-template <bool TF32, typename OutT, bool ROUTED>
+template <bool TF32, typename OutT, bool ROUTED, int TN>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_tc_kernel(const DevGroup* __restrict__ groups, const DevTile* __restrict__ tiles, const int n_all,
                    const int64_t* __restrict__ rowoff, const uint64_t* __restrict__ out_tab, int32_t* err_flag,
@@ -202,12 +204,14 @@ __global__ void __launch_bounds__(THREADS, 1)
   // TMEM accumulators: the routed instance runs 4 (all 512 columns), so the
   // MMAs run up to three tiles ahead of its longer epilogue
   constexpr int NACC = ROUTED ? 4 : ::tnx::NACC;
-  constexpr int TMEM_COLS = NACC * TBN;
+  constexpr int TMEM_COLS = NACC * TN;
+  constexpr int RING = STAGES * NT * TILE_BYTES;
+  static_assert(TN == TBN || (TN == 2 * TBN && !ROUTED && TMEM_COLS <= 512), "128 or 256 columns");
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * NT * TILE_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + RING);
   uint64_t* empty = full + MAXS;
   uint64_t* tfull = empty + MAXS;
   uint64_t* tempty = tfull + NACC;
@@ -221,13 +225,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                 "barriers, TMEM address and abort flag fit the 256 bytes before the epilogue staging");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   // epilogue staging: one 32 x 33 fp32 buffer per epilogue warp, after 256 B of barriers
-  float* epi_stage = reinterpret_cast<float*>(smem + STAGES * NT * TILE_BYTES + 256);
+  float* epi_stage = reinterpret_cast<float*>(smem + RING + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int width = ROUTED ? TBN : width_;  // columns of this launch's tiles
+  const int width = ROUTED || TN != TBN ? TN : width_;  // columns of this launch's tiles
   const uint32_t b_tile = static_cast<uint32_t>(width) * 128u;               // bytes of one B plane of a stage
   const uint32_t stage_bytes = static_cast<uint32_t>(NT / 2) * (TILE_BYTES + b_tile);
-  const int nst = width == TBN ? STAGES : min(MAXS, STAGES * NT * TILE_BYTES / static_cast<int>(stage_bytes));
+  const int nst = width == TBN ? STAGES : min(MAXS, RING / static_cast<int>(stage_bytes));
   if (threadIdx.x == 0) {
     for (int s = 0; s < nst; ++s) {
       mbar_init(&full[s], 1);
@@ -267,13 +271,16 @@ __global__ void __launch_bounds__(THREADS, 1)
       bool ok = true;
       for (TileIter it(tiles, groups, n_tiles, blockIdx.x); it.t < n_tiles && ok; it.advance()) {
         it.prefetch();
-        const TileCols tc(it.tl, it.g);
+        const TileCols<TN> tc(it.tl, it.g);
         const uint8_t* ga =
             reinterpret_cast<const uint8_t*>(it.g.a_addr) + static_cast<int64_t>(it.tl.mt) * it.g.nKt * TILE_BYTES;
         const uint8_t* gb = reinterpret_cast<const uint8_t*>(it.g.b_addr) +
-                            static_cast<int64_t>(it.tl.nt) * it.g.nKt * TILE_BYTES + (tc.col0 - it.tl.nt * TBN) * 128;
+                            static_cast<int64_t>(it.tl.nt) * (TN / TBN) * it.g.nKt * TILE_BYTES +
+                            (tc.col0 - it.tl.nt * TN) * 128;
         const int64_t a_lo = it.g.a_lo, b_lo = it.g.b_lo;
+        const int64_t b_next = static_cast<int64_t>(it.g.nKt) * TILE_BYTES;  // the next 128 rows of B's image
         const uint32_t ab = warp_uniform(tc.a_bytes), bb = warp_uniform(tc.b_bytes);
+        const uint32_t b1 = min(bb, static_cast<uint32_t>(TILE_BYTES)), b2 = bb - b1;
         const int nKt = static_cast<int>(warp_uniform(it.g.nKt));
         for (int kt = 0; kt < nKt; ++kt) {
           if (!warp_wait_or_abort(&empty[s], ph ^ 1u, abort_flag, err_flag)) {
@@ -285,15 +292,21 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (TF32) {
             mbar_expect_tx_on(lead, fb, ab + bb);
             bulk_g2s_on(lead, st, ga + ko, ab, fb);
-            bulk_g2s_on(lead, st + TILE_BYTES, gb + ko, bb, fb);
+            bulk_g2s_on(lead, st + TILE_BYTES, gb + ko, b1, fb);
+            if (TN != TBN)
+              bulk_g2s_on(b2 ? lead : 0u, st + 2 * TILE_BYTES, gb + b_next + ko, b2, fb);
           } else {
             // stage layout [A hi][A lo][B hi][B lo]; hi planes first
             mbar_expect_tx_on(lead, fb, ab + bb);
             bulk_g2s_on(lead, st, ga + ko, ab, fb);
-            bulk_g2s_on(lead, st + 2 * TILE_BYTES, gb + ko, bb, fb);
+            bulk_g2s_on(lead, st + 2 * TILE_BYTES, gb + ko, b1, fb);
+            if (TN != TBN)
+              bulk_g2s_on(b2 ? lead : 0u, st + 3 * TILE_BYTES, gb + b_next + ko, b2, fb);
             mbar_expect_tx_on(lead, fb2, ab + bb);
             bulk_g2s_on(lead, st + TILE_BYTES, ga + a_lo + ko, ab, fb2);
-            bulk_g2s_on(lead, st + 2 * TILE_BYTES + b_tile, gb + b_lo + ko, bb, fb2);
+            bulk_g2s_on(lead, st + 2 * TILE_BYTES + b_tile, gb + b_lo + ko, b1, fb2);
+            if (TN != TBN)
+              bulk_g2s_on(b2 ? lead : 0u, st + 3 * TILE_BYTES + b_tile, gb + b_lo + b_next + ko, b2, fb2);
           }
           last_par[s] = static_cast<int>(ph);
           if (++s == nst) {
@@ -341,7 +354,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // MMA extent trimmed to the tile's valid columns (rounded to 16) and
         // the last slab's valid K steps: the operand images are zero beyond
         // both, so the skipped products are exact zeros
-        const uint32_t n_mma = warp_uniform((TileCols(it.tl, it.g).ncols + 15) / 16 * 16);
+        const uint32_t n_mma = warp_uniform((TileCols<TN>(it.tl, it.g).ncols + 15) / 16 * 16);
         const uint32_t idesc = idesc0 | ((n_mma >> 3) << 17);
         const int nKt = static_cast<int>(warp_uniform(it.g.nKt));
         const int ksub_last = static_cast<int>(warp_uniform(it.g.kk_last > 0 ? it.g.kk_last : KSUB));
@@ -350,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem0 + static_cast<uint32_t>(acc * TBN);
+        const uint32_t d_tmem = tmem0 + static_cast<uint32_t>(acc * TN);
         for (int kt = 0; kt < nKt; ++kt) {
           if (!warp_wait_or_abort(&full[s], ph, abort_flag, err_flag)) {
             ok = false;
@@ -419,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     const int r_in_tile = q * 32 + lane;
     const int e = warp - 2;  // epilogue warp 0..EPI_WARPS-1
-    constexpr int kColsPerWarp = TBN / (EPI_WARPS / 4);
+    constexpr int kColsPerWarp = TN / (EPI_WARPS / 4);
     const int c_begin = (e / 4) * kColsPerWarp;
     float* stg = epi_stage + e * 32 * kStagePitch;
     int acc = 0;
@@ -518,7 +531,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           __syncwarp();
           if (!wait_or_abort(&tfull[acc], aph, abort_flag, err_flag)) break;
           tc_fence_after();
-          const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * TBN);
+          const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * TN);
 #pragma unroll
           for (int j = 0; j < NCH; ++j) {
             const int c0 = 32 * (e / 4) + 32 * (EPI_WARPS / 4) * j;
@@ -598,7 +611,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (!wait_or_abort(&tfull[acc], aph, abort_flag, err_flag)) break;
       tc_fence_after();
       OutT* out = reinterpret_cast<OutT*>(out_tab[g.out_slot]);
-      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * TBN);
+      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * TN);
       // group scales are powers of two, so the multiply is exact in the
       // output's own precision (FP32 outputs only ever carry scale 1; a
       // per-element FP64 round trip there doubled the epilogue's cost)
@@ -607,7 +620,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       // fragments; otherwise each lane holds one row (32x32b) and 32x32
       // chunks are staged through shared memory so that every store
       // instruction writes 32 consecutive columns of one row.
-      const TileCols tc(tl, g);
+      const TileCols<TN> tc(tl, g);
       const int c_end = min(tc.width, (sizeof(OutT) == 4 && g.vec_ld > 0 ? g.vec_ld : g.N) - tc.col0);  // columns to store
 #pragma unroll 1
       for (int c0 = c_begin; c0 < c_begin + kColsPerWarp && c0 < c_end; c0 += 32) {
@@ -681,17 +694,17 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-template <bool TF32, typename OutT, bool ROUTED>
+template <bool TF32, typename OutT, bool ROUTED, int TN>
 void launch_tc_impl(const DevGroup* groups, const DevTile* tiles, int n_tiles, const int64_t* rowoff,
                     const uint64_t* out_tab, int32_t* err_flag, const int32_t* skip, cudaStream_t st,
                     const DevRouteTabs& rt, int width) {
   constexpr int smem = gemm_tc_smem<TF32, ROUTED>();
-  if (cudaFuncSetAttribute(gemm_tc_kernel<TF32, OutT, ROUTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+  if (cudaFuncSetAttribute(gemm_tc_kernel<TF32, OutT, ROUTED, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return;  // the thread's last CUDA error, checked by every caller
   int grid = device_sm_count();
   if (grid > n_tiles) grid = n_tiles;
-  launch_pdl(gemm_tc_kernel<TF32, OutT, ROUTED>, grid, THREADS, smem, st, 1, n_tiles, groups, tiles, n_tiles, rowoff,
+  launch_pdl(gemm_tc_kernel<TF32, OutT, ROUTED, TN>, grid, THREADS, smem, st, 1, n_tiles, groups, tiles, n_tiles, rowoff,
              out_tab, err_flag, skip, rt, width);
 }
 }  // namespace
@@ -701,20 +714,21 @@ void launch_gemm_tc(int mode, const DevGroup* groups, const DevTile* tiles, int 
                     int width, const DevRouteTabs& rt) {
   if (n_tiles <= 0) return;
   const bool routed = rt.win != nullptr;  // every group routed, FP32 results
+  auto go = [&](auto impl) { impl(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width); };
   if (mode == IMG_TF32) {
-    if (out_f64)
-      launch_tc_impl<true, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
-    else if (routed)
-      launch_tc_impl<true, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
+    if (routed)
+      go(launch_tc_impl<true, float, true, 128>);
+    else if (out_f64)
+      width == 256 ? go(launch_tc_impl<true, double, false, 256>) : go(launch_tc_impl<true, double, false, 128>);
     else
-      launch_tc_impl<true, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
+      width == 256 ? go(launch_tc_impl<true, float, false, 256>) : go(launch_tc_impl<true, float, false, 128>);
   } else {
-    if (out_f64)
-      launch_tc_impl<false, double, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
-    else if (routed)
-      launch_tc_impl<false, float, true>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
+    if (routed)
+      go(launch_tc_impl<false, float, true, 128>);
+    else if (out_f64)
+      width == 256 ? go(launch_tc_impl<false, double, false, 256>) : go(launch_tc_impl<false, double, false, 128>);
     else
-      launch_tc_impl<false, float, false>(groups, tiles, n_tiles, rowoff, out_tab, err_flag, skip, st, rt, width);
+      width == 256 ? go(launch_tc_impl<false, float, false, 256>) : go(launch_tc_impl<false, float, false, 128>);
   }
 }
 

@@ -44,3 +44,17 @@ def test_plan_buffers_hold_nothing_of_the_last_call(precision):
     dense._PLANS.clear()
     dense.einsum("mak,kna->nm", torch.full_like(a, float("nan")), b * 1e30, precision=precision)
     assert torch.equal(dense.einsum("mak,kna->nm", a, b, precision=precision), fresh)
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "tf32"])
+@pytest.mark.parametrize("n,k", [(129, 31), (200, 64), (256, 130), (300, 65), (513, 33)])
+def test_wide_tiles_equal_narrow(precision, n, k):
+    """Launches of many tiles take 256 columns at a time: the same bits as one
+    row tile alone (32 or 64 columns)."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    a = torch.randn(128 * 620, k, generator=g, dtype=torch.float64, device="cuda")
+    b = torch.randn(n, k, generator=g, dtype=torch.float64, device="cuda")
+    big = dense.einsum("mk,nk->mn", a, b, precision=precision)
+    for r0 in (0, 128 * 333):
+        rows = a[r0:r0 + 100].contiguous()
+        assert torch.equal(dense.einsum("mk,nk->mn", rows, b, precision=precision), big[r0:r0 + 100])
