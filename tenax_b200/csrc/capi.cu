@@ -2081,45 +2081,49 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
     for (size_t k = 0; k < H.R.keys.size(); ++k) r_by[{H.R.keys[k][0], H.R.keys[k][1]}].push_back(k);
     for (size_t p = 0; p < H.pairs.size(); ++p) {
       const MpoPair& mp = H.pairs[p];
-      size_t u = 0;  // terms are sorted by output slot
+      // terms of each output slot (they are sorted by it), their weights' R copies
+      std::vector<int32_t> tb(mp.n_out_slots + 1, 0), wi(mp.terms.size(), -1);
+      for (size_t v = 0; v < mp.terms.size(); ++v) {
+        ++tb[mp.terms[v].out_slot + 1];
+        const auto w = std::find(h->weights.begin(), h->weights.end(), mp.terms[v].w);
+        if (w != h->weights.end()) wi[v] = static_cast<int32_t>(w - h->weights.begin());
+      }
+      for (int32_t o = 0; o < mp.n_out_slots; ++o) tb[o + 1] += tb[o];
       for (size_t k = 0; k < mp.outs.size(); ++k) {
         const MpoOut& o = mp.outs[k];
         const Key& ok = H.mpo_out_keys[p][k];  // (q_s, q_t, q_f)
         const auto rb = r_by.find({mp.qd, ok[2]});
-        for (int32_t e = 0; e < o.ms * o.mt * o.mf; ++e) {
-          const int32_t slot = mp.out_slot0[k] + e, st = e / o.mf, f = e % o.mf;
-          size_t u1 = u;
-          while (u1 < mp.terms.size() && mp.terms[u1].out_slot == slot) ++u1;
-          if (u1 > u && rb != r_by.end())
-            for (size_t rk : rb->second) {
-              const auto& rd = H.R.dims[rk];
-              if (rd[0] != mp.md || rd[1] != o.mf || rd[2] == 0) continue;
-              const auto ti = th_idx.find(Key{mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
-              if (ti == th_idx.end()) continue;
-              auto& dst = prod[ti->second].at(st);
-              ContractSpan g{};
-              g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
-              g.ar_str = static_cast<int32_t>(even(mp.md));
-              g.ak_str = 1;
-              g.br_str = 1;
-              g.bk_str = stride32(rd[1] * even(rd[2]));
-              g.K = mp.md;
-              const int64_t r = r0 + h->r_off[rk] + f * even(rd[2]);
-              if (formed[i][p][slot]) {
-                g.a_off = static_cast<int64_t>(x3_base / 8) + x3[i][p][slot];
-                g.b_off = r;
-                dst.push_back(g);
-              } else {
-                for (size_t v = u; v < u1; ++v) {
-                  const auto w = std::find(h->weights.begin(), h->weights.end(), mp.terms[v].w);
-                  if (w == h->weights.end()) throw PlanError{TNX_ERR_RUNTIME, "internal: MPO weight without its R copy"};
-                  g.a_off = static_cast<int64_t>(x1_base / 8) + x1[i][p][mp.terms[v].in_slot];
-                  g.b_off = r + static_cast<int64_t>(w - h->weights.begin()) * h->r_total;
-                  dst.push_back(g);
-                }
-              }
+        if (rb == r_by.end()) continue;
+        for (size_t rk : rb->second) {
+          const auto& rd = H.R.dims[rk];
+          if (rd[0] != mp.md || rd[1] != o.mf || rd[2] == 0) continue;
+          const auto ti = th_idx.find(Key{mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
+          if (ti == th_idx.end()) continue;
+          ContractSpan g{};
+          g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
+          g.ar_str = static_cast<int32_t>(even(mp.md));
+          g.ak_str = 1;
+          g.br_str = 1;
+          g.bk_str = stride32(rd[1] * even(rd[2]));
+          g.K = mp.md;
+          for (int32_t e = 0; e < o.ms * o.mt * o.mf; ++e) {
+            const int32_t slot = mp.out_slot0[k] + e, st = e / o.mf, f = e % o.mf;
+            if (tb[slot] == tb[slot + 1]) continue;
+            auto& dst = prod[ti->second].at(st);
+            const int64_t r = r0 + h->r_off[rk] + f * even(rd[2]);
+            if (formed[i][p][slot]) {
+              g.a_off = static_cast<int64_t>(x3_base / 8) + x3[i][p][slot];
+              g.b_off = r;
+              dst.push_back(g);
+              continue;
             }
-          u = u1;
+            for (int32_t v = tb[slot]; v < tb[slot + 1]; ++v) {
+              if (wi[v] < 0) throw PlanError{TNX_ERR_RUNTIME, "internal: MPO weight without its R copy"};
+              g.a_off = static_cast<int64_t>(x1_base / 8) + x1[i][p][mp.terms[v].in_slot];
+              g.b_off = r + wi[v] * h->r_total;
+              dst.push_back(g);
+            }
+          }
         }
       }
     }

@@ -220,7 +220,7 @@ struct DevLPanelSeg {
 
 // One aligned chunk of kMpoVec consecutive K of one image row (k a multiple
 // of kMpoVec): a single 16-byte swizzle unit of a BF16 row (hi and lo
-// images), two for TF32, four double pairs for FP64.
+// images), two for TF32.
 constexpr int kMpoVec = kMpoKAlignDev;
 
 template <int MODE, typename AccT>
@@ -250,12 +250,6 @@ static __device__ __forceinline__ void img_store_chunk(uint8_t* img, int64_t lo_
       *reinterpret_cast<uint4*>(img + img_byte_offset(MODE, 0, nKt, row, k + 4 * h)) = make_uint4(t[0], t[1], t[2],
                                                                                                    t[3]);
     }
-  } else {
-    // FP64 tiles XOR bits 2-3 of the in-row index: element pairs (2u, 2u+1) stay adjacent
-#pragma unroll
-    for (int u = 0; u < kMpoVec; u += 2)
-      *reinterpret_cast<double2*>(img + img_byte_offset(MODE, 0, nKt, row, k + u)) =
-          make_double2(static_cast<double>(v[u]), static_cast<double>(v[u + 1]));
   }
 }
 

@@ -390,8 +390,9 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
     e = cudaMallocAsync(&ws, sizeof(double) * BM * BN * static_cast<size_t>(L.n_tiles) * L.parts, st);
     if (e != cudaSuccess) return e;
   }
+  // a tile is a few us: the launch overlap still shows at 10^4 tiles
   e = launch_pdl(kernel, static_cast<unsigned>(L.n_tiles) * L.split * L.parts, 32 * WM * WN, smem, st, L.split,
-                 L.n_tiles, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws, L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
+                 L.n_tiles / 16, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws, L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
   if (L.parts > 1) {
     if (e == cudaSuccess) {
       contract_parts_kernel<<<dim3(L.n_tiles, (BM * BN + 255) / 256), 256, 0, st>>>(ws, L.c, L.tiles, L.tab, L.parts,
@@ -496,20 +497,25 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_spl
 std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks,
                                          int shape) {
   const Shape& h = kShapes[shape];
-  std::vector<std::pair<int64_t, ContractTile>> tl;
+  struct Rec {
+    int64_t cost;
+    int32_t blk, m0, n0;
+  };
+  std::vector<Rec> tl;
   for (size_t i = 0; i < proto.size(); ++i)
     for (int64_t m0 = 0; m0 < proto[i].M; m0 += h.bm)
       for (int64_t n0 = 0; n0 < proto[i].N; n0 += h.bn) {
-        ContractTile t = proto[i];
-        t.m0 = static_cast<int32_t>(m0);
-        t.n0 = static_cast<int32_t>(n0);
-        const int64_t fm = (std::min<int64_t>(h.bm, t.M - m0) + 7) / 8, fn = (std::min<int64_t>(h.bn, t.N - n0) + 7) / 8;
-        tl.push_back({blks[i].k4 * fm * fn, t});
+        const int64_t fm = (std::min<int64_t>(h.bm, proto[i].M - m0) + 7) / 8,
+                      fn = (std::min<int64_t>(h.bn, proto[i].N - n0) + 7) / 8;
+        tl.push_back({blks[i].k4 * fm * fn, static_cast<int32_t>(i), static_cast<int32_t>(m0), static_cast<int32_t>(n0)});
       }
-  std::stable_sort(tl.begin(), tl.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-  std::vector<ContractTile> out;
-  out.reserve(tl.size());
-  for (const auto& x : tl) out.push_back(x.second);
+  std::stable_sort(tl.begin(), tl.end(), [](const Rec& a, const Rec& b) { return a.cost > b.cost; });
+  std::vector<ContractTile> out(tl.size());
+  for (size_t k = 0; k < tl.size(); ++k) {
+    out[k] = proto[tl[k].blk];
+    out[k].m0 = tl[k].m0;
+    out[k].n0 = tl[k].n0;
+  }
   return out;
 }
 
