@@ -10,6 +10,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/tenax_b200.h"
@@ -2003,16 +2004,34 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
     for (size_t k = 0; k < H.L.keys.size(); ++k) l_blk[H.L.offs[k]] = k;
     const int64_t r0 = static_cast<int64_t>(reinterpret_cast<uint64_t>(h->r_img.p) / 8);
     // stage 1: (group, row or column origin) -> K origin -> block
-    std::map<std::pair<int32_t, int32_t>, std::map<int32_t, const PackSeg*>> lmap, tmap;
-    for (const PackSeg& s : H.s1.packA) lmap[{s.group, s.row0}][s.k0] = &s;
-    for (const PackSeg& s : H.s1.packB) tmap[{s.group, s.row0}][s.k0] = &s;
+    using SegRef = std::tuple<int32_t, int32_t, int32_t, const PackSeg*>;
+    auto by_origin = [](const std::vector<PackSeg>& segs) {
+      std::vector<SegRef> v;
+      v.reserve(segs.size());
+      for (const PackSeg& s : segs) v.emplace_back(s.group, s.row0, s.k0, &s);
+      std::sort(v.begin(), v.end());
+      // an empty block shares its origin with the next one: the last stands
+      size_t n = 0;
+      for (size_t k = 0; k < v.size(); ++k)
+        if (k + 1 == v.size() || std::get<0>(v[k]) != std::get<0>(v[k + 1]) || std::get<1>(v[k]) != std::get<1>(v[k + 1]) ||
+            std::get<2>(v[k]) != std::get<2>(v[k + 1]))
+          v[n++] = v[k];
+      v.resize(n);
+      return v;
+    };
+    const std::vector<SegRef> lseg = by_origin(H.s1.packA), tseg = by_origin(H.s1.packB);
+    auto range = [](const std::vector<SegRef>& v, int32_t g, int32_t row0) {
+      const auto lo = std::lower_bound(v.begin(), v.end(), SegRef{g, row0, INT32_MIN, nullptr});
+      auto hi = lo;
+      while (hi != v.end() && std::get<0>(*hi) == g && std::get<1>(*hi) == row0) ++hi;
+      return std::make_pair(lo, hi);
+    };
     for (size_t p = 0; p < H.pairs.size(); ++p) {
       const MpoPair& mp = H.pairs[p];
       for (size_t k = 0; k < mp.ins.size(); ++k) {
         const MpoIn& in = mp.ins[k];
-        const auto il = lmap.find({in.g1, in.row0});
-        const auto it = tmap.find({in.g1, in.col0});
-        if (il == lmap.end() || it == tmap.end()) throw PlanError{TNX_ERR_RUNTIME, "internal: X1 block without operands"};
+        const auto il = range(lseg, in.g1, in.row0), it = range(tseg, in.g1, in.col0);
+        if (il.first == il.second || it.first == it.second) throw PlanError{TNX_ERR_RUNTIME, "internal: X1 block without operands"};
         for (int32_t pq = 0; pq < in.mp * in.mq; ++pq)
           for (int32_t b0 = 0; b0 < in.mb;) {
             auto at = [&](int32_t bb) { return x1[i][p][mp.in_slot0[k] + bb * in.mp * in.mq + pq]; };
@@ -2023,10 +2042,12 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
             int32_t b1 = b0 + 1;
             while (b1 < in.mb && at(b1) >= 0) ++b1;
             const size_t first = s1[i].spans.size();
-            for (const auto& kv : il->second) {
-              const auto jt = it->second.find(kv.first);
-              if (jt == it->second.end()) continue;
-              const PackSeg &l = *kv.second, &t = *jt->second;  // L[a, b, c], theta[a, p, q, d]
+            auto jt = it.first;
+            for (auto lt = il.first; lt != il.second; ++lt) {  // both in order of K
+              const int32_t k0 = std::get<2>(*lt);
+              while (jt != it.second && std::get<2>(*jt) < k0) ++jt;
+              if (jt == it.second || std::get<2>(*jt) != k0) continue;
+              const PackSeg &l = *std::get<3>(*lt), &t = *std::get<3>(*jt);  // L[a, b, c], theta[a, p, q, d]
               ContractSpan g{};
               g.a_off = l0 + h->l_off[l_blk.at(l.src_off)] + b0 * even(mp.mc);
               g.b_off = t.src_off + static_cast<int64_t>(pq) * mp.md;
@@ -2073,8 +2094,11 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
       }
     }
     // stage 4: products by theta block and (s, t)
-    std::map<Key, size_t> th_idx;
-    for (size_t k = 0; k < H.th.keys.size(); ++k) th_idx[H.th.keys[k]] = k;
+    std::map<std::array<int32_t, 4>, size_t> th_idx;
+    for (size_t k = 0; k < H.th.keys.size(); ++k) {
+      const Key& q = H.th.keys[k];
+      th_idx[{q[0], q[1], q[2], q[3]}] = k;
+    }
     std::vector<std::vector<std::vector<ContractSpan>>> prod(H.th.keys.size());
     for (size_t k = 0; k < H.th.keys.size(); ++k) prod[k].resize(H.th.dims[k][1] * H.th.dims[k][2]);
     std::map<std::pair<int32_t, int32_t>, std::vector<size_t>> r_by;  // (q_d, q_f) -> R blocks
@@ -2097,7 +2121,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
         for (size_t rk : rb->second) {
           const auto& rd = H.R.dims[rk];
           if (rd[0] != mp.md || rd[1] != o.mf || rd[2] == 0) continue;
-          const auto ti = th_idx.find(Key{mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
+          const auto ti = th_idx.find({mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
           if (ti == th_idx.end()) continue;
           ContractSpan g{};
           g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
@@ -2110,6 +2134,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
             const int32_t slot = mp.out_slot0[k] + e, st = e / o.mf, f = e % o.mf;
             if (tb[slot] == tb[slot + 1]) continue;
             auto& dst = prod[ti->second].at(st);
+            if (dst.empty()) dst.reserve(32);
             const int64_t r = r0 + h->r_off[rk] + f * even(rd[2]);
             if (formed[i][p][slot]) {
               g.a_off = static_cast<int64_t>(x3_base / 8) + x3[i][p][slot];

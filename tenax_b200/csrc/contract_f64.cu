@@ -497,24 +497,39 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_spl
 std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks,
                                          int shape) {
   const Shape& h = kShapes[shape];
-  struct Rec {
-    int64_t cost;
-    int32_t blk, m0, n0;
+  // a block's tiles fall into four rectangles of one cost each (interior, last
+  // column, last row, corner): these are sorted, not the tiles
+  struct Rect {
+    int64_t cost, m0, m1, n0, n1;
+    size_t blk;
   };
-  std::vector<Rec> tl;
-  for (size_t i = 0; i < proto.size(); ++i)
-    for (int64_t m0 = 0; m0 < proto[i].M; m0 += h.bm)
-      for (int64_t n0 = 0; n0 < proto[i].N; n0 += h.bn) {
-        const int64_t fm = (std::min<int64_t>(h.bm, proto[i].M - m0) + 7) / 8,
-                      fn = (std::min<int64_t>(h.bn, proto[i].N - n0) + 7) / 8;
-        tl.push_back({blks[i].k4 * fm * fn, static_cast<int32_t>(i), static_cast<int32_t>(m0), static_cast<int32_t>(n0)});
+  std::vector<Rect> rects;
+  rects.reserve(4 * proto.size());
+  int64_t n = 0;
+  for (size_t i = 0; i < proto.size(); ++i) {
+    const int64_t M = proto[i].M, N = proto[i].N, mf = M / h.bm * h.bm, nf = N / h.bn * h.bn;
+    auto add = [&](int64_t m0, int64_t m1, int64_t n0, int64_t n1) {
+      if (m0 >= m1 || n0 >= n1) return;
+      const int64_t fm = (std::min<int64_t>(h.bm, m1 - m0) + 7) / 8, fn = (std::min<int64_t>(h.bn, n1 - n0) + 7) / 8;
+      rects.push_back({blks[i].k4 * fm * fn, m0, m1, n0, n1, i});
+      n += ((m1 - m0 + h.bm - 1) / h.bm) * ((n1 - n0 + h.bn - 1) / h.bn);
+    };
+    add(0, mf, 0, nf);
+    add(0, mf, nf, N);
+    add(mf, M, 0, nf);
+    add(mf, M, nf, N);
+  }
+  std::stable_sort(rects.begin(), rects.end(), [](const Rect& a, const Rect& b) { return a.cost > b.cost; });
+  std::vector<ContractTile> out;
+  out.reserve(static_cast<size_t>(n));
+  for (const Rect& r : rects) {
+    ContractTile t = proto[r.blk];
+    for (int64_t m0 = r.m0; m0 < r.m1; m0 += h.bm)
+      for (int64_t n0 = r.n0; n0 < r.n1; n0 += h.bn) {
+        t.m0 = static_cast<int32_t>(m0);
+        t.n0 = static_cast<int32_t>(n0);
+        out.push_back(t);
       }
-  std::stable_sort(tl.begin(), tl.end(), [](const Rec& a, const Rec& b) { return a.cost > b.cost; });
-  std::vector<ContractTile> out(tl.size());
-  for (size_t k = 0; k < tl.size(); ++k) {
-    out[k] = proto[tl[k].blk];
-    out[k].m0 = tl[k].m0;
-    out[k].n0 = tl[k].n0;
   }
   return out;
 }
