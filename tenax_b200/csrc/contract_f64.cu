@@ -390,7 +390,8 @@ cudaError_t go(const ContractLaunch& L, cudaStream_t st) {
     e = cudaMallocAsync(&ws, sizeof(double) * BM * BN * static_cast<size_t>(L.n_tiles) * L.parts, st);
     if (e != cudaSuccess) return e;
   }
-  // a tile is a few us: the launch overlap still shows at 10^4 tiles
+  // a tile is a few us: the launch overlap still shows at 10^4 tiles (an
+  // environment update's three steps, chi = 512: 93 us without it, 85 with)
   e = launch_pdl(kernel, static_cast<unsigned>(L.n_tiles) * L.split * L.parts, 32 * WM * WN, smem, st, L.split,
                  L.n_tiles / 16, L.a, L.b, L.c, L.tiles, L.spans, L.tab, L.split, L.parts, ws, L.a_ptrs, L.b_ptrs, L.c_ptrs, L.skip);
   if (L.parts > 1) {
