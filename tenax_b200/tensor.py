@@ -102,6 +102,12 @@ class SymmetricTensor:
         self._key_pos = layout.key_pos
         self._blocks_cache = None
 
+    def __setstate__(self, state):
+        for name, value in state[1].items():
+            setattr(self, name, value)
+        if "_layout" not in state[1]:  # pickled before layouts were kept
+            self._layout = Layout(tuple(self._keys), self._offsets, self._shapes, self._key_pos)
+
     @classmethod
     def from_flat(cls, indices, keys, data: torch.Tensor) -> "SymmetricTensor":
         """Wrap an existing flat buffer (blocks in the given sorted key order)."""
@@ -121,7 +127,8 @@ class SymmetricTensor:
         if not self._indices:
             return
         sym = self._indices[0].symmetry
-        if type(sym) in _INTEGER_FUSE and self._keys and len(self._indices) > 1:
+        n_legs = len(self._indices)
+        if type(sym) in _INTEGER_FUSE and self._keys and n_legs > 1 and all(len(k) == n_legs for k in self._keys):
             # charges that add (mod n): every block in one product
             tot = np.array(self._keys, dtype=np.int64) @ np.array([int(i.flow) for i in self._indices], np.int64)
             n = sym.n_values()

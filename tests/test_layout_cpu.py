@@ -1,7 +1,9 @@
 """Block layouts counted once per leg, and the conservation check of all blocks at once."""
 
+import copy
 import itertools
 import math
+import pickle
 
 import numpy as np
 import pytest
@@ -45,3 +47,24 @@ def test_validate_agrees_with_fuse_many(sym, n):
         else:
             with pytest.raises(ValueError, match="charge conservation"):
                 t._validate()
+
+
+def test_pickles_with_and_without_a_layout():
+    idx = _legs(U1Symmetry(), 2)
+    keys = [(q, q) for q in range(3) if math.prod(block_shape(idx, (q, q)))]
+    n = sum(math.prod(block_shape(idx, k)) for k in keys)
+    t = SymmetricTensor.from_flat(idx, keys, torch.arange(n, dtype=torch.float64))
+    state = {s: getattr(t, s) for s in SymmetricTensor.__slots__ if s != "_layout"}
+    old = object.__new__(SymmetricTensor)
+    old.__setstate__((None, state))  # as a tensor written before layouts were kept comes back
+    for u in (pickle.loads(pickle.dumps(t)), copy.deepcopy(t), old):
+        assert u._layout.keys == tuple(keys) and u._layout.shapes == t._layout.shapes
+        assert u._layout.offsets.tolist() == t._layout.offsets.tolist() and u._layout.key_pos == t._layout.key_pos
+        assert torch.equal(u.data if hasattr(u, "data") else u._data, t._data)
+
+
+def test_validate_reads_only_the_charges_a_leg_has():
+    idx = _legs(U1Symmetry(), 2)
+    t = SymmetricTensor.from_flat(idx, [(0, 0)], torch.zeros(math.prod(block_shape(idx, (0, 0))), dtype=torch.float64))
+    t._keys = [(0, 0, 5), (1, 1, 7)]
+    t._validate()
