@@ -828,14 +828,15 @@ bool build_direct(const PairPlan& P, StepDev& d) {
   L.b_kfast = b_kfast;
   L.a_vec = a_vec;
   L.b_vec = b_vec;
-  const std::vector<ContractTile> tiles = contract_tiles(proto, blks, L.shape);
-  if (static_cast<int64_t>(tiles.size()) * L.split * L.parts > INT32_MAX) return false;
-  L.n_tiles = static_cast<int>(tiles.size());
   // one buffer, one copy: spans, tiles, axis tables
-  const size_t o_t = spans.size() * sizeof(ContractSpan), o_x = o_t + tiles.size() * sizeof(ContractTile);
-  std::vector<uint8_t> h(std::max<size_t>(64, o_x + T.tab.size() * sizeof(int32_t)));
-  if (!spans.empty()) std::memcpy(h.data(), spans.data(), spans.size() * sizeof(ContractSpan));
-  if (!tiles.empty()) std::memcpy(h.data() + o_t, tiles.data(), tiles.size() * sizeof(ContractTile));
+  const size_t o_t = spans.size() * sizeof(ContractSpan);
+  std::vector<uint8_t> h(o_t);
+  if (o_t) std::memcpy(h.data(), spans.data(), o_t);
+  const int64_t n_tiles = contract_tiles(proto, blks, L.shape, h);
+  if (n_tiles * L.split * L.parts > INT32_MAX) return false;
+  L.n_tiles = static_cast<int>(n_tiles);
+  const size_t o_x = h.size();
+  h.resize(std::max<size_t>(64, o_x + T.tab.size() * sizeof(int32_t)));
   if (!T.tab.empty()) std::memcpy(h.data() + o_x, T.tab.data(), T.tab.size() * sizeof(int32_t));
   upload(d.blob, h);
   uint8_t* base = d.blob.as<uint8_t>();
@@ -1826,8 +1827,9 @@ struct tnx_heff_batch {
   int32_t route_win_max = 0;  // records in the largest (tile, lane quarter, chunk) window
   const int32_t* skip = nullptr;
   // FP64: stage 1 (L . theta -> X1 slots), the sums of the multi-term slots
-  // (mpo_* tables, outputs in f64_oslots) and stage 4, all on plain blocks
-  DevMem f64_oslots;
+  // (tables in f64_mpo, these offsets) and stage 4, all on plain blocks
+  DevMem f64_mpo;
+  size_t f64_mpo_off[5] = {0, 0, 0, 0, 0};  // pairs, X1 slots, sums, terms, chunks
   std::vector<std::unique_ptr<DevMem>> f64_blobs;
   std::vector<ContractLaunch> f64_s1, f64_s4;  // one launch per K split among the operators
   // FP64 of one operator: theta and the output travel as kernel arguments, so an
@@ -1909,18 +1911,17 @@ std::vector<ContractLaunch> f64_launches(const std::vector<F64Stage>& ops, bool 
   for (const auto& kv : by) {
     ContractLaunch L{};
     contract_choose(kv.second.blks, sms, kv.first, kv.first, &L.shape, &L.split, &L.parts);
-    const std::vector<ContractTile> tiles = contract_tiles(kv.second.proto, kv.second.blks, L.shape);
-    if (static_cast<int64_t>(tiles.size()) * L.split > INT32_MAX)
-      throw PlanError{TNX_ERR_UNSUPPORTED, "too many output tiles in one batch"};
-    L.n_tiles = static_cast<int>(tiles.size());
+    const size_t o_t = kv.second.spans.size() * sizeof(ContractSpan);
+    std::vector<uint8_t> h(o_t);
+    if (o_t) std::memcpy(h.data(), kv.second.spans.data(), o_t);
+    const int64_t n_tiles = contract_tiles(kv.second.proto, kv.second.blks, L.shape, h);
+    if (n_tiles * L.split > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "too many output tiles in one batch"};
+    L.n_tiles = static_cast<int>(n_tiles);
+    h.resize(std::max<size_t>(64, h.size()));
     L.a_kfast = a_kfast;
     L.b_kfast = false;
     L.a_vec = true;  // padded copies and slots; bases are null, offsets absolute
     L.b_vec = b_vec;
-    const size_t o_t = kv.second.spans.size() * sizeof(ContractSpan);
-    std::vector<uint8_t> h(std::max<size_t>(64, o_t + tiles.size() * sizeof(ContractTile)));
-    if (o_t) std::memcpy(h.data(), kv.second.spans.data(), o_t);
-    if (!tiles.empty()) std::memcpy(h.data() + o_t, tiles.data(), tiles.size() * sizeof(ContractTile));
     blobs.push_back(std::make_unique<DevMem>());
     upload(*blobs.back(), h);
     L.spans = reinterpret_cast<const ContractSpan*>(blobs.back()->as<uint8_t>());
@@ -2175,12 +2176,23 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
   b->f64_s1 = f64_launches(s1, false, false, b->f64_blobs);
   // stage 4: X1 slots [c, d] and R[d, f, g], both padded
   b->f64_s4 = f64_launches(s4, true, true, b->f64_blobs);
-  upload(b->mpo_pairs, MP);
-  upload(b->mpo_slots, MI);
-  upload(b->f64_oslots, MO);
-  upload(b->mpo_terms, MT);
-  upload(b->mpo_chunks, MC);
   b->n_mpo_chunks = static_cast<int>(MC.size());
+  if (b->n_mpo_chunks > 0) {  // one buffer, one copy
+    std::vector<uint8_t> tab;
+    int part = 0;
+    auto add = [&](const auto& v) {
+      b->f64_mpo_off[part++] = tab.size();
+      const auto* raw = reinterpret_cast<const uint8_t*>(v.data());
+      tab.insert(tab.end(), raw, raw + v.size() * sizeof(v[0]));
+      tab.resize((tab.size() + 15) / 16 * 16);
+    };
+    add(MP);
+    add(MI);
+    add(MO);
+    add(MT);
+    add(MC);
+    upload(b->f64_mpo, tab);
+  }
   if (!b->one()) {
     b->src_tab.alloc(sizeof(PtrTab));
     b->out_tab4.alloc(sizeof(PtrTab));
@@ -2853,8 +2865,10 @@ static void heff_batch_stage(tnx_heff_batch* b, int stage, cudaStream_t st, cons
         CUDA_OK(launch_contract_f64(L, st));
       }
     } else if (stage == 2) {
-      launch_mpo_sum(b->mpo_pairs.as<DevMpoPair>(), b->mpo_slots.as<DevMpoSlot>(), b->f64_oslots.as<DevMpoSlot>(),
-                     b->mpo_terms.as<DevMpoTerm>(), b->mpo_chunks.as<int2>(), b->n_mpo_chunks, b->skip, st);
+      auto tab = [&](int part) { return b->f64_mpo.as<uint8_t>() + b->f64_mpo_off[part]; };
+      launch_mpo_sum(reinterpret_cast<const DevMpoPair*>(tab(0)), reinterpret_cast<const DevMpoSlot*>(tab(1)),
+                     reinterpret_cast<const DevMpoSlot*>(tab(2)), reinterpret_cast<const DevMpoTerm*>(tab(3)),
+                     reinterpret_cast<const int2*>(tab(4)), b->n_mpo_chunks, b->skip, st);
     }
     return;
   }

@@ -28,6 +28,7 @@
 // ms (31.6 TFLOP/s; the packed path's GEMM alone 4.15 ms).  Below about a
 // thousand tiles the last wave and one or two CTAs an SM are what is lost.
 #include <algorithm>
+#include <cstring>
 
 #include "common.cuh"
 #include "contract_f64.hpp"
@@ -495,8 +496,8 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_spl
   }
 }
 
-std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks,
-                                         int shape) {
+int64_t contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks, int shape,
+                       std::vector<uint8_t>& dst) {
   const Shape& h = kShapes[shape];
   // a block's tiles fall into four rectangles of one cost each (interior, last
   // column, last row, corner): these are sorted, not the tiles
@@ -521,18 +522,19 @@ std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto,
     add(mf, M, nf, N);
   }
   std::stable_sort(rects.begin(), rects.end(), [](const Rect& a, const Rect& b) { return a.cost > b.cost; });
-  std::vector<ContractTile> out;
-  out.reserve(static_cast<size_t>(n));
+  size_t at = dst.size();
+  dst.resize(at + static_cast<size_t>(n) * sizeof(ContractTile));
   for (const Rect& r : rects) {
     ContractTile t = proto[r.blk];
     for (int64_t m0 = r.m0; m0 < r.m1; m0 += h.bm)
       for (int64_t n0 = r.n0; n0 < r.n1; n0 += h.bn) {
         t.m0 = static_cast<int32_t>(m0);
         t.n0 = static_cast<int32_t>(n0);
-        out.push_back(t);
+        std::memcpy(dst.data() + at, &t, sizeof(t));
+        at += sizeof(t);
       }
   }
-  return out;
+  return n;
 }
 
 cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st) {

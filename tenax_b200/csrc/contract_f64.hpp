@@ -57,10 +57,10 @@ constexpr int kContractShapes = 4;
 // on the tile shape.
 void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_split, int max_split, int* shape,
                      int* split, int* parts);
-// tiles of the blocks `proto` (M, N and the block's axes set) in the launch's
-// shape, longest first
-std::vector<ContractTile> contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks,
-                                         int shape);
+// appends to `dst` the tiles of the blocks `proto` (M, N and the block's axes
+// set) in the launch's shape, longest first; returns their number
+int64_t contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks, int shape,
+                       std::vector<uint8_t>& dst);
 cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st);
 
 }  // namespace tnx
