@@ -758,13 +758,14 @@ __global__ void lanczos_axpy_kernel(double* __restrict__ w, const double* __rest
 
 // beta = ||w|| from the partial sums; stop when beta < tol (the reference's
 // absolute test) or, with an inexact matvec, when beta < tol_rel * |alpha|
-// (below the matvec's noise); otherwise v_next = w / beta.  A block that finds
-// *done set by block 0 of this launch has nothing to write: every block makes
-// the same decision.
+// (below the matvec's noise); otherwise v_next = w / beta.  Block 0 sets *done
+// in the launch whose other blocks read it, so one thread reads it for its
+// block: a block leaves whole or reduces whole.  One that leaves because block 0
+// has just stopped would have stopped too (every block forms the same sum).
 __global__ void lanczos_next_kernel(const double* w, double* vnext, int64_t n, const double* __restrict__ pnorm,
                                     double* __restrict__ beta_out, const double* __restrict__ alpha, double tol,
-                                    double tol_rel, int32_t* done) {
-  if (*done) return;
+                                    double tol_rel, volatile int32_t* done) {
+  if (__syncthreads_or(threadIdx.x == 0 && *done)) return;
   const double b = sqrt(partials_total(pnorm));
   const bool stop = b < tol || b < tol_rel * fabs(*alpha);
   if (blockIdx.x == 0 && threadIdx.x == 0) {

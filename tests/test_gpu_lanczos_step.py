@@ -72,3 +72,19 @@ def test_dot_and_norm(n):
     assert abs(d - math.fsum((x * y).tolist())) <= (n + 2) * U * math.fsum((x * y).abs().tolist())
     nn = float(vector.nrm2(x.cuda()))
     assert abs(nn - math.sqrt(math.fsum((x * x).tolist()))) <= (n + 4) * U * max(nn, 1e-300)
+
+
+@pytest.mark.parametrize("n", [65537, 300001, 2000003])
+def test_no_block_writes_the_next_vector_on_a_stop(n):
+    """The three-launch step stops in the launch that would write v_next, while
+    its blocks start: none of them may write, in any of many steps."""
+    w, v = torch.ones(n, dtype=torch.float64, device="cuda"), torch.ones(n, dtype=torch.float64, device="cuda")
+    alpha = torch.zeros(2, dtype=torch.float64, device="cuda")
+    beta = torch.zeros(3, dtype=torch.float64, device="cuda")
+    done = torch.zeros(1, dtype=torch.int32, device="cuda")
+    vn = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+    for _ in range(200):
+        w.fill_(1.0)
+        done.zero_()
+        _step(w, v, None, vn, n, alpha, beta, 0, 1e300, 0.0, done)
+    assert int(done) == 1 and bool((vn == 7.0).all())
