@@ -1494,6 +1494,7 @@ struct tnx_heff {
   // divided by their powers of two; output slots with a single term of one of
   // these weights are never formed, the others are when mpo_sum is set
   std::vector<double> weights;
+  std::vector<std::vector<int32_t>> term_copy;  // per pair and term: the copy of R of its weight, or -1
   bool mpo_sum = false;
   std::vector<int64_t> l_off, r_off;  // element offset of each block in its copy
   int64_t l_total = 0, r_total = 0;   // elements of one copy
@@ -1618,33 +1619,84 @@ void padded_copies(const TensorStruct& T, const double* src, const double* scale
   CUDA_OK(cudaStreamSynchronize(st));
 }
 
+// The distinct values among the terms' weights, by their bits.  An MPO has a
+// handful, found fastest by looking through them; a map beyond that.
+struct WeightIds {
+  std::vector<double> value;
+  std::unordered_map<uint64_t, int32_t> many;
+  int32_t id(double w) {
+    uint64_t bits;
+    std::memcpy(&bits, &w, 8);
+    if (value.size() <= 16) {
+      for (size_t i = 0; i < value.size(); ++i)
+        if (std::memcmp(&value[i], &w, 8) == 0) return static_cast<int32_t>(i);
+    } else if (auto it = many.find(bits); it != many.end()) {
+      return it->second;
+    }
+    const int32_t n = static_cast<int32_t>(value.size());
+    value.push_back(w);
+    if (value.size() == 17)
+      for (int32_t i = 0; i < n; ++i) {
+        uint64_t v;
+        std::memcpy(&v, &value[i], 8);
+        many[v] = i;
+      }
+    if (value.size() >= 17) many[bits] = n;
+    return n;
+  }
+};
+
 void choose_f64_weights(tnx_heff* h) {
   const HeffPlan& H = h->H;
-  std::map<double, int64_t> single, all;
+  std::map<int32_t, int64_t> widest;  // columns stage 4 gives the slots of a d sector
+  for (size_t b = 0; b < H.R.keys.size(); ++b) {
+    int64_t& m = widest[H.R.keys[b][0]];
+    m = std::max(m, H.R.dims[b][2]);
+  }
+  WeightIds ids;
+  std::vector<int64_t> single, all;
+  h->term_copy.assign(H.pairs.size(), {});
   double extra = 0.0;
-  for (const MpoPair& mp : H.pairs) {
-    std::vector<int32_t> n(mp.n_out_slots, 0);
+  std::vector<int32_t> n;
+  for (size_t p = 0; p < H.pairs.size(); ++p) {
+    const MpoPair& mp = H.pairs[p];
+    n.assign(mp.n_out_slots, 0);
     for (const MpoTerm& t : mp.terms) ++n[t.out_slot];
-    int64_t mg = 0;  // columns stage 4 gives this pair's slots
-    for (size_t b = 0; b < H.R.keys.size(); ++b)
-      if (H.R.keys[b][0] == mp.qd) mg = std::max(mg, H.R.dims[b][2]);
+    const auto wd = widest.find(mp.qd);
+    const int64_t mg = wd == widest.end() ? 0 : wd->second;
+    std::vector<int32_t>& id = h->term_copy[p];
+    id.reserve(mp.terms.size());
     for (const MpoTerm& t : mp.terms) {
-      ++all[t.w];
-      if (n[t.out_slot] == 1) ++single[t.w];
+      id.push_back(ids.id(t.w));
+      if (ids.value.size() > all.size()) {
+        all.push_back(0);
+        single.push_back(0);
+      }
+      ++all[id.back()];
+      if (n[t.out_slot] == 1) ++single[id.back()];
     }
     for (int32_t k : n)
       if (k > 1) extra += 2.0 * (k - 1) * static_cast<double>(mp.mc) * mp.md * static_cast<double>(mg);
   }
   h->mpo_sum = extra > kF64ExtraFlops || all.size() > kF64Weights;
-  std::vector<std::pair<int64_t, double>> by;
-  for (const auto& kv : h->mpo_sum ? single : all)
-    if (kv.first != 1.0) by.push_back({kv.second, kv.first});
-  std::sort(by.begin(), by.end(), [](const auto& x, const auto& y) {
-    return x.first != y.first ? x.first > y.first : x.second < y.second;
+  std::vector<int32_t> by;  // weights worth a copy, most used first
+  const std::vector<int64_t>& count = h->mpo_sum ? single : all;
+  for (size_t i = 0; i < all.size(); ++i)
+    if (ids.value[i] != 1.0 && !std::isnan(ids.value[i]) && count[i] > 0) by.push_back(static_cast<int32_t>(i));
+  std::sort(by.begin(), by.end(), [&](int32_t x, int32_t y) {
+    return count[x] != count[y] ? count[x] > count[y] : ids.value[x] < ids.value[y];
   });
   h->weights.assign(1, 1.0);
-  for (const auto& w : by)
-    if (h->weights.size() < kF64Weights) h->weights.push_back(w.second);
+  std::vector<int32_t> copy(all.size(), -1);
+  for (size_t i = 0; i < all.size(); ++i)
+    if (ids.value[i] == 1.0) copy[i] = 0;
+  for (int32_t i : by)
+    if (h->weights.size() < kF64Weights) {
+      copy[i] = static_cast<int32_t>(h->weights.size());
+      h->weights.push_back(ids.value[i]);
+    }
+  for (auto& v : h->term_copy)
+    for (int32_t& i : v) i = copy[i];
 }
 }  // namespace
 
@@ -1867,16 +1919,25 @@ struct tnx_heff_batch {
 }  // extern "C"
 
 namespace {
+struct Key4Hash {
+  size_t operator()(const std::array<int32_t, 4>& k) const noexcept {
+    uint64_t h = 0;
+    for (int32_t v : k) h = (h ^ static_cast<uint32_t>(v)) * 0x9e3779b97f4a7c15ull, h ^= h >> 29;
+    return static_cast<size_t>(h);
+  }
+};
+
 // One operator's products of one stage.
 struct F64Stage {
   std::vector<ContractSpan> spans;
   std::vector<ContractTile> proto;
   std::vector<ContractBlk> blks;
-  void close(ContractTile t, size_t first) {
+  // output matrix `t` sums the products [first, last)
+  void close(ContractTile t, size_t first, size_t last) {
     ContractBlk k{};
     t.span0 = static_cast<int32_t>(first);
-    t.nspan = static_cast<int32_t>(spans.size() - first);
-    for (size_t u = first; u < spans.size(); ++u) {
+    t.nspan = static_cast<int32_t>(last - first);
+    for (size_t u = first; u < last; ++u) {
       k.ktiles += cdiv(spans[u].K, 16);
       k.k4 += cdiv(spans[u].K, 4);
     }
@@ -1894,27 +1955,44 @@ struct F64Stage {
 std::vector<ContractLaunch> f64_launches(const std::vector<F64Stage>& ops, bool a_kfast, bool b_vec,
                                          std::vector<std::unique_ptr<DevMem>>& blobs) {
   const int sms = device_sm_count();
-  std::map<int, F64Stage> by;
-  int shape = 0, split = 1, parts = 1;
+  struct Group {
+    int shape = 0, split = 1, parts = 1;
+    std::vector<const F64Stage*> ops;
+  };
+  std::map<int, Group> by;
   for (const F64Stage& o : ops) {
-    contract_choose(o.blks, sms, 1, 8, &shape, &split, &parts);
-    F64Stage& g = by[split];
-    const int32_t s0 = static_cast<int32_t>(g.spans.size());
-    g.spans.insert(g.spans.end(), o.spans.begin(), o.spans.end());
-    g.blks.insert(g.blks.end(), o.blks.begin(), o.blks.end());
-    for (ContractTile t : o.proto) {
-      t.span0 += s0;
-      g.proto.push_back(t);
-    }
+    Group c;
+    contract_choose(o.blks, sms, 1, 8, &c.shape, &c.split, &c.parts);
+    c.ops = std::move(by[c.split].ops);
+    c.ops.push_back(&o);
+    by[c.split] = std::move(c);
   }
   std::vector<ContractLaunch> out;
-  for (const auto& kv : by) {
+  for (auto& kv : by) {
+    Group& c = kv.second;
+    F64Stage joined;
+    const F64Stage* g = c.ops[0];
+    if (c.ops.size() > 1) {
+      for (const F64Stage* o : c.ops) {
+        const int32_t s0 = static_cast<int32_t>(joined.spans.size());
+        joined.spans.insert(joined.spans.end(), o->spans.begin(), o->spans.end());
+        joined.blks.insert(joined.blks.end(), o->blks.begin(), o->blks.end());
+        for (ContractTile t : o->proto) {
+          t.span0 += s0;
+          joined.proto.push_back(t);
+        }
+      }
+      g = &joined;
+      contract_choose(g->blks, sms, kv.first, kv.first, &c.shape, &c.split, &c.parts);
+    }
     ContractLaunch L{};
-    contract_choose(kv.second.blks, sms, kv.first, kv.first, &L.shape, &L.split, &L.parts);
-    const size_t o_t = kv.second.spans.size() * sizeof(ContractSpan);
+    L.shape = c.shape;
+    L.split = c.split;
+    L.parts = c.parts;
+    const size_t o_t = g->spans.size() * sizeof(ContractSpan);
     std::vector<uint8_t> h(o_t);
-    if (o_t) std::memcpy(h.data(), kv.second.spans.data(), o_t);
-    const int64_t n_tiles = contract_tiles(kv.second.proto, kv.second.blks, L.shape, h);
+    if (o_t) std::memcpy(h.data(), g->spans.data(), o_t);
+    const int64_t n_tiles = contract_tiles(g->proto, g->blks, L.shape, h);
     if (n_tiles * L.split > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "too many output tiles in one batch"};
     L.n_tiles = static_cast<int>(n_tiles);
     h.resize(std::max<size_t>(64, h.size()));
@@ -1951,6 +2029,8 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
   std::vector<std::vector<std::vector<int64_t>>> x1(n), x3(n);  // [problem][pair][slot] -> element, -1
   std::vector<std::vector<std::vector<char>>> formed(n);        // [problem][pair][out slot]
   int64_t n1 = 0, n3 = 0;
+  std::vector<int32_t> cnt;
+  std::vector<char> plain, used;
   for (int i = 0; i < n; ++i) {
     const tnx_heff* h = b->hs[i];
     const HeffPlan& H = h->H;
@@ -1960,12 +2040,15 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
     for (size_t p = 0; p < H.pairs.size(); ++p) {
       const MpoPair& mp = H.pairs[p];
       const int64_t sz = even(mp.mc) * even(mp.md);  // pitch and rows even: 16-byte reads
-      std::vector<int32_t> cnt(mp.n_out_slots, 0);
-      std::vector<char> plain(mp.n_out_slots, 1), used(mp.n_in_slots, 0);
-      for (const MpoTerm& t : mp.terms) {
+      const std::vector<int32_t>& copy = h->term_copy[p];
+      cnt.assign(mp.n_out_slots, 0);
+      plain.assign(mp.n_out_slots, 1);
+      used.assign(mp.n_in_slots, 0);
+      for (size_t v = 0; v < mp.terms.size(); ++v) {
+        const MpoTerm& t = mp.terms[v];
         ++cnt[t.out_slot];
         used[t.in_slot] = 1;
-        if (std::find(h->weights.begin(), h->weights.end(), t.w) == h->weights.end()) plain[t.out_slot] = 0;
+        if (copy[v] < 0) plain[t.out_slot] = 0;
       }
       formed[i][p].assign(mp.n_out_slots, 0);
       x3[i][p].assign(mp.n_out_slots, -1);
@@ -1997,12 +2080,14 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
   std::vector<DevMpoSlot> MI, MO;
   std::vector<DevMpoTerm> MT;
   std::vector<int2> MC;
+  std::vector<int32_t> in_id, tb;
   for (int i = 0; i < n; ++i) {
     const tnx_heff* h = b->hs[i];
     const HeffPlan& H = h->H;
     const int64_t l0 = static_cast<int64_t>(reinterpret_cast<uint64_t>(h->l_img.p) / 8);
-    std::map<int64_t, size_t> l_blk;  // L block by its offset in the caller's buffer
-    for (size_t k = 0; k < H.L.keys.size(); ++k) l_blk[H.L.offs[k]] = k;
+    auto l_blk = [&](int64_t off) {  // L block by its offset in the caller's buffer (an empty one has the next one's)
+      return static_cast<size_t>(std::upper_bound(H.L.offs.begin(), H.L.offs.end(), off) - H.L.offs.begin()) - 1;
+    };
     const int64_t r0 = static_cast<int64_t>(reinterpret_cast<uint64_t>(h->r_img.p) / 8);
     // stage 1: (group, row or column origin) -> K origin -> block
     using SegRef = std::tuple<int32_t, int32_t, int32_t, const PackSeg*>;
@@ -2050,7 +2135,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
               if (jt == it.second || std::get<2>(*jt) != k0) continue;
               const PackSeg &l = *std::get<3>(*lt), &t = *std::get<3>(*jt);  // L[a, b, c], theta[a, p, q, d]
               ContractSpan g{};
-              g.a_off = l0 + h->l_off[l_blk.at(l.src_off)] + b0 * even(mp.mc);
+              g.a_off = l0 + h->l_off[l_blk(l.src_off)] + b0 * even(mp.mc);
               g.b_off = t.src_off + static_cast<int64_t>(pq) * mp.md;
               g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
               g.ar_str = 1;
@@ -2069,7 +2154,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
             t.r_str = static_cast<int32_t>(even(mp.md));
             t.c_str = 1;
             t.scale = 1.0;
-            s1[i].close(t, first);
+            s1[i].close(t, first, s1[i].spans.size());
             b0 = b1;
           }
       }
@@ -2080,13 +2165,23 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
       dp.in0 = static_cast<int32_t>(MI.size());
       dp.out0 = static_cast<int32_t>(MO.size());
       dp.term0 = static_cast<int32_t>(MT.size());
-      for (const MpoTerm& t : mp.terms)
-        if (formed[i][p][t.out_slot]) MT.push_back({t.out_slot, t.in_slot, t.w});
+      in_id.assign(mp.n_in_slots, -1);  // the slots that are read or formed, numbered in order of use
+      int32_t cur = -1;
+      for (const MpoTerm& t : mp.terms) {  // sorted by out_slot
+        if (!formed[i][p][t.out_slot]) continue;
+        if (t.out_slot != cur) {
+          cur = t.out_slot;
+          MO.push_back({x3_base + static_cast<uint64_t>(x3[i][p][cur]) * 8, even(mp.md)});
+        }
+        int32_t& in = in_id[t.in_slot];
+        if (in < 0) {
+          in = static_cast<int32_t>(MI.size()) - dp.in0;
+          MI.push_back({x1_base + static_cast<uint64_t>(x1[i][p][t.in_slot]) * 8, even(mp.md)});
+        }
+        MT.push_back({static_cast<int32_t>(MO.size()) - 1 - dp.out0, in, t.w});
+      }
       dp.n_terms = static_cast<int32_t>(MT.size()) - dp.term0;
       if (dp.n_terms > 0) {
-        for (int64_t e : x1[i][p]) MI.push_back({x1_base + static_cast<uint64_t>(std::max<int64_t>(0, e)) * 8, even(mp.md)});
-        for (int64_t e : x3[i][p])
-          MO.push_back({x3_base + static_cast<uint64_t>(std::max<int64_t>(0, e)) * 8, even(mp.md)});
         const int id = static_cast<int>(MP.size());
         MP.push_back(dp);
         const int64_t pts = static_cast<int64_t>(mp.mc) * mp.md;
@@ -2094,28 +2189,30 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
         for (int64_t p0 = 0; p0 < pts; p0 += mpo_points_per_cta()) MC.push_back(make_int2(id, static_cast<int>(p0)));
       }
     }
-    // stage 4: products by theta block and (s, t)
-    std::map<std::array<int32_t, 4>, size_t> th_idx;
+    // stage 4: products by theta block and (s, t), collected in order and then
+    // dealt to their output matrix
+    std::unordered_map<std::array<int32_t, 4>, size_t, Key4Hash> th_idx;
+    th_idx.reserve(H.th.keys.size());
+    std::vector<int32_t> st0(H.th.keys.size() + 1, 0);  // first output matrix of each theta block
     for (size_t k = 0; k < H.th.keys.size(); ++k) {
       const Key& q = H.th.keys[k];
       th_idx[{q[0], q[1], q[2], q[3]}] = k;
+      st0[k + 1] = st0[k] + static_cast<int32_t>(H.th.dims[k][1] * H.th.dims[k][2]);
     }
-    std::vector<std::vector<std::vector<ContractSpan>>> prod(H.th.keys.size());
-    for (size_t k = 0; k < H.th.keys.size(); ++k) prod[k].resize(H.th.dims[k][1] * H.th.dims[k][2]);
+    std::vector<ContractSpan> prod;
+    std::vector<int32_t> dest, first(st0.back() + 1, 0);
     std::map<std::pair<int32_t, int32_t>, std::vector<size_t>> r_by;  // (q_d, q_f) -> R blocks
     for (size_t k = 0; k < H.R.keys.size(); ++k) r_by[{H.R.keys[k][0], H.R.keys[k][1]}].push_back(k);
     for (size_t p = 0; p < H.pairs.size(); ++p) {
       const MpoPair& mp = H.pairs[p];
-      // terms of each output slot (they are sorted by it), their weights' R copies
-      std::vector<int32_t> tb(mp.n_out_slots + 1, 0), wi(mp.terms.size(), -1);
-      for (size_t v = 0; v < mp.terms.size(); ++v) {
-        ++tb[mp.terms[v].out_slot + 1];
-        const auto w = std::find(h->weights.begin(), h->weights.end(), mp.terms[v].w);
-        if (w != h->weights.end()) wi[v] = static_cast<int32_t>(w - h->weights.begin());
-      }
+      const std::vector<int32_t>& copy = h->term_copy[p];
+      tb.assign(mp.n_out_slots + 1, 0);  // terms of each output slot (they are sorted by it)
+      for (const MpoTerm& t : mp.terms) ++tb[t.out_slot + 1];
       for (int32_t o = 0; o < mp.n_out_slots; ++o) tb[o + 1] += tb[o];
       for (size_t k = 0; k < mp.outs.size(); ++k) {
         const MpoOut& o = mp.outs[k];
+        const int32_t slot0 = mp.out_slot0[k], n_slots = o.ms * o.mt * o.mf;
+        if (tb[slot0] == tb[slot0 + n_slots]) continue;
         const Key& ok = H.mpo_out_keys[p][k];  // (q_s, q_t, q_f)
         const auto rb = r_by.find({mp.qd, ok[2]});
         if (rb == r_by.end()) continue;
@@ -2124,6 +2221,8 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
           if (rd[0] != mp.md || rd[1] != o.mf || rd[2] == 0) continue;
           const auto ti = th_idx.find({mp.qc, ok[0], ok[1], H.R.keys[rk][2]});
           if (ti == th_idx.end()) continue;
+          if (o.ms * o.mt > st0[ti->second + 1] - st0[ti->second])
+            throw PlanError{TNX_ERR_RUNTIME, "internal: MPO output beyond its theta block"};
           ContractSpan g{};
           g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
           g.ar_str = static_cast<int32_t>(even(mp.md));
@@ -2131,34 +2230,37 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
           g.br_str = 1;
           g.bk_str = stride32(rd[1] * even(rd[2]));
           g.K = mp.md;
-          for (int32_t e = 0; e < o.ms * o.mt * o.mf; ++e) {
-            const int32_t slot = mp.out_slot0[k] + e, st = e / o.mf, f = e % o.mf;
+          for (int32_t e = 0; e < n_slots; ++e) {
+            const int32_t slot = slot0 + e, st = st0[ti->second] + e / o.mf, f = e % o.mf;
             if (tb[slot] == tb[slot + 1]) continue;
-            auto& dst = prod[ti->second].at(st);
-            if (dst.empty()) dst.reserve(32);
             const int64_t r = r0 + h->r_off[rk] + f * even(rd[2]);
+            auto add = [&](int64_t a_off, int64_t b_off) {
+              g.a_off = a_off;
+              g.b_off = b_off;
+              prod.push_back(g);
+              dest.push_back(st);
+              ++first[st + 1];
+            };
             if (formed[i][p][slot]) {
-              g.a_off = static_cast<int64_t>(x3_base / 8) + x3[i][p][slot];
-              g.b_off = r;
-              dst.push_back(g);
+              add(static_cast<int64_t>(x3_base / 8) + x3[i][p][slot], r);
               continue;
             }
             for (int32_t v = tb[slot]; v < tb[slot + 1]; ++v) {
-              if (wi[v] < 0) throw PlanError{TNX_ERR_RUNTIME, "internal: MPO weight without its R copy"};
-              g.a_off = static_cast<int64_t>(x1_base / 8) + x1[i][p][mp.terms[v].in_slot];
-              g.b_off = r + wi[v] * h->r_total;
-              dst.push_back(g);
+              if (copy[v] < 0) throw PlanError{TNX_ERR_RUNTIME, "internal: MPO weight without its R copy"};
+              add(static_cast<int64_t>(x1_base / 8) + x1[i][p][mp.terms[v].in_slot], r + copy[v] * h->r_total);
             }
           }
         }
       }
     }
+    for (size_t k = 0; k + 1 < first.size(); ++k) first[k + 1] += first[k];
+    s4[i].spans.resize(prod.size());
+    std::vector<int32_t> at(first.begin(), first.end() - 1);
+    for (size_t u = 0; u < prod.size(); ++u) s4[i].spans[at[dest[u]]++] = prod[u];
     for (size_t k = 0; k < H.th.keys.size(); ++k) {
       const auto& td = H.th.dims[k];
       if (td[0] == 0 || td[3] == 0) continue;
-      for (size_t st = 0; st < prod[k].size(); ++st) {
-        const size_t first = s4[i].spans.size();
-        s4[i].spans.insert(s4[i].spans.end(), prod[k][st].begin(), prod[k][st].end());
+      for (int32_t st = 0; st < st0[k + 1] - st0[k]; ++st) {
         ContractTile t{};
         t.out_off = H.th.offs[k] + static_cast<int64_t>(st) * td[3];
         t.M = static_cast<int32_t>(td[0]);
@@ -2168,7 +2270,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
         t.c_str = 1;
         t.out_slot = 1 + i;
         t.scale = h->out_scale;  // undoes the power-of-two scaling of L and R
-        s4[i].close(t, first);
+        s4[i].close(t, first[st0[k] + st], first[st0[k] + st + 1]);
       }
     }
   }

@@ -432,6 +432,43 @@ struct Shape {
 // blocks; 128 x 16: narrow column blocks (an MPO leg), whose rows are many
 constexpr Shape kShapes[kContractShapes] = {
     {64, 64, 2, 2, 3, 1.0}, {32, 32, 2, 2, 4, 0.87}, {128, 16, 4, 1, 3, 0.75}, {64, 32, 2, 2, 4, 0.95}};
+
+// What a step's blocks come to in one tile shape: clocks of all CTAs and of the
+// longest, output elements, CTAs, K tiles of the longest.  A template, because
+// a division by a tile extent is then a shift: it runs for every block of every
+// new operator.
+struct ShapeWork {
+  double sum = 0.0, work_max = 0.0, cells = 0.0;
+  int64_t n = 0, kmax = 0;
+};
+template <int S>
+ShapeWork shape_work(const std::vector<ContractBlk>& blks) {
+  constexpr uint32_t bm = kShapes[S].bm, bn = kShapes[S].bn, wm = kShapes[S].wm, wn = kShapes[S].wn;
+  ShapeWork w;
+  for (const ContractBlk& b : blks) {
+    w.kmax = std::max(w.kmax, b.ktiles);
+    const uint32_t M = static_cast<uint32_t>(b.M), N = static_cast<uint32_t>(b.N);
+    const int64_t fm = M / bm, fn = N / bn;  // full tiles, then the ragged edges
+    const uint32_t em = M % bm, en = N % bn;
+    auto add = [&](int64_t count, uint32_t r, uint32_t c) {
+      if (count <= 0 || r == 0 || c == 0) return;
+      const uint32_t fr = ((r + 7) / 8 + wm - 1) / wm, fc = ((c + 7) / 8 + wn - 1) / wn;
+      const double mma = 16.0 * static_cast<double>(fr * fc) * static_cast<double>(b.k4);
+      const double mem = static_cast<double>((r + c) * b.ktiles) * 16.0 * 8.0 / 48.0;
+      const double x = std::max(mma, mem);
+      w.sum += static_cast<double>(count) * x;
+      w.work_max = std::max(w.work_max, x);
+      w.cells += static_cast<double>(count * r * c);
+      w.n += count;
+    };
+    add(fm * fn, bm, bn);
+    add(fn, em, bn);
+    add(fm, bm, en);
+    add(em > 0 && en > 0 ? 1 : 0, em, en);
+  }
+  return w;
+}
+
 }  // namespace
 
 // Estimated clocks of a step for every tile shape and number of K shares (up
@@ -452,28 +489,9 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_spl
   *parts = min_split / *split;
   for (int s : {1, 3, 2, 0}) {  // the smallest tile of equal estimates
     const Shape& h = kShapes[s];
-    double sum = 0.0, work_max = 0.0, cells = 0.0;
-    int64_t n = 0, kmax = 0;
-    for (const ContractBlk& b : blks) {
-      kmax = std::max(kmax, b.ktiles);
-      const int64_t fm = b.M / h.bm, fn = b.N / h.bn;  // full tiles, then the ragged edges
-      const int64_t em = b.M % h.bm, en = b.N % h.bn;
-      auto add = [&](int64_t count, int64_t r, int64_t c) {
-        if (count <= 0 || r <= 0 || c <= 0) return;
-        const int64_t fr = ((r + 7) / 8 + h.wm - 1) / h.wm, fc = ((c + 7) / 8 + h.wn - 1) / h.wn;
-        const double mma = 16.0 * static_cast<double>(fr * fc) * static_cast<double>(b.k4);
-        const double mem = static_cast<double>((r + c) * b.ktiles) * 16.0 * 8.0 / 48.0;
-        const double x = std::max(mma, mem);
-        sum += static_cast<double>(count) * x;
-        work_max = std::max(work_max, x);
-        cells += static_cast<double>(count * r * c);
-        n += count;
-      };
-      add(fm * fn, h.bm, h.bn);
-      add(fn, em, h.bn);
-      add(fm, h.bm, en);
-      add(em > 0 && en > 0 ? 1 : 0, em, en);
-    }
+    const ShapeWork w = s == 0 ? shape_work<0>(blks) : s == 1 ? shape_work<1>(blks) : s == 2 ? shape_work<2>(blks) : shape_work<3>(blks);
+    const double sum = w.sum, work_max = w.work_max, cells = w.cells;
+    const int64_t n = w.n, kmax = w.kmax;
     if (n == 0) continue;
     const double cell = cells / static_cast<double>(n);
     for (int sp = min_split; sp <= max_split; sp *= 2) {
@@ -498,36 +516,47 @@ void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_spl
 
 int64_t contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks, int shape,
                        std::vector<uint8_t>& dst) {
-  const Shape& h = kShapes[shape];
+  const int bm = kShapes[shape].bm, bn = kShapes[shape].bn;
   // a block's tiles fall into four rectangles of one cost each (interior, last
-  // column, last row, corner): these are sorted, not the tiles
+  // column, last row, corner): these are sorted, not the tiles, into classes of
+  // costs within 1/32 of each other (binary exponent and five bits), longest
+  // first, in the blocks' order inside a class
   struct Rect {
-    int64_t cost, m0, m1, n0, n1;
-    size_t blk;
+    int32_t blk, m0, m1, n0, n1, cls;
   };
+  constexpr int kClasses = 64 * 32;
   std::vector<Rect> rects;
   rects.reserve(4 * proto.size());
+  std::vector<int32_t> first(kClasses + 1, 0);
   int64_t n = 0;
   for (size_t i = 0; i < proto.size(); ++i) {
-    const int64_t M = proto[i].M, N = proto[i].N, mf = M / h.bm * h.bm, nf = N / h.bn * h.bn;
-    auto add = [&](int64_t m0, int64_t m1, int64_t n0, int64_t n1) {
+    const int32_t M = proto[i].M, N = proto[i].N, mf = M & ~(bm - 1), nf = N & ~(bn - 1);
+    auto add = [&](int32_t m0, int32_t m1, int32_t n0, int32_t n1) {
       if (m0 >= m1 || n0 >= n1) return;
-      const int64_t fm = (std::min<int64_t>(h.bm, m1 - m0) + 7) / 8, fn = (std::min<int64_t>(h.bn, n1 - n0) + 7) / 8;
-      rects.push_back({blks[i].k4 * fm * fn, m0, m1, n0, n1, i});
-      n += ((m1 - m0 + h.bm - 1) / h.bm) * ((n1 - n0 + h.bn - 1) / h.bn);
+      const uint64_t fm = (std::min(bm, m1 - m0) + 7) / 8, fn = (std::min(bn, n1 - n0) + 7) / 8;
+      const uint64_t cost = static_cast<uint64_t>(blks[i].k4) * fm * fn;
+      const int e = cost ? 63 - __builtin_clzll(cost) : 0;
+      const int fine = static_cast<int>((e >= 5 ? cost >> (e - 5) : cost << (5 - e)) & 31);
+      rects.push_back({static_cast<int32_t>(i), m0, m1, n0, n1, kClasses - 1 - (e * 32 + fine)});
+      ++first[rects.back().cls + 1];
+      // M and N are below 2^31, so m1 - m0 + bm - 1 is not
+      n += ((static_cast<int64_t>(m1) - m0 + bm - 1) / bm) * ((static_cast<int64_t>(n1) - n0 + bn - 1) / bn);
     };
     add(0, mf, 0, nf);
     add(0, mf, nf, N);
     add(mf, M, 0, nf);
     add(mf, M, nf, N);
   }
-  std::stable_sort(rects.begin(), rects.end(), [](const Rect& a, const Rect& b) { return a.cost > b.cost; });
+  for (int c = 0; c < kClasses; ++c) first[c + 1] += first[c];
+  std::vector<int32_t> order(rects.size());
+  for (size_t r = 0; r < rects.size(); ++r) order[first[rects[r].cls]++] = static_cast<int32_t>(r);
   size_t at = dst.size();
   dst.resize(at + static_cast<size_t>(n) * sizeof(ContractTile));
-  for (const Rect& r : rects) {
+  for (int32_t o : order) {
+    const Rect& r = rects[o];
     ContractTile t = proto[r.blk];
-    for (int64_t m0 = r.m0; m0 < r.m1; m0 += h.bm)
-      for (int64_t n0 = r.n0; n0 < r.n1; n0 += h.bn) {
+    for (int64_t m0 = r.m0; m0 < r.m1; m0 += bm)
+      for (int64_t n0 = r.n0; n0 < r.n1; n0 += bn) {
         t.m0 = static_cast<int32_t>(m0);
         t.n0 = static_cast<int32_t>(n0);
         std::memcpy(dst.data() + at, &t, sizeof(t));
