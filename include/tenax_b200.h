@@ -127,7 +127,8 @@ int tnx_plan_output(const tnx_plan* plan, int64_t* n_blocks, int32_t* keys, int6
                     int32_t* has_target, int64_t* target);
 int tnx_plan_workspace(const tnx_plan* plan, int32_t precision, size_t* bytes);
 double tnx_plan_flops(const tnx_plan* plan);
-/* Execute on device FP64 data: inputs[i] are the operands' block buffers. */
+/* Execute on device FP64 data: inputs[i] are the operands' block buffers.
+ * `out` may overlap an input (which it then overwrites). */
 int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, int32_t precision, void* workspace,
                      size_t workspace_bytes, void* stream);
 void tnx_plan_destroy(tnx_plan* plan);

@@ -92,6 +92,28 @@ struct DevMem {
   }
 };
 
+// Scratch of one call on its own stream: allocated and freed in stream order.
+struct StreamMem {
+  cudaStream_t st;
+  void* p = nullptr;
+  explicit StreamMem(cudaStream_t s) : st(s) {}
+  StreamMem(const StreamMem&) = delete;
+  StreamMem& operator=(const StreamMem&) = delete;
+  ~StreamMem() {
+    if (p) cudaFreeAsync(p, st);
+  }
+  void* alloc(size_t bytes) {
+    CUDA_OK(cudaMallocAsync(&p, bytes, st));
+    return p;
+  }
+};
+
+// whether two buffers of n and m doubles share memory
+bool overlap(const double* x, int64_t n, const double* y, int64_t m) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+  return a < b + static_cast<uintptr_t>(m) * 8 && b < a + static_cast<uintptr_t>(n) * 8;
+}
+
 template <class T>
 void upload(DevMem& m, const std::vector<T>& v, cudaStream_t st = nullptr) {
   m.alloc(v.size() * sizeof(T));
@@ -1002,17 +1024,25 @@ int tnx_plan_execute(tnx_plan* plan, const double* const* inputs, double* out, i
       const double* a_ptr = plan->a_src[s] >= 0 ? inputs[plan->a_src[s]] : plan->inter[s - 1]->as<double>();
       const double* b_ptr = plan->has_scalar ? plan->scalar_one.as<double>() : inputs[plan->b_src[s]];
       double* o_ptr = (s + 1 == plan->steps.size()) ? out : plan->inter[s]->as<double>();
-      if (d.direct) {
-        ContractLaunch L = d.dl;
-        L.a = d.swapped ? b_ptr : a_ptr;
-        L.b = d.swapped ? a_ptr : b_ptr;
-        L.c = o_ptr;
-        CUDA_OK(launch_contract_f64(L, st));
-        continue;
-      }
-      if (d.copy) {
-        launch_strided_copy(a_ptr, o_ptr, d.scat.as<DevCopySeg>(), d.chunksS.as<DevChunk>(), d.n_copy, st);
-        CUDA_OK(cudaGetLastError());
+      if (d.direct || d.copy) {
+        // both read their operands while they write: a result that overlaps an
+        // operand of its step is formed beside it and copied
+        const int64_t total = plan->steps[s].out.total;
+        StreamMem aside(st);
+        if (o_ptr == out && ((plan->a_src[s] >= 0 && overlap(out, total, a_ptr, plan->ins[plan->a_src[s]].total)) ||
+                             (!plan->has_scalar && overlap(out, total, b_ptr, plan->ins[plan->b_src[s]].total))))
+          o_ptr = static_cast<double*>(aside.alloc(total * sizeof(double)));
+        if (d.direct) {
+          ContractLaunch L = d.dl;
+          L.a = d.swapped ? b_ptr : a_ptr;
+          L.b = d.swapped ? a_ptr : b_ptr;
+          L.c = o_ptr;
+          CUDA_OK(launch_contract_f64(L, st));
+        } else {
+          launch_strided_copy(a_ptr, o_ptr, d.scat.as<DevCopySeg>(), d.chunksS.as<DevChunk>(), d.n_copy, st);
+          CUDA_OK(cudaGetLastError());
+        }
+        if (aside.p) CUDA_OK(cudaMemcpyAsync(out, aside.p, total * sizeof(double), cudaMemcpyDeviceToDevice, st));
         continue;
       }
       // three launches: the images' padding was cleared with the plan, and the
