@@ -620,44 +620,6 @@ int tnx_plan_workspace(const tnx_plan* plan, int32_t precision, size_t* bytes) {
 }
 
 namespace {
-// Offset tables of one step's axes: an axis of legs (extent, stride), outermost
-// first, is affine where the legs merge into one stride, and otherwise a table
-// shared by every axis of the same legs.
-struct AxisTabs {
-  std::vector<int32_t> tab;
-  std::map<std::vector<std::pair<int64_t, int64_t>>, int32_t> seen;
-  void add(const std::vector<std::pair<int64_t, int64_t>>& legs, int32_t* t, int32_t* str) {
-    std::vector<std::pair<int64_t, int64_t>> m;
-    for (const auto& l : legs) {
-      if (l.first == 1) continue;
-      if (!m.empty() && m.back().second == l.first * l.second)
-        m.back() = {m.back().first * l.first, l.second};
-      else
-        m.push_back(l);
-    }
-    *t = -1;
-    *str = m.empty() ? 0 : static_cast<int32_t>(m[0].second);
-    if (m.size() < 2) return;
-    *str = static_cast<int32_t>(m.back().second);
-    auto it = seen.find(m);
-    if (it == seen.end()) {
-      it = seen.emplace(m, static_cast<int32_t>(tab.size())).first;
-      int64_t n = 1;
-      for (const auto& l : m) n *= l.first;
-      if (static_cast<int64_t>(tab.size()) + n > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "axis tables too large"};
-      for (int64_t i = 0; i < n; ++i) {
-        int64_t rem = i, off = 0;
-        for (size_t l = m.size(); l-- > 0;) {
-          off += (rem % m[l].first) * m[l].second;
-          rem /= m[l].first;
-        }
-        tab.push_back(static_cast<int32_t>(off));
-      }
-    }
-    *t = it->second;
-  }
-};
-
 // The legs with a nonzero stride in `order` (the planner's row, K or column
 // flattening), outermost first, with their strides inside the row-major block.
 std::vector<std::pair<int64_t, int64_t>> axis_legs(int nlegs, const int32_t* dims, const int32_t* order) {
@@ -717,10 +679,11 @@ bool pairs_ok(int64_t off, const std::vector<std::pair<int64_t, int64_t>>& fast,
 }
 
 // Tables of the one-launch FP64 kernel for one step.  It serves every step
-// whose blocks hold fewer than 2^31 elements (its in-block offsets are 32-bit)
-// and carry no fermionic sign; the others keep the packed path, which negates
-// on the way in and out.  Measured, packed against one launch: theta of
-// chi = 64 24 -> 3 us of device time, a CTM step's 196 products 33 -> 6 ms.
+// whose blocks hold fewer than 2^31 elements (its in-block offsets are 32-bit),
+// whose axis tables fit their limit and whose blocks carry no fermionic sign; the
+// others keep the packed path, which negates on the way in and out.  Measured,
+// packed against one launch: theta of chi = 64 24 -> 3 us of device time, a CTM
+// step's 196 products 33 -> 6 ms.
 bool build_direct(const PairPlan& P, StepDev& d) {
   constexpr int64_t kMaxBlock = int64_t{1} << 31;
   for (const auto* v : {&P.packA, &P.packB})
@@ -762,6 +725,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     }
     return legs;
   };
+  bool fits = true;  // the axis tables
   auto index = [&](const std::vector<PackSeg>& segs, const std::string& subs, bool kfast, bool* vec) {
     *vec = true;
     std::map<std::pair<int32_t, int32_t>, std::map<int32_t, Side>> by;  // (group, row0) -> k0 -> block
@@ -771,8 +735,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
       x.off = s.src_off;
       x.rows = extent_of(r);
       x.k = extent_of(k);
-      T.add(r, &x.rt, &x.rs);
-      T.add(k, &x.kt, &x.ks);
+      fits = fits && T.add(r, &x.rt, &x.rs) && T.add(k, &x.kt, &x.ks);
       *vec = *vec && pairs_ok(s.src_off, kfast ? k : r, kfast ? r : k);
       by[{s.group, s.row0}][s.k0] = x;
     }
@@ -780,6 +743,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
   };
   bool a_vec = false, b_vec = false;
   const auto A = index(P.packA, P.a_subs, a_kfast, &a_vec), B = index(P.packB, P.b_subs, b_kfast, &b_vec);
+  if (!fits) return false;
   // rows are the longer side of a tile (128 x 16)
   int64_t sm = 0, sn = 0;
   for (const auto& sc : P.scatter) {
@@ -799,8 +763,7 @@ bool build_direct(const PairPlan& P, StepDev& d) {
     t.out_off = sc.dst_off;
     t.M = static_cast<int32_t>(extent_of(r));
     t.N = static_cast<int32_t>(extent_of(c));
-    T.add(r, &t.r_tab, &t.r_str);
-    T.add(c, &t.c_tab, &t.c_str);
+    if (!T.add(r, &t.r_tab, &t.r_str) || !T.add(c, &t.c_tab, &t.c_str)) return false;
     t.span0 = static_cast<int32_t>(spans.size());
     auto ia = A.find({sc.group, sc.row0});
     auto ib = B.find({sc.group, sc.col0});

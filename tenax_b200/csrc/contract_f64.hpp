@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <utility>
 #include <vector>
 
 namespace tnx {
@@ -28,6 +30,49 @@ struct ContractTile {
   double scale;      // the result's factor
 };
 static_assert(sizeof(ContractTile) == 64, "one record a tile");
+
+// Offset tables of one step's axes: an axis of legs (extent, stride), outermost
+// first, is affine where the legs merge into one stride, and otherwise a table
+// shared by every axis of the same legs.
+struct AxisTabs {
+  // entries of all tables (they are indexed by int32_t); a step that needs more
+  // takes the packed path, whose tables do not grow with the extents
+  int64_t limit = INT32_MAX;
+  std::vector<int32_t> tab;
+  std::map<std::vector<std::pair<int64_t, int64_t>>, int32_t> seen;
+  // false, with nothing filled: beyond the limit
+  bool add(const std::vector<std::pair<int64_t, int64_t>>& legs, int32_t* t, int32_t* str) {
+    std::vector<std::pair<int64_t, int64_t>> m;
+    for (const auto& l : legs) {
+      if (l.first == 1) continue;
+      if (!m.empty() && m.back().second == l.first * l.second)
+        m.back() = {m.back().first * l.first, l.second};
+      else
+        m.push_back(l);
+    }
+    *t = -1;
+    *str = m.empty() ? 0 : static_cast<int32_t>(m[0].second);
+    if (m.size() < 2) return true;
+    *str = static_cast<int32_t>(m.back().second);
+    auto it = seen.find(m);
+    if (it == seen.end()) {
+      int64_t n = 1;
+      for (const auto& l : m) n *= l.first;
+      if (static_cast<int64_t>(tab.size()) + n > limit) return false;
+      it = seen.emplace(m, static_cast<int32_t>(tab.size())).first;
+      const size_t first = tab.size();
+      tab.resize(first + static_cast<size_t>(n));
+      // the innermost leg, then that pattern shifted by each outer leg in turn
+      int64_t len = 1;
+      for (size_t l = m.size(); n > 0 && l-- > 0; len *= m[l].first)
+        for (int64_t k = 1; k < m[l].first; ++k)
+          for (int64_t i = 0; i < len; ++i)
+            tab[first + k * len + i] = tab[first + i] + static_cast<int32_t>(k * m[l].second);
+    }
+    *t = it->second;
+    return true;
+  }
+};
 
 // an output block as the choice of tile shape sees it
 struct ContractBlk {
