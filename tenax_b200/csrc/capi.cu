@@ -1043,6 +1043,7 @@ int tnx_fuse_plan_create(const tnx_tensor_desc* in, int32_t modulus, int32_t axi
     TensorStruct T = parse_desc(in, in->subs ? nullptr : subs.c_str());
     auto p = std::make_unique<tnx_fuse_plan>();
     p->F = plan_fuse(T, axis_a, axis_b, fused_flow, modulus);
+    for (const CopySeg& c : p->F.segs) p->covered += c.count;
     *out = p.release();
     return TNX_OK;
   })
@@ -1082,7 +1083,6 @@ int tnx_fuse_execute(tnx_fuse_plan* p, const double* in, double* out, void* stre
         }
         const int id = static_cast<int>(segs.size());
         segs.push_back(d);
-        p->covered += c.count;
         for (int64_t s = 0; s < c.count; s += 2048) chunks.push_back({id, 0, s, std::min<int64_t>(2048, c.count - s)});
       }
       upload(p->segs, segs);
