@@ -1991,7 +1991,9 @@ std::vector<ContractLaunch> f64_launches(const std::vector<F64Stage>& ops, bool 
     h.resize(std::max<size_t>(64, h.size()));
     L.a_kfast = a_kfast;
     L.b_kfast = false;
-    L.a_vec = true;  // padded copies and slots; bases are null, offsets absolute
+    // padded copies and slots, whose bases are null and offsets absolute; a
+    // product cut inside its K may start on an odd element
+    L.a_vec = std::all_of(g->spans.begin(), g->spans.end(), [](const ContractSpan& u) { return u.a_off % 2 == 0; });
     L.b_vec = b_vec;
     blobs.push_back(std::make_unique<DevMem>());
     upload(*blobs.back(), h);
@@ -2002,10 +2004,21 @@ std::vector<ContractLaunch> f64_launches(const std::vector<F64Stage>& ops, bool 
   return out;
 }
 
-int32_t stride32(int64_t s) {
-  // in-tile offsets (up to 128 rows) are formed in 32 bits
-  if (s >= (int64_t{1} << 24)) throw PlanError{TNX_ERR_UNSUPPORTED, "H_eff block stride exceeds 2^24 elements"};
-  return static_cast<int32_t>(s);
+// One product as spans: `g` whole, or in parts where a K stride (in elements:
+// ak, bk) is too long for the kernel's tiles.
+template <class F>
+void f64_spans(ContractSpan g, int64_t ak, int64_t bk, F add) {
+  const int64_t K = g.K, step = span_k(K, std::max(ak, bk));
+  // a stride beyond 32 bits comes with steps of one, which do not use it
+  g.ak_str = static_cast<int32_t>(std::min<int64_t>(ak, INT32_MAX));
+  g.bk_str = static_cast<int32_t>(std::min<int64_t>(bk, INT32_MAX));
+  for (int64_t k = 0; k < K; k += step) {
+    ContractSpan u = g;
+    u.a_off += k * ak;
+    u.b_off += k * bk;
+    u.K = static_cast<int32_t>(std::min(step, K - k));
+    add(u);
+  }
 }
 
 // FP64 tables.  X1 slots (b, p, q) of every MPO pair are c x d matrices; slots
@@ -2132,12 +2145,11 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
               g.b_off = t.src_off + static_cast<int64_t>(pq) * mp.md;
               g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
               g.ar_str = 1;
-              g.ak_str = stride32(l.dims[1] * even(l.dims[2]));
               g.br_str = 1;
-              g.bk_str = stride32(static_cast<int64_t>(t.dims[1]) * t.dims[2] * t.dims[3]);
               g.K = l.dims[0];
               g.b_slot = i;
-              s1[i].spans.push_back(g);
+              f64_spans(g, l.dims[1] * even(l.dims[2]), static_cast<int64_t>(t.dims[1]) * t.dims[2] * t.dims[3],
+                        [&](const ContractSpan& u) { s1[i].spans.push_back(u); });
             }
             ContractTile t{};
             t.out_off = static_cast<int64_t>(x1_base / 8) + at(b0);
@@ -2219,9 +2231,7 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
           ContractSpan g{};
           g.ar_tab = g.ak_tab = g.br_tab = g.bk_tab = -1;
           g.ar_str = static_cast<int32_t>(even(mp.md));
-          g.ak_str = 1;
           g.br_str = 1;
-          g.bk_str = stride32(rd[1] * even(rd[2]));
           g.K = mp.md;
           for (int32_t e = 0; e < n_slots; ++e) {
             const int32_t slot = slot0 + e, st = st0[ti->second] + e / o.mf, f = e % o.mf;
@@ -2230,9 +2240,11 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
             auto add = [&](int64_t a_off, int64_t b_off) {
               g.a_off = a_off;
               g.b_off = b_off;
-              prod.push_back(g);
-              dest.push_back(st);
-              ++first[st + 1];
+              f64_spans(g, 1, rd[1] * even(rd[2]), [&](const ContractSpan& u) {
+                prod.push_back(u);
+                dest.push_back(st);
+                ++first[st + 1];
+              });
             };
             if (formed[i][p][slot]) {
               add(static_cast<int64_t>(x3_base / 8) + x3[i][p][slot], r);
@@ -2253,17 +2265,35 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
     for (size_t k = 0; k < H.th.keys.size(); ++k) {
       const auto& td = H.th.dims[k];
       if (td[0] == 0 || td[3] == 0) continue;
+      const int64_t row = td[1] * td[2] * td[3];
+      if (row > INT32_MAX) throw PlanError{TNX_ERR_UNSUPPORTED, "a theta block's row has more than 2^31 elements"};
       for (int32_t st = 0; st < st0[k + 1] - st0[k]; ++st) {
         ContractTile t{};
         t.out_off = H.th.offs[k] + static_cast<int64_t>(st) * td[3];
-        t.M = static_cast<int32_t>(td[0]);
         t.N = static_cast<int32_t>(td[3]);
         t.r_tab = t.c_tab = -1;
-        t.r_str = stride32(td[1] * td[2] * td[3]);
+        t.r_str = static_cast<int32_t>(row);
         t.c_str = 1;
         t.out_slot = 1 + i;
         t.scale = h->out_scale;  // undoes the power-of-two scaling of L and R
-        s4[i].close(t, first[st0[k] + st], first[st0[k] + st + 1]);
+        const size_t u0 = first[st0[k] + st], u1 = first[st0[k] + st + 1];
+        int64_t a_row = 0;  // the longest row stride among the products
+        for (size_t u = u0; u < u1; ++u) a_row = std::max<int64_t>(a_row, s4[i].spans[u].ar_str);
+        const int64_t rows = matrix_rows(td[0], a_row);
+        t.M = static_cast<int32_t>(std::min(rows, td[0]));
+        s4[i].close(t, u0, u1);
+        for (int64_t m = rows; m < td[0]; m += rows) {  // the rest, with the same products further down
+          const size_t v0 = s4[i].spans.size();
+          for (size_t u = u0; u < u1; ++u) {
+            ContractSpan g = s4[i].spans[u];
+            g.a_off += m * g.ar_str;
+            s4[i].spans.push_back(g);
+          }
+          ContractTile r = t;
+          r.out_off += m * row;
+          r.M = static_cast<int32_t>(std::min(rows, td[0] - m));
+          s4[i].close(r, v0, s4[i].spans.size());
+        }
       }
     }
   }

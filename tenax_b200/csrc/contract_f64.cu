@@ -432,6 +432,7 @@ struct Shape {
 // blocks; 128 x 16: narrow column blocks (an MPO leg), whose rows are many
 constexpr Shape kShapes[kContractShapes] = {
     {64, 64, 2, 2, 3, 1.0}, {32, 32, 2, 2, 4, 0.87}, {128, 16, 4, 1, 3, 0.75}, {64, 32, 2, 2, 4, 0.95}};
+static_assert(BK == kTileK && kShapes[2].bm == kTileRows, "the 32-bit offsets of a tile");
 
 // What a step's blocks come to in one tile shape: clocks of all CTAs and of the
 // longest, output elements, CTAs, K tiles of the longest.  A template, because

@@ -74,6 +74,18 @@ struct AxisTabs {
   }
 };
 
+// The kernel forms the offsets inside a tile, up to 16 K steps and 128 rows, in
+// 32 bits.  Blocks of fewer than 2^31 elements cannot leave that range; for
+// larger ones these are the K steps a span and the rows an output matrix may
+// have, given the longest stride of either.
+constexpr int64_t kTileK = 16, kTileRows = 128;
+inline int64_t span_k(int64_t K, int64_t stride) {
+  return (kTileK - 1) * stride <= INT32_MAX ? K : INT32_MAX / stride + 1;
+}
+inline int64_t matrix_rows(int64_t M, int64_t stride) {
+  return (kTileRows - 1) * stride <= INT32_MAX ? M : INT32_MAX / stride + 1;
+}
+
 // an output block as the choice of tile shape sees it
 struct ContractBlk {
   int64_t M, N, ktiles, k4;  // k4: 4-deep K steps of all pairs

@@ -50,11 +50,34 @@ int main() {
 """
 
 
+# the longest K span and the most rows whose offsets inside a tile fit 32 bits
+LIMITS = r"""
+#include "contract_f64.hpp"
+static int64_t most(int64_t deep, int64_t stride) {  // steps of `stride` from 0 that end below 2^31, at most `deep`
+  int64_t n = 1;
+  while (n < deep && n * stride <= INT32_MAX) ++n;
+  return n;
+}
+int main() {
+  int bad = 0;
+  for (int64_t s : {int64_t{0}, int64_t{1}, int64_t{1} << 24, int64_t{INT32_MAX} / 127, int64_t{INT32_MAX} / 127 + 1,
+                    int64_t{INT32_MAX} / 15, int64_t{INT32_MAX} / 15 + 1, int64_t{1} << 30, int64_t{INT32_MAX},
+                    int64_t{INT32_MAX} + 1, int64_t{1} << 40}) {
+    const int64_t k = tnx::span_k(5000, s), m = tnx::matrix_rows(5000, s);
+    bad += k != (most(16, s) == 16 ? 5000 : most(16, s));
+    bad += m != (most(128, s) == 128 ? 5000 : most(128, s));
+  }
+  return bad;
+}
+"""
+
+
 @pytest.mark.skipif(not shutil.which("g++") or not os.path.isdir(os.path.join(CUDA, "include")),
                     reason="needs g++ and the CUDA headers")
-def test_axis_tables(tmp_path):
+@pytest.mark.parametrize("code", [CHECK, LIMITS], ids=["tables", "limits"])
+def test_axis_tables(tmp_path, code):
     src, exe = tmp_path / "check.cpp", tmp_path / "check"
-    src.write_text(CHECK)
+    src.write_text(code)
     subprocess.run(["g++", "-std=c++17", "-O1", f"-I{os.path.join(ROOT, 'tenax_b200', 'csrc')}",
                     f"-I{os.path.join(CUDA, 'include')}", str(src), "-o", str(exe)], check=True)
     assert subprocess.run([str(exe)], timeout=60).returncode == 0

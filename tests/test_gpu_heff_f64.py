@@ -92,3 +92,33 @@ def test_extreme_ranges_of_the_environments():
     R = SymmetricTensor.from_flat(p.R.indices, p.R.keys, p.R.data * sc)
     op2 = tb.HeffOperator(L, p.Wl, p.Wr, R, p.theta.indices, p.theta.keys, "fp64")
     assert torch.equal(op2.apply(x), y)
+
+
+def test_long_block_strides():
+    """theta[a, p, q, d] of 32 x 32 x 16384: its K stride is 2^24 elements, which
+    in-tile offsets of 128 rows would not reach.  W_l W_r is the identity, so
+    the result is L . theta . R; each of the two sums rounds within
+    (K + 2) u of the sum of its magnitudes."""
+    u1 = tb.U1Symmetry()
+    IN, OUT = tb.FlowDirection.IN, tb.FlowDirection.OUT
+    a, p, d = 2, 32, 16384
+
+    def leg(n, flow, label):
+        return tb.TensorIndex(u1, np.zeros(n, np.int32), flow, label)
+
+    def tensor(*legs, data):
+        return SymmetricTensor.from_flat(legs, [(0,) * len(legs)], data)
+
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda n: torch.randn(n, generator=g, dtype=torch.float64, device="cuda")  # noqa: E731
+    eye = torch.eye(p, dtype=torch.float64, device="cuda").reshape(-1)
+    L = tensor(leg(a, OUT, "a"), leg(1, IN, "b"), leg(a, IN, "c"), data=rnd(a * a))
+    th = tensor(leg(a, IN, "a"), leg(p, IN, "p"), leg(p, IN, "q"), leg(d, OUT, "d"), data=rnd(a * p * p * d))
+    W = [tensor(leg(1, OUT, "l"), leg(p, OUT, "i"), leg(p, IN, "o"), leg(1, IN, "r"), data=eye.clone()) for _ in range(2)]
+    R = tensor(leg(d, IN, "d"), leg(1, OUT, "f"), leg(d, OUT, "g"), data=rnd(d * d))
+    op = tb.HeffOperator(L, W[0], W[1], R, th.indices, th.keys, "fp64")
+    got = op.apply(th.data).view(a, p * p, d)
+    Lm, Rm, t = L.data.view(a, a), R.data.view(d, d), th.data.view(a, p * p * d)
+    ref = ((Lm.T @ t).view(a * p * p, d) @ Rm).view(a, p * p, d)
+    mag = ((Lm.abs().T @ t.abs()).view(a * p * p, d) @ Rm.abs()).view(a, p * p, d)
+    assert bool(((got - ref).abs() <= 2.0 * (a + d + 4) * 2.0 ** -53 * mag).all())
