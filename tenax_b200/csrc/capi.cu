@@ -2275,8 +2275,10 @@ void heff_batch_build_f64(tnx_heff_batch* b) {
         t.r_str = static_cast<int32_t>(row);
         t.c_str = 1;
         t.out_slot = 1 + i;
-        t.scale = h->out_scale;  // undoes the power-of-two scaling of L and R
         const size_t u0 = first[st0[k] + st], u1 = first[st0[k] + st + 1];
+        // undoes the power-of-two scaling of L and R; blocks that no product
+        // reaches are zero also where that overflows (0 * inf)
+        t.scale = u0 < u1 ? h->out_scale : 1.0;
         int64_t a_row = 0;  // the longest row stride among the products
         for (size_t u = u0; u < u1; ++u) a_row = std::max<int64_t>(a_row, s4[i].spans[u].ar_str);
         const int64_t rows = matrix_rows(td[0], a_row);

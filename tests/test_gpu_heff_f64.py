@@ -16,7 +16,7 @@ if not torch.cuda.is_available():  # pragma: no cover
 
 import tenax_b200 as tb  # noqa: E402
 from tenax_b200.auto_mpo import build_auto_mpo_sites, to_symmetric  # noqa: E402
-from tenax_b200.tensor import SymmetricTensor, embed_in_keys  # noqa: E402
+from tenax_b200.tensor import SymmetricTensor, embed_in_keys, restrict_to_keys  # noqa: E402
 from tenax_b200.workloads import chain_bulk_w, cylinder_bulk_w, make_heff_problem  # noqa: E402
 
 
@@ -122,3 +122,19 @@ def test_long_block_strides():
     ref = ((Lm.T @ t).view(a * p * p, d) @ Rm).view(a, p * p, d)
     mag = ((Lm.abs().T @ t.abs()).view(a * p * p, d) @ Rm.abs()).view(a, p * p, d)
     assert bool(((got - ref).abs() <= 2.0 * (a + d + 4) * 2.0 ** -53 * mag).all())
+
+
+def test_unreached_blocks_are_zero_when_the_scale_overflows():
+    """L and R near 2^600: the factor that undoes their scaling is infinite, and
+    theta blocks that no product reaches are still cleared."""
+    p, op = _op("chain", 40, 6, n_sectors=6, hi=12, lo=1)
+    x = embed_in_keys(p.theta, op.keys)
+    qc = sorted({k[2] for k in p.L.keys})[2]
+    keys = [k for k in p.L.keys if k[2] != qc]
+    L = SymmetricTensor.from_flat(p.L.indices, keys, restrict_to_keys(p.L, keys).data * 2.0 ** 600)
+    R = SymmetricTensor.from_flat(p.R.indices, p.R.keys, p.R.data * 2.0 ** 600)
+    op2 = tb.HeffOperator(L, p.Wl, p.Wr, R, p.theta.indices, op.keys, "fp64")
+    out = op2.apply(embed_in_keys(x, op2.keys).data, torch.full((op2.size,), 7.0, dtype=torch.float64, device="cuda"))
+    got = SymmetricTensor.from_flat(p.theta.indices, op2.keys, out).numpy_blocks()
+    unreached = [k for k in got if k[0] == qc]
+    assert unreached and all(np.array_equal(got[k], np.zeros_like(got[k])) for k in unreached)
