@@ -1584,9 +1584,12 @@ int64_t even(int64_t n) { return (n + 1) / 2 * 2; }
 
 // The FP64 copies of an environment T: blocks with their last leg padded to an
 // even extent (zeros), so that the products read it by 16 bytes; one copy per
-// scale, `total` elements each.  Returns once the copies are made.
-void padded_copies(const TensorStruct& T, const double* src, const double* scale, int nscale, DevMem& dst,
-                   std::vector<int64_t>& off, int64_t* total, cudaStream_t st) {
+// weight, `total` elements each.  An element is scaled by `unit` first, a power
+// of two: unit * weight may be out of range where the element's share is not.
+// Returns once the copies are made.
+void padded_copies(const TensorStruct& T, const double* src, double unit, const std::vector<double>& weight,
+                   DevMem& dst, std::vector<int64_t>& off, int64_t* total, cudaStream_t st) {
+  const int copies = static_cast<int>(weight.size());
   std::vector<DevPadSeg> segs;
   std::vector<DevChunk> chunks;
   off.clear();
@@ -1601,13 +1604,13 @@ void padded_copies(const TensorStruct& T, const double* src, const double* scale
     segs.push_back({T.offs[k], off.back(), static_cast<int32_t>(d[2]), static_cast<int32_t>(even(d[2]))});
     for (int64_t e = 0; e < n; e += 4096) chunks.push_back({id, 0, e, std::min<int64_t>(4096, n - e)});
   }
-  dst.alloc(std::max<int64_t>(2, *total) * sizeof(double) * nscale);
+  dst.alloc(std::max<int64_t>(2, *total) * sizeof(double) * copies);
   CUDA_OK(cudaMemsetAsync(dst.p, 0, dst.n, st));
   DevMem ds, dc;
   upload(ds, segs, st);
   upload(dc, chunks, st);
   launch_padded_copies(src, dst.as<double>(), ds.as<DevPadSeg>(), dc.as<DevChunk>(), static_cast<int>(chunks.size()),
-                       *total, scale, nscale, st);
+                       *total, unit, weight.data(), copies, st);
   CUDA_OK(cudaGetLastError());
   CUDA_OK(cudaStreamSynchronize(st));
 }
@@ -1765,12 +1768,8 @@ int tnx_heff_set_operators(tnx_heff* h, const double* L, const double* Wl, const
     h->out_scale = sL * sR;
     if (mode == IMG_F64) {
       choose_f64_weights(h);
-      const int nw = static_cast<int>(h->weights.size());
-      std::vector<double> rs(nw);
-      for (int j = 0; j < nw; ++j) rs[j] = h->weights[j] / sR;
-      const double ls = 1.0 / sL;
-      padded_copies(H.L, L, &ls, 1, h->l_img, h->l_off, &h->l_total, st);
-      padded_copies(H.R, R, rs.data(), nw, h->r_img, h->r_off, &h->r_total, st);
+      padded_copies(H.L, L, 1.0 / sL, {1.0}, h->l_img, h->l_off, &h->l_total, st);
+      padded_copies(H.R, R, 1.0 / sR, h->weights, h->r_img, h->r_off, &h->r_total, st);
       h->lp_img.alloc(0);
       h->prec = precision;
       return TNX_OK;

@@ -341,23 +341,23 @@ struct Scales {
 };
 __global__ void padded_copies_kernel(const double* __restrict__ src, double* __restrict__ dst,
                                      const DevPadSeg* __restrict__ segs, const DevChunk* __restrict__ chunks,
-                                     int64_t stride, Scales sc, int nscale) {
+                                     int64_t stride, double unit, Scales sc, int nscale) {
   const DevChunk ch = chunks[blockIdx.x];
   const DevPadSeg s = segs[ch.seg];
   for (int64_t e = ch.start + threadIdx.x; e < ch.start + ch.count; e += blockDim.x) {
     const int64_t row = e / s.inner;
-    const double v = src[s.src_off + e];
+    const double v = src[s.src_off + e] * unit;
     double* d = dst + s.dst_off + row * s.pitch + (e - row * s.inner);
     for (int j = 0; j < nscale; ++j) d[j * stride] = v * sc.s[j];
   }
 }
 
 void launch_padded_copies(const double* src, double* dst, const DevPadSeg* segs, const DevChunk* chunks, int n_chunks,
-                          int64_t stride, const double* scale, int nscale, cudaStream_t st) {
+                          int64_t stride, double unit, const double* scale, int nscale, cudaStream_t st) {
   if (n_chunks <= 0 || nscale <= 0) return;
   Scales sc{};
   for (int j = 0; j < nscale && j < kMaxScales; ++j) sc.s[j] = scale[j];
-  padded_copies_kernel<<<n_chunks, 256, 0, st>>>(src, dst, segs, chunks, stride, sc, nscale);
+  padded_copies_kernel<<<n_chunks, 256, 0, st>>>(src, dst, segs, chunks, stride, unit, sc, nscale);
 }
 
 // ---------------------------------------------------------------------------

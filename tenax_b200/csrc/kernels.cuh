@@ -66,14 +66,14 @@ void launch_mpo_apply(int mode, const DevMpoPair* pairs, const DevMpoSlot* islot
 void launch_mpo_sum(const DevMpoPair* pairs, const DevMpoSlot* islots, const DevMpoSlot* oslots,
                     const DevMpoTerm* terms, const int2* chunks, int n_chunks, const int32_t* skip, cudaStream_t st);
 int mpo_points_per_cta();
-// blocks as rows of `inner` elements -> rows of `pitch`, nscale copies each times its scale, copy j at j * stride
+// blocks as rows of `inner` elements -> rows of `pitch`, nscale copies, times unit and then each its scale, copy j at j * stride
 constexpr int kMaxScales = 8;
 struct DevPadSeg {
   int64_t src_off, dst_off;
   int32_t inner, pitch;
 };
 void launch_padded_copies(const double* src, double* dst, const DevPadSeg* segs, const DevChunk* chunks, int n_chunks,
-                          int64_t stride, const double* scale, int nscale, cudaStream_t st);
+                          int64_t stride, double unit, const double* scale, int nscale, cudaStream_t st);
 // dst[seg.dst_off + sum idx_l dstr_l] = src[seg.src_off + e] for each chunk's range of elements e
 void launch_strided_copy(const double* src, double* dst, const DevCopySeg* segs, const DevChunk* chunks, int n_chunks,
                          cudaStream_t st);

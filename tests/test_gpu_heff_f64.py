@@ -138,3 +138,21 @@ def test_unreached_blocks_are_zero_when_the_scale_overflows():
     got = SymmetricTensor.from_flat(p.theta.indices, op2.keys, out).numpy_blocks()
     unreached = [k for k in got if k[0] == qc]
     assert unreached and all(np.array_equal(got[k], np.zeros_like(got[k])) for k in unreached)
+
+
+def test_large_weights_with_a_tiny_environment():
+    """|R| in [2^-1021, 2^-1020) and W_l W_r weights above 2^5: R's share is
+    scaled up before a weight multiplies it (2^1021 times the weight is out of
+    range).  All factors are powers of two, so the bits are those of R near 1."""
+    Wl, Wr = chain_bulk_w()
+    Wl = SymmetricTensor.from_flat(Wl.indices, Wl.keys, Wl.data * 64.0)
+    p = make_heff_problem(40, 40, Wl, Wr, np.random.default_rng(7), n_sectors=6, hi=12, lo=1)
+    r = torch.sign(p.R.data) * (1.0 + p.R.data.abs().frac())
+    ops = []
+    for sL, sR in ((1.0, 1.0), (2.0 ** 600, 2.0 ** -1021)):
+        L = SymmetricTensor.from_flat(p.L.indices, p.L.keys, p.L.data * sL)
+        R = SymmetricTensor.from_flat(p.R.indices, p.R.keys, r * sR)
+        ops.append(tb.HeffOperator(L, Wl, Wr, R, p.theta.indices, p.theta.keys, "fp64"))
+    x = embed_in_keys(p.theta, ops[0].keys).data
+    y, tiny = (op.apply(x) for op in ops)
+    assert bool(torch.isfinite(y).all()) and torch.equal(tiny * 2.0 ** 421, y)
