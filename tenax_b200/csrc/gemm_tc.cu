@@ -35,7 +35,8 @@ static_assert(EPI_WARPS == 4 || EPI_WARPS == 8, "epilogue warps: 4 or 8");
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 // TMEM accumulators: the MMAs may run NACC - 1 tiles ahead of the epilogue.
 // Four (all 512 columns) measured the same as two on the 64-problem H_eff
-// batch (stage 1: 1.84-1.88 vs 1.84-1.86 ms).
+// batch (stage 1: 1.84-1.88 vs 1.84-1.86 ms).  The option is for tiles of 128
+// columns and narrower.
 #ifndef TNX_TMEM_ACC
 #define TNX_TMEM_ACC 2
 #endif
@@ -202,8 +203,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   constexpr int MAXS = ROUTED ? STAGES : (TF32 ? 9 : 4);
   constexpr int KSUB = 4;                   // MMAs per 128-byte K slab (32 B each)
   // TMEM accumulators: the routed instance runs 4 (all 512 columns), so the
-  // MMAs run up to three tiles ahead of its longer epilogue
-  constexpr int NACC = ROUTED ? 4 : ::tnx::NACC;
+  // MMAs run up to three tiles ahead of its longer epilogue; two of 256 columns
+  // are all 512
+  constexpr int NACC = ROUTED ? 4 : TN > TBN ? 2 : ::tnx::NACC;
   constexpr int TMEM_COLS = NACC * TN;
   constexpr int RING = STAGES * NT * TILE_BYTES;
   static_assert(TN == TBN || (TN == 2 * TBN && !ROUTED && TMEM_COLS <= 512), "128 or 256 columns");
