@@ -102,3 +102,40 @@ def test_non_finite_values_stay_in_their_row():
     assert bool(torch.isnan(got[5]).all())
     keep = [i for i in range(70) if i != 5]
     assert bool((got[keep] == 37.0).all())
+
+
+# K shared out over several clusters of one output tile, whose parts a second
+# launch adds: 16 to 32 parts of these shapes
+@pytest.mark.parametrize("subs", ORDERS)
+@pytest.mark.parametrize("m,n,k", [(16, 16, 8000), (4, 4, 102400), (5, 13, 20001), (13, 5, 20000), (33, 70, 20011),
+                                   (70, 33, 20011), (129, 9, 30000)])
+def test_long_k_in_parts(subs, m, n, k):
+    d = {"m": m, "n": n, "k": k}
+    lhs = subs.split("->")[0].split(",")
+    _check(subs, tuple(d[c] for c in lhs[0]), tuple(d[c] for c in lhs[1]), seed=m * 7 + n * 3 + k)
+
+
+@pytest.mark.parametrize("subs,sa,sb", [
+    ("aklx,ylkb->bxya", (3, 150, 140, 5), (7, 140, 150, 4)),   # output legs of both operands interleaved
+    ("kalx,ylbk->xyab", (150, 3, 140, 9), (7, 140, 4, 150)),
+])
+def test_long_k_in_parts_leg_orders(subs, sa, sb):
+    _check(subs, sa, sb)
+
+
+@pytest.mark.parametrize("order", ["ab", "ba"])
+def test_long_k_in_parts_of_blocks(order):
+    """Three sectors of different K, so shares of different lengths in one
+    launch; ragged rows and columns; the output in both orders."""
+    u1 = tb.U1Symmetry()
+    rows = np.repeat(np.array([-1, 0, 1], np.int32), (5, 9, 13))
+    cols = np.repeat(np.array([-1, 0, 1], np.int32), (11, 3, 8))
+    k = np.repeat(np.array([-1, 0, 1], np.int32), (20011, 7000, 12345))
+    a = tb.SymmetricTensor.random_normal((tb.TensorIndex(u1, rows, IN, "a"), tb.TensorIndex(u1, k, OUT, "k")), key=1)
+    b = tb.SymmetricTensor.random_normal((tb.TensorIndex(u1, k, IN, "k"), tb.TensorIndex(u1, cols, OUT, "b")), key=2)
+    idx = {"a": a.indices[0], "b": b.indices[1]}
+    plan = get_plan([a, b], ["ak", "kb"], order, _capi.MATCH_UNFILTERED, tuple(idx[c] for c in order))
+    got = plan.wrap(tuple(idx[c] for c in order), plan.execute([a, b], "fp64")).todense()
+    da, db = a.todense(), b.todense()
+    ref, mag = torch.einsum(f"ak,kb->{order}", da, db), torch.einsum(f"ak,kb->{order}", da.abs(), db.abs())
+    assert bool(((got - ref).abs() <= 2.0 * (20011 + 2) * 2.0 ** -53 * mag).all())
