@@ -103,9 +103,12 @@ class SymmetricTensor:
         self._blocks_cache = None
 
     def __setstate__(self, state):
-        for name, value in state[1].items():
+        attributes, slots = state
+        if attributes:  # a subclass's own
+            self.__dict__.update(attributes)
+        for name, value in slots.items():
             setattr(self, name, value)
-        if "_layout" not in state[1]:  # pickled before layouts were kept
+        if "_layout" not in slots:  # pickled before layouts were kept
             self._layout = Layout(tuple(self._keys), self._offsets, self._shapes, self._key_pos)
 
     @classmethod

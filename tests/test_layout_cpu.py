@@ -68,3 +68,16 @@ def test_validate_reads_only_the_charges_a_leg_has():
     t = SymmetricTensor.from_flat(idx, [(0, 0)], torch.zeros(math.prod(block_shape(idx, (0, 0))), dtype=torch.float64))
     t._keys = [(0, 0, 5), (1, 1, 7)]
     t._validate()
+
+
+class _Annotated(SymmetricTensor):
+    """A subclass with attributes of its own (no slots)."""
+
+
+def test_pickles_of_a_subclass_keep_its_attributes():
+    idx = _legs(U1Symmetry(), 2)
+    n = math.prod(block_shape(idx, (0, 0)))
+    t = _Annotated.from_flat(idx, [(0, 0)], torch.arange(n, dtype=torch.float64))
+    t.note = "left"
+    for u in (pickle.loads(pickle.dumps(t)), copy.deepcopy(t), copy.copy(t)):
+        assert type(u) is _Annotated and u.note == "left" and u._keys == [(0, 0)] and torch.equal(u._data, t._data)
