@@ -90,6 +90,8 @@ def fuse_indices(tensor: SymmetricTensor, axis_a: int, axis_b: int, fused_label,
     new_indices = tuple(others[:a]) + (fused_idx,) + tuple(others[a:])
     out = torch.empty(max(1, plan.total), dtype=torch.float64, device=tensor.data.device)
     if plan.total:
+        if out.device.type != "cuda":
+            raise ValueError(f"fuse_indices expects a tensor on a cuda device, but got: {out.device}")
         _capi.check(_capi.LIB.tnx_fuse_execute(plan.handle, tensor.data.data_ptr(), out.data_ptr(),
                                                torch._C._cuda_getCurrentRawStream(out.device.index)))
     if plan.layout is None:

@@ -13,6 +13,7 @@ torch = pytest.importorskip("torch")
 from tenax_b200.core import (FermionicU1, FermionParity, FlowDirection, TensorIndex, U1Symmetry,  # noqa: E402
                              ZnSymmetry)
 from tenax_b200.tensor import SymmetricTensor, block_shape, make_layout  # noqa: E402
+from tenax_b200.tensor_utils import fuse_indices  # noqa: E402
 
 SYMS = [U1Symmetry(), ZnSymmetry(2), ZnSymmetry(3), FermionParity(), FermionicU1()]
 
@@ -81,3 +82,10 @@ def test_pickles_of_a_subclass_keep_its_attributes():
     t.note = "left"
     for u in (pickle.loads(pickle.dumps(t)), copy.deepcopy(t), copy.copy(t)):
         assert type(u) is _Annotated and u.note == "left" and u._keys == [(0, 0)] and torch.equal(u._data, t._data)
+
+
+def test_fusing_a_tensor_on_the_host_is_a_value_error():
+    idx = _legs(U1Symmetry(), 2)
+    t = SymmetricTensor.from_flat(idx, [(0, 0)], torch.zeros(math.prod(block_shape(idx, (0, 0))), dtype=torch.float64))
+    with pytest.raises(ValueError, match="cuda device"):
+        fuse_indices(t, 0, 1, "f", FlowDirection.IN)
