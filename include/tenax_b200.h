@@ -195,7 +195,8 @@ int tnx_heff_out_keys(const tnx_heff* h, int64_t* n_keys, int32_t* keys);
 /* Keys of theta that H_eff actually writes (others come out zero). */
 double tnx_heff_flops(const tnx_heff* h);
 /* Pack L, W_l, W_r, R (device FP64 block buffers) into GEMM operand images
- * for the given precision; done once per site, reused by every matvec. */
+ * for the given precision (FP64: padded copies of L and R); done once per
+ * site, reused by every matvec. */
 int tnx_heff_set_operators(tnx_heff* h, const double* L, const double* Wl, const double* Wr, const double* R,
                            int32_t precision, void* stream);
 void tnx_heff_destroy(tnx_heff* h);
@@ -222,7 +223,8 @@ int tnx_heff_batch_apply_host(tnx_heff_batch* b, const double* const* host_in, d
 int tnx_heff_batch_size(const tnx_heff_batch* b, int64_t* total, int64_t* offsets);
 /* Re-run one stage of the last apply (0 pack theta, 1 stage-1 GEMM, 2 fused
  * MPO, 3 stage-4 GEMM; with fused stages 1-3: 0 theta panels, 1 the fused
- * kernel, 2 nothing) with the same buffers -- per-kernel timing. */
+ * kernel, 2 nothing; in FP64 0 does nothing) with the same buffers -- per-kernel
+ * timing. */
 int tnx_heff_batch_apply_stage(tnx_heff_batch* b, int32_t stage, void* stream);
 /* Algorithmic flops of stage 1 (L.theta), stages 2+3 (MPO), stage 4 (.R). */
 int tnx_heff_stage_flops(const tnx_heff* h, double* flops3);

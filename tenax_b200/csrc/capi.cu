@@ -1576,7 +1576,8 @@ namespace {
 // operators is less than the launch that would sum them first.  Measured on
 // the cylinder, products against the summing launch: chi = 60 15.5 / 22.6 us,
 // 200 30.9 / 35.0, 300 54.0 / 55.4 (7e7 extra FLOPs), 400 95.5 / 90.1 (1.4e8),
-// 600 211 / 190.
+// 600 211 / 190.  Measured on that one operator, alone; the limit is taken per
+// operator in a batch too, so that its sums are the same there.
 constexpr double kF64ExtraFlops = 1e8;
 constexpr size_t kF64Weights = 6;  // copies of R at most
 

@@ -158,8 +158,9 @@ struct DevRouteTabs {
 };
 
 struct DevTile {
-  int32_t g, mt, nt;
-  int32_t sub;  // tcgen05: columns of a narrow tile << 16 | its first column inside the 128-column tile; 0: all 128
+  int32_t g, mt;
+  int32_t nt;   // column tile: of 256 columns in a tcgen05 launch of that width, else of 128
+  int32_t sub;  // tcgen05: columns of a narrow tile << 16 | its first column inside tile nt; 0: the launch's full width
 };
 
 struct DevMpoPair {
@@ -258,9 +259,12 @@ static __device__ __forceinline__ void img_store_chunk(uint8_t* img, int64_t lo_
 // ---------------------------------------------------------------------------
 
 // Programmatic dependent launch.  A kernel launched by launch_pdl may start
-// while its predecessor in the stream still runs; it reads only tables written
-// before the plan or batch was first used until pdl_wait(), which returns once
-// the predecessor has completed and its writes are visible.  pdl_trigger() lets
+// while its predecessor in the stream still runs, if that is a kernel (a copy or
+// a memset is waited for in full).  Until pdl_wait(), which returns once the
+// predecessor has completed and its writes are visible, it reads only tables
+// that no kernel writes: uploaded with the plan or batch, or by copies of the
+// same call (tnx_plan_execute_static, tnx_heff_set_operators), which every
+// later launch of the stream comes after.  pdl_trigger() lets
 // the successor start likewise.  Every kernel launched this way waits before its
 // first dependent access (the skip flag included), so completion stays in stream
 // order; what overlaps is the launch and the prologue.

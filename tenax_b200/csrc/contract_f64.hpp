@@ -115,7 +115,7 @@ constexpr int kContractShapes = 4;
 void contract_choose(const std::vector<ContractBlk>& blks, int n_sm, int min_split, int max_split, int* shape,
                      int* split, int* parts);
 // appends to `dst` the tiles of the blocks `proto` (M, N and the block's axes
-// set) in the launch's shape, longest first; returns their number
+// set) in the launch's shape, longest first to within 1/32; returns their number
 int64_t contract_tiles(const std::vector<ContractTile>& proto, const std::vector<ContractBlk>& blks, int shape,
                        std::vector<uint8_t>& dst);
 cudaError_t launch_contract_f64(const ContractLaunch& L, cudaStream_t st);

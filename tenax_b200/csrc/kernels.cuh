@@ -12,8 +12,10 @@ namespace tnx {
 // `cluster` CTAs where that is above 1.  A failure is also the thread's last
 // CUDA error.  What the overlap saves is a launch gap of 1 to 2 us a kernel:
 // H_eff in TF32 at chi = 512, four launches, 58.8 -> 52.4 us; the FP64 chain at
-// chi = 64, two, 12.3 -> 9.4 us.  Launches of more than kPdlWork units run for
-// hundreds of us and go without (a 16-problem batch: within 2 % either way).
+// chi = 64, two, 12.3 -> 9.4 us.  `work` stands for how long the launch runs: its
+// CTAs or tiles, a sixteenth of them where a tile is a few us (contract_f64).
+// Above kPdlWork it is hundreds of us and goes without (a 16-problem batch:
+// within 2 % either way, so where the line lies matters little).
 // The tcgen05 GEMM does not trigger its successor early: CTAs of the MPO kernel
 // resident beside it keep the SM's carve-out, so that kernel would run with its
 // L1 at a few KB (TF32 chi = 512: 85 us).
@@ -110,7 +112,7 @@ void launch_renorm_adjoint(const RenormArgs& a, int nt, double eps, const double
 void launch_gemm_f64(const DevGroup* groups, const DevTile* tiles, int n_tiles, const int64_t* rowoff,
                      const uint64_t* out_tab, const int32_t* skip, cudaStream_t st);
 // tcgen05 grouped GEMM; mode IMG_BF16 (3 products over hi/lo images) or IMG_TF32.
-// width: columns of every tile (128, 64 or 32; routed launches 128)
+// width: columns of every tile (256, 128, 64 or 32; routed launches 128); the tile list is made for it (DevTile)
 // rt: the routed groups' tables (FP32 results only; empty when no group is routed)
 void launch_gemm_tc(int mode, const DevGroup* groups, const DevTile* tiles, int n_tiles, const int64_t* rowoff,
                     const uint64_t* out_tab, bool out_f64, int32_t* err_flag, const int32_t* skip, cudaStream_t st,

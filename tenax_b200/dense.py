@@ -2,14 +2,16 @@
 
 A dense tensor is a block-sparse tensor with one block: every leg carries
 the trivial charge 0, so the planner sees a single sector and the contraction
-becomes one permute-pack, one grouped tensor-core GEMM and one scatter in the
-library -- the same kernels as the symmetric path.  ``einsum`` evaluates one
+runs the kernels of the symmetric path: in FP64 one launch that gathers,
+multiplies and stores, in the mixed precisions one pack, one grouped
+tensor-core GEMM and one scatter.  ``einsum`` evaluates one
 pairwise contraction (or a single-operand permutation) given as subscripts;
 ``Contract`` makes it differentiable: the adjoint of ``C = A *_{s} B`` is two
 more contractions of the same engine, dA = C' *_{sC,sB} B and dB = A *_{sA,sC} C'.
 
-Plans are cached per (subscripts, shapes); each owns its device buffers, and
-calls that share a plan are ordered by the stream they run on.
+Plans are cached per (subscripts, shapes, precision); each owns its device
+tables and, in the mixed precisions, its operand images and result matrix, so
+calls that share such a plan have to run on one stream.
 """
 
 from __future__ import annotations

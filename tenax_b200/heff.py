@@ -12,8 +12,11 @@ three stages over all sectors at once:
    the theta block layout.
 
 Operator images (L, R, W_l W_r terms) are packed once per site; a matvec
-only packs theta.  Many independent problems share each launch
-(``HeffBatch``).
+only packs theta.  In FP64 there are no images: L and R are copied once per
+site with padded rows (R once per common W_l W_r weight), theta is read and
+the result written in place, stage 2 forms only the sums worth a launch and
+stage 3 sums one product per remaining term.  Many independent problems share
+each launch (``HeffBatch``).
 """
 
 from __future__ import annotations
