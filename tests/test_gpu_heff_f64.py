@@ -16,7 +16,8 @@ if not torch.cuda.is_available():  # pragma: no cover
 
 import tenax_b200 as tb  # noqa: E402
 from tenax_b200.auto_mpo import build_auto_mpo_sites, to_symmetric  # noqa: E402
-from tenax_b200.tensor import SymmetricTensor, embed_in_keys, restrict_to_keys  # noqa: E402
+from tenax_b200.tensor import SymmetricTensor, embed_in_keys  # noqa: E402
+from tenax_b200.tensor import restrict_to_keys  # noqa: E402
 from tenax_b200.workloads import chain_bulk_w, cylinder_bulk_w, make_heff_problem  # noqa: E402
 
 
